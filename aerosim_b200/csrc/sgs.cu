@@ -17,8 +17,6 @@
 namespace aerosim {
 namespace {
 
-constexpr int kTrainBlock = 128;
-
 // Forward pass of one sample; keeps the pre-activations for the backward pass.
 __device__ __forceinline__ float mlp_forward_keep(const float* P, const float (&x)[kMlpIn], float (&z1)[kMlpHidden],
                                                   float (&z2)[kMlpHidden], float& o) {
@@ -43,59 +41,265 @@ __device__ __forceinline__ float mlp_forward_keep(const float* P, const float (&
   return softplus_f(o);
 }
 
-// Loss and gradient of the mean squared error (prediction - target)^2 over n samples
-// (rows of X, or the rows listed in idx), accumulated into G and *loss.
-__global__ void __launch_bounds__(kTrainBlock) mlp_grad_kernel(const float* __restrict__ Pg, const float* __restrict__ X,
-                                                               const float* __restrict__ Y,
-                                                               const long long* __restrict__ idx, long long n,
-                                                               float inv_n, float* __restrict__ G,
-                                                               double* __restrict__ loss) {
-  __shared__ float P[kMlpParams];
-  __shared__ float sG[kMlpParams];
-  for (int p = threadIdx.x; p < kMlpParams; p += blockDim.x) {
-    P[p] = Pg[p];
-    sG[p] = 0.0f;
+// ---- training: loss and gradient of the mean squared error (prediction - target)^2 ----
+// One warp takes kGradRows samples at a time, lane = hidden unit: the lane's rows of W1 and
+// W2 and its share of the gradient (rows of dW1 and dW2, the biases, dW3) stay in registers
+// over all samples of the warp; activations and back-propagated errors pass between the
+// lanes through a few hundred bytes of shared memory per warp as broadcast loads.  The
+// contractions over a row pair run as packed FP32 (f32x2) FMAs.  Nothing is accumulated
+// with atomics: a CTA adds its warps' registers in order and writes one row of partial sums,
+// and the kernel that applies them adds the CTAs' rows in a fixed order, so a training run
+// is reproducible bit for bit.  The work is far too small to fill the chip's FP32 pipes
+// (65 MFMA a batch of 16384): what bounds it is the latency of a sample's chain (gather,
+// two layers, the output sum, two layers back), which kGradRows samples in flight per warp
+// and 16 warps per SM hide.  Batch of 16384 (B200): one thread per sample with shared-memory
+// atomics 6360 us an iteration, now 27 us with the parameter update (batch 512: 10.7 us).
+constexpr int kGradRows = 4;
+constexpr int kGradWarps = 16;
+static_assert(kGradRows == 4, "a group of samples is one float4 of back-propagated errors");
+// Partial sums of a CTA: column c, lane j at c * 32 + j (coalesced for both kernels).
+// c = 0..7: dW1[j][c]; 8: db1[j]; 9..40: dW2[j][c - 9]; 41: db2[j]; 42: dW3[j]; 43: db3 (lane 0).
+constexpr int kGradCols = 44, kGradSlots = kGradCols * 32;
+constexpr int kGradStage = kGradRows * (kMlpIn + 2 * kMlpHidden);  // floats of a warp's exchange area
+constexpr int kGradW2Row = kMlpHidden + 4;  // padded row of W2 in shared memory: rows and columns read without conflicts
+constexpr int kGradSmem = (kMlpHidden * kGradW2Row + kGradWarps * (kGradStage + kGradSlots)) * 4;
+
+// Parameter of column c, lane j; -1 where there is none.
+__host__ __device__ constexpr int grad_param(int c, int j) {
+  return c < 8 ? kMlpW1 + j * kMlpIn + c : c == 8 ? kMlpB1 + j : c < 41 ? kMlpW2 + j * kMlpHidden + (c - 9)
+       : c == 41 ? kMlpB2 + j : c == 42 ? kMlpW3 + j : (j == 0 ? kMlpB3 : -1);
+}
+
+// GELU and its derivative from one tanh.
+__device__ __forceinline__ float gelu_both(float x, float& grad) {
+  const float t = tanhf(kGeluK * (x + 0.044715f * x * x * x));
+  grad = 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * kGeluK * (1.0f + 3.0f * 0.044715f * x * x);
+  return 0.5f * x * (1.0f + t);
+}
+
+// Row of sample i of a mini-batch: a splitmix64 hash of (seed, iteration, i) modulo n.
+struct BatchRows {
+  unsigned long long seed;
+  unsigned long long n;      // rows to draw from; 0: sample i is row i
+  unsigned long long recip;  // (2^64 - 1) / n
+  int it;
+  __device__ __forceinline__ long long row(long long i) const {
+    if (n == 0) return i;
+    unsigned long long z = seed + 0x9e3779b97f4a7c15ull * ((unsigned long long)it * 1000003ull + (unsigned long long)i + 1ull);
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
+    z ^= z >> 31;
+    // z mod n: the quotient from the reciprocal is at most two too small
+    unsigned long long r = z - __umul64hi(z, recip) * n;
+    if (r >= n) r -= n;
+    if (r >= n) r -= n;
+    return (long long)r;
   }
+};
+
+__global__ void __launch_bounds__(kGradWarps * 32, 1)
+    mlp_grad_kernel(const float* __restrict__ Pg, const float* __restrict__ X, const float* __restrict__ Y,
+                    const BatchRows rows, long long n, float inv_n, float* __restrict__ partial,
+                    double* __restrict__ loss_partial) {
+  extern __shared__ __align__(16) float gsm[];
+  __shared__ double s_loss[kGradWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* const sW2 = gsm;                                              // [j][k]
+  float* const red = gsm + kMlpHidden * kGradW2Row;                    // [warp][slot]
+  float* const sx = red + kGradWarps * kGradSlots + warp * kGradStage;  // [row][8]
+  float* const sh = sx + kGradRows * kMlpIn;                           // [row][k]
+  float* const sd = sh + kGradRows * kMlpHidden;                       // [j][row]
+  const long long groups = (n + kGradRows - 1) / kGradRows;
+  const long long stride = (long long)gridDim.x * kGradWarps;
+  long long g = (long long)blockIdx.x * kGradWarps + warp;
+  // the samples of a group: lane l holds input l % 8 of its row l / 8; lane l < kGradRows its target
+  auto load = [&](long long gi, float& x, float& y) {
+    const long long i = gi * kGradRows + (lane >> 3);
+    x = i < n ? X[rows.row(i) * kMlpIn + (lane & 7)] : 0.0f;
+    const long long iy = gi * kGradRows + lane;
+    y = (lane < kGradRows && iy < n) ? Y[rows.row(iy)] : 0.0f;
+  };
+  float xn = 0.0f, yn = 0.0f;
+  if (g < groups) load(g, xn, yn);  // the samples do not change between iterations
+  // launched as a programmatic dependent of the kernel that updates the parameters
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  for (int i = threadIdx.x; i < kMlpHidden * kMlpHidden; i += blockDim.x)
+    sW2[(i / kMlpHidden) * kGradW2Row + i % kMlpHidden] = __ldcg(&Pg[kMlpW2 + i]);
+  float w1[kMlpIn], a1[kMlpIn];
+  float2 w2[kMlpHidden / 2], a2[kMlpHidden / 2];
+#pragma unroll
+  for (int i = 0; i < kMlpIn; ++i) {
+    w1[i] = __ldcg(&Pg[kMlpW1 + lane * kMlpIn + i]);
+    a1[i] = 0.0f;
+  }
+  const float b1 = __ldcg(&Pg[kMlpB1 + lane]), b2 = __ldcg(&Pg[kMlpB2 + lane]), w3 = __ldcg(&Pg[kMlpW3 + lane]),
+              b3 = __ldcg(&Pg[kMlpB3]);
   __syncthreads();
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < kMlpHidden / 4; ++k) {
+    const float4 w = *reinterpret_cast<const float4*>(sW2 + lane * kGradW2Row + 4 * k);
+    w2[2 * k] = make_float2(w.x, w.y);
+    w2[2 * k + 1] = make_float2(w.z, w.w);
+    a2[2 * k] = a2[2 * k + 1] = make_float2(0.0f, 0.0f);
+  }
+  float ab1 = 0.0f, ab2 = 0.0f, aw3 = 0.0f, ab3 = 0.0f;
   double l = 0.0;
-  if (t < n) {
-    const long long r = idx ? idx[t] : t;
-    float x[kMlpIn];
+  for (; g < groups; g += stride) {
+    sx[lane] = xn;
+    const float yc = yn;
+    __syncwarp();
+    if (g + stride < groups) load(g + stride, xn, yn);
+    float g1[kGradRows], d[kGradRows];
 #pragma unroll
-    for (int i = 0; i < kMlpIn; ++i) x[i] = X[r * kMlpIn + i];
-    float z1[kMlpHidden], z2[kMlpHidden], o;
-    const float pred = mlp_forward_keep(P, x, z1, z2, o);
-    const float e = pred - Y[r];
-    l = (double)e * e;
-    const float d_o = 2.0f * e * sigmoid_f(o) * inv_n;
-    atomicAdd(&sG[kMlpB3], d_o);
-    float d1[kMlpHidden];
+    for (int r = 0; r < kGradRows; ++r) {
+      const float4 xa = *reinterpret_cast<const float4*>(sx + r * kMlpIn), xb = *reinterpret_cast<const float4*>(sx + r * kMlpIn + 4);
+      float s = b1;
+      s = fmaf(w1[0], xa.x, s); s = fmaf(w1[1], xa.y, s); s = fmaf(w1[2], xa.z, s); s = fmaf(w1[3], xa.w, s);
+      s = fmaf(w1[4], xb.x, s); s = fmaf(w1[5], xb.y, s); s = fmaf(w1[6], xb.z, s); s = fmaf(w1[7], xb.w, s);
+      sh[r * kMlpHidden + lane] = gelu_both(s, g1[r]);
+    }
+    __syncwarp();
+    float h2[kGradRows], g2[kGradRows], o[kGradRows];
 #pragma unroll
-    for (int k = 0; k < kMlpHidden; ++k) d1[k] = 0.0f;
-    for (int j = 0; j < kMlpHidden; ++j) {
-      const float h2 = gelu_f(z2[j]);
-      atomicAdd(&sG[kMlpW3 + j], d_o * h2);
-      const float d2 = d_o * P[kMlpW3 + j] * gelu_grad(z2[j]);
-      atomicAdd(&sG[kMlpB2 + j], d2);
+    for (int r = 0; r < kGradRows; ++r) {
+      float2 s = make_float2(b2, 0.0f);
 #pragma unroll
-      for (int k = 0; k < kMlpHidden; ++k) {
-        atomicAdd(&sG[kMlpW2 + j * kMlpHidden + k], d2 * gelu_f(z1[k]));
-        d1[k] = fmaf(d2, P[kMlpW2 + j * kMlpHidden + k], d1[k]);
+      for (int k = 0; k < kMlpHidden / 4; ++k) {
+        const float4 h = *reinterpret_cast<const float4*>(sh + r * kMlpHidden + 4 * k);
+        s = __ffma2_rn(w2[2 * k], make_float2(h.x, h.y), s);
+        s = __ffma2_rn(w2[2 * k + 1], make_float2(h.z, h.w), s);
+      }
+      h2[r] = gelu_both(s.x + s.y, g2[r]);
+      o[r] = w3 * h2[r];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+#pragma unroll
+      for (int r = 0; r < kGradRows; ++r) o[r] += __shfl_xor_sync(0xffffffffu, o[r], off);
+    }
+#pragma unroll
+    for (int r = 0; r < kGradRows; ++r) {
+      const float ov = o[r] + b3;
+      const float e = softplus_f(ov) - __shfl_sync(0xffffffffu, yc, r);
+      const bool in = g * kGradRows + r < n;
+      if (in) l += (double)e * e;
+      const float d_o = in ? 2.0f * e * sigmoid_f(ov) * inv_n : 0.0f;
+      ab3 += d_o;
+      aw3 = fmaf(d_o, h2[r], aw3);
+      d[r] = d_o * w3 * g2[r];
+      ab2 += d[r];
+    }
+    *reinterpret_cast<float4*>(sd + lane * kGradRows) = make_float4(d[0], d[1], d[2], d[3]);
+    __syncwarp();
+    // dW2[j][k] += d2[j] h1[k], lane j
+#pragma unroll
+    for (int r = 0; r < kGradRows; ++r) {
+      const float2 dd = make_float2(d[r], d[r]);
+#pragma unroll
+      for (int k = 0; k < kMlpHidden / 4; ++k) {
+        const float4 h = *reinterpret_cast<const float4*>(sh + r * kMlpHidden + 4 * k);
+        a2[2 * k] = __ffma2_rn(dd, make_float2(h.x, h.y), a2[2 * k]);
+        a2[2 * k + 1] = __ffma2_rn(dd, make_float2(h.z, h.w), a2[2 * k + 1]);
       }
     }
-    for (int k = 0; k < kMlpHidden; ++k) {
-      const float dk = d1[k] * gelu_grad(z1[k]);
-      atomicAdd(&sG[kMlpB1 + k], dk);
+    // d1[k] = sum_j d2[j] W2[j][k], lane k, two samples to a packed pair
+    float2 e01 = make_float2(0.0f, 0.0f), e23 = e01;
+#pragma unroll 8
+    for (int j = 0; j < kMlpHidden; ++j) {
+      const float w = sW2[j * kGradW2Row + lane];
+      const float4 dj = *reinterpret_cast<const float4*>(sd + j * kGradRows);
+      e01 = __ffma2_rn(make_float2(w, w), make_float2(dj.x, dj.y), e01);
+      e23 = __ffma2_rn(make_float2(w, w), make_float2(dj.z, dj.w), e23);
+    }
+    const float e1[kGradRows] = {e01.x * g1[0], e01.y * g1[1], e23.x * g1[2], e23.y * g1[3]};
 #pragma unroll
-      for (int i = 0; i < kMlpIn; ++i) atomicAdd(&sG[kMlpW1 + k * kMlpIn + i], dk * x[i]);
+    for (int r = 0; r < kGradRows; ++r) {
+      const float4 xa = *reinterpret_cast<const float4*>(sx + r * kMlpIn), xb = *reinterpret_cast<const float4*>(sx + r * kMlpIn + 4);
+      ab1 += e1[r];
+      a1[0] = fmaf(e1[r], xa.x, a1[0]); a1[1] = fmaf(e1[r], xa.y, a1[1]);
+      a1[2] = fmaf(e1[r], xa.z, a1[2]); a1[3] = fmaf(e1[r], xa.w, a1[3]);
+      a1[4] = fmaf(e1[r], xb.x, a1[4]); a1[5] = fmaf(e1[r], xb.y, a1[5]);
+      a1[6] = fmaf(e1[r], xb.z, a1[6]); a1[7] = fmaf(e1[r], xb.w, a1[7]);
+    }
+    __syncwarp();  // the exchange area is free for the next group
+  }
+  float* const rw = red + warp * kGradSlots + lane;
+#pragma unroll
+  for (int i = 0; i < kMlpIn; ++i) rw[i * 32] = a1[i];
+  rw[8 * 32] = ab1;
+#pragma unroll
+  for (int k = 0; k < kMlpHidden / 2; ++k) {
+    rw[(9 + 2 * k) * 32] = a2[k].x;
+    rw[(10 + 2 * k) * 32] = a2[k].y;
+  }
+  rw[41 * 32] = ab2;
+  rw[42 * 32] = aw3;
+  rw[43 * 32] = lane == 0 ? ab3 : 0.0f;
+  if (lane == 0) s_loss[warp] = l;
+  __syncthreads();
+  for (int i = threadIdx.x; i < kGradSlots; i += blockDim.x) {
+    float s = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kGradWarps; ++w) s += red[w * kGradSlots + i];
+    partial[(size_t)blockIdx.x * kGradSlots + i] = s;
+  }
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int w = 0; w < kGradWarps; ++w) s += s_loss[w];
+    loss_partial[blockIdx.x] = s;
+  }
+}
+
+// Adds the partial sums of `ctas` CTAs in a fixed order (CTA c: one column of 32
+// parameters) and either writes the gradient (G) or takes an Adam step (Kingma & Ba, 2015)
+// on the FP32 parameters; CTA 0 adds the loss.
+struct AdamState {
+  float *P, *m, *v;
+  float lr, b1t, b2t;
+};
+constexpr int kApplyThreads = 512;
+__global__ void __launch_bounds__(kApplyThreads)
+    mlp_apply_kernel(const float* __restrict__ partial, const double* __restrict__ loss_partial, int ctas, float inv_n,
+                     float* __restrict__ G, const AdamState st, double* __restrict__ loss) {
+  __shared__ float s[kApplyThreads];
+  __shared__ double sl[32];
+  const int c = blockIdx.x, lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  float acc = 0.0f;
+#pragma unroll 4
+  for (int k = part; k < ctas; k += kApplyThreads / 32) acc += __ldcg(&partial[(size_t)k * kGradSlots + c * 32 + lane]);
+  s[threadIdx.x] = acc;
+  if (c == 0 && part == 0) {
+    double d = 0.0;
+    for (int k = lane; k < ctas; k += 32) d += __ldcg(&loss_partial[k]);
+    sl[lane] = d;
+  }
+  __syncthreads();
+  if (part == 0) {
+    float g = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kApplyThreads / 32; ++k) g += s[k * 32 + lane];
+    const int p = grad_param(c, lane);
+    if (p >= 0) {
+      if (G) {
+        G[p] = g;
+      } else {
+        const float mp = 0.9f * st.m[p] + 0.1f * g;
+        const float vp = 0.999f * st.v[p] + 0.001f * g * g;
+        st.m[p] = mp;
+        st.v[p] = vp;
+        const float mh = mp / (1.0f - st.b1t), vh = vp / (1.0f - st.b2t);
+        st.P[p] -= st.lr * mh / (sqrtf(vh) + 1e-8f);
+      }
+    }
+    if (c == 0 && lane == 0) {
+      double d = 0.0;
+      for (int k = 0; k < 32; ++k) d += sl[k];
+      *loss = d * (double)inv_n;
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
-  if ((threadIdx.x & 31) == 0 && l != 0.0) atomicAdd(loss, l * (double)inv_n);
-  __syncthreads();
-  for (int p = threadIdx.x; p < kMlpParams; p += blockDim.x) atomicAdd(&G[p], sG[p]);
 }
 
 __global__ void mlp_forward_kernel(const float* __restrict__ Pg, const float* __restrict__ X, long long n,
@@ -232,31 +436,6 @@ __global__ void __launch_bounds__(kUmmaRows) mlp_forward_umma_kernel(const uint4
   __syncthreads();
   tc_fence_after();
   if (warp == 0) tmem_dealloc(tbase, kUmmaCols);
-}
-
-// Adam (Kingma & Ba, 2015) on the FP32 parameters.
-__global__ void adam_kernel(float* __restrict__ P, float* __restrict__ m, float* __restrict__ v,
-                            const float* __restrict__ G, float lr, float b1t, float b2t) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kMlpParams) return;
-  const float g = G[p];
-  const float mp = 0.9f * m[p] + 0.1f * g;
-  const float vp = 0.999f * v[p] + 0.001f * g * g;
-  m[p] = mp;
-  v[p] = vp;
-  const float mh = mp / (1.0f - b1t), vh = vp / (1.0f - b2t);
-  P[p] -= lr * mh / (sqrtf(vh) + 1e-8f);
-}
-
-// Mini-batch rows: a splitmix64 hash of (seed, iteration, slot) modulo n.
-__global__ void batch_index_kernel(long long* __restrict__ idx, int B, unsigned long long seed, int it, long long n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= B) return;
-  unsigned long long z = seed + 0x9e3779b97f4a7c15ull * ((unsigned long long)it * 1000003ull + (unsigned long long)i + 1ull);
-  z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
-  z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
-  z ^= z >> 31;
-  idx[i] = (long long)(z % (unsigned long long)n);
 }
 
 // ---- wall distance: jump flooding over the solid cells (Rong & Tan, 2006) ----------
@@ -479,6 +658,66 @@ struct DevBuf {
   template <class T> T* as() { return static_cast<T*>(p); }
 };
 
+// Device buffers of a training or gradient call, in one allocation: parameters, Adam
+// moments, samples, the CTAs' partial sums and the losses.
+constexpr int kMlpPad = (kMlpParams + 63) / 64 * 64;
+struct TrainBufs {
+  DevBuf mem;
+  float *P = nullptr, *M = nullptr, *V = nullptr, *X = nullptr, *Y = nullptr, *partial = nullptr;
+  double *loss_partial = nullptr, *loss = nullptr;
+  int max_ctas = 1;
+  cudaError_t alloc(int64_t n, int64_t batch, int64_t losses) {
+    int dev = 0, sms = 1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem);
+    if (e != cudaSuccess) return e;
+    const int64_t groups = (batch + kGradRows - 1) / kGradRows;
+    max_ctas = (int)std::min<int64_t>(sms, (groups + kGradWarps - 1) / kGradWarps);
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t bx = up((size_t)n * kMlpIn * 4), by = up((size_t)n * 4), bp = up((size_t)max_ctas * kGradSlots * 4),
+                 bl = up((size_t)max_ctas * 8), bL = up((size_t)losses * 8);
+    e = mem.alloc(3 * kMlpPad * 4 + bx + by + bp + bl + bL);
+    if (e != cudaSuccess) return e;
+    char* c = mem.as<char>();
+    P = reinterpret_cast<float*>(c);
+    M = P + kMlpPad;
+    V = M + kMlpPad;
+    c += 3 * kMlpPad * 4;
+    X = reinterpret_cast<float*>(c); c += bx;
+    Y = reinterpret_cast<float*>(c); c += by;
+    partial = reinterpret_cast<float*>(c); c += bp;
+    loss_partial = reinterpret_cast<double*>(c); c += bl;
+    loss = reinterpret_cast<double*>(c);
+    return cudaSuccess;
+  }
+};
+
+// Gradient of n samples and its use, on the default stream, each kernel a programmatic
+// dependent of the one before it.
+cudaError_t launch_train_step(const TrainBufs& t, const BatchRows& rows, int64_t n, float* G, const AdamState& st,
+                              double* loss) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  const float inv_n = 1.0f / (float)n;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)t.max_ctas);
+  cfg.blockDim = dim3(kGradWarps * 32);
+  cfg.dynamicSmemBytes = kGradSmem;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, mlp_grad_kernel, (const float*)t.P, (const float*)t.X, (const float*)t.Y, rows,
+                                     (long long)n, inv_n, t.partial, t.loss_partial);
+  if (e != cudaSuccess) return e;
+  cfg.gridDim = dim3(kGradCols);
+  cfg.blockDim = dim3(kApplyThreads);
+  cfg.dynamicSmemBytes = 0;
+  return cudaLaunchKernelEx(&cfg, mlp_apply_kernel, (const float*)t.partial, (const double*)t.loss_partial, t.max_ctas,
+                            inv_n, G, st, loss);
+}
+
 }  // namespace
 
 // Jump-flood wall distance of a dense flag array (device), written as float distances
@@ -628,22 +867,15 @@ int aerosim_mlp_last_timing(double* ms) {
 int aerosim_mlp_gradients(const float* params, const float* X, const float* Y, int64_t n, float* grad,
                           double* loss) {
   if (!params || !X || !Y || !grad || !loss || n < 1) return sgs_fail(AEROSIM_ERR_ARG, "mlp_gradients: bad argument");
-  DevBuf P, Xd, Yd, G, L;
-  SCU(P.alloc(kMlpParams * 4));
-  SCU(Xd.alloc((size_t)n * kMlpIn * 4));
-  SCU(Yd.alloc((size_t)n * 4));
-  SCU(G.alloc(kMlpParams * 4));
-  SCU(L.alloc(8));
-  SCU(cudaMemcpy(P.p, params, kMlpParams * 4, cudaMemcpyHostToDevice));
-  SCU(cudaMemcpy(Xd.p, X, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice));
-  SCU(cudaMemcpy(Yd.p, Y, (size_t)n * 4, cudaMemcpyHostToDevice));
-  SCU(cudaMemset(G.p, 0, kMlpParams * 4));
-  SCU(cudaMemset(L.p, 0, 8));
-  mlp_grad_kernel<<<(unsigned)((n + kTrainBlock - 1) / kTrainBlock), kTrainBlock>>>(
-      P.as<float>(), Xd.as<float>(), Yd.as<float>(), nullptr, n, 1.0f / (float)n, G.as<float>(), L.as<double>());
-  SCU(cudaGetLastError());
-  SCU(cudaMemcpy(grad, G.p, kMlpParams * 4, cudaMemcpyDeviceToHost));
-  SCU(cudaMemcpy(loss, L.p, 8, cudaMemcpyDeviceToHost));
+  TrainBufs t;
+  SCU(t.alloc(n, n, 1));
+  SCU(cudaMemcpy(t.P, params, kMlpParams * 4, cudaMemcpyHostToDevice));
+  SCU(cudaMemcpy(t.X, X, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice));
+  SCU(cudaMemcpy(t.Y, Y, (size_t)n * 4, cudaMemcpyHostToDevice));
+  AdamState st{};
+  SCU(launch_train_step(t, BatchRows{0, 0, 0, 0}, n, t.M, st, t.loss));
+  SCU(cudaMemcpy(grad, t.M, kMlpParams * 4, cudaMemcpyDeviceToHost));
+  SCU(cudaMemcpy(loss, t.loss, 8, cudaMemcpyDeviceToHost));
   return AEROSIM_OK;
 }
 
@@ -651,39 +883,23 @@ int aerosim_mlp_train(float* params, const float* X, const float* Y, int64_t n, 
                       float lr, uint64_t seed, float* loss_curve) {
   if (!params || !X || !Y || n < 1 || iters < 0 || batch < 1 || !(lr > 0.0f))
     return sgs_fail(AEROSIM_ERR_ARG, "mlp_train: bad argument");
-  DevBuf P, Xd, Yd, G, M, V, L, I;
-  SCU(P.alloc(kMlpParams * 4));
-  SCU(Xd.alloc((size_t)n * kMlpIn * 4));
-  SCU(Yd.alloc((size_t)n * 4));
-  SCU(G.alloc(kMlpParams * 4));
-  SCU(M.alloc(kMlpParams * 4));
-  SCU(V.alloc(kMlpParams * 4));
-  SCU(L.alloc((size_t)std::max(iters, 1) * 8));
-  SCU(I.alloc((size_t)batch * 8));
-  SCU(cudaMemcpy(P.p, params, kMlpParams * 4, cudaMemcpyHostToDevice));
-  SCU(cudaMemcpy(Xd.p, X, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice));
-  SCU(cudaMemcpy(Yd.p, Y, (size_t)n * 4, cudaMemcpyHostToDevice));
-  SCU(cudaMemset(M.p, 0, kMlpParams * 4));
-  SCU(cudaMemset(V.p, 0, kMlpParams * 4));
-  SCU(cudaMemset(L.p, 0, (size_t)std::max(iters, 1) * 8));
-  float b1t = 1.0f, b2t = 1.0f;
+  TrainBufs t;
+  SCU(t.alloc(n, batch, std::max(iters, 1)));
+  SCU(cudaMemcpy(t.P, params, kMlpParams * 4, cudaMemcpyHostToDevice));
+  SCU(cudaMemcpy(t.X, X, (size_t)n * kMlpIn * 4, cudaMemcpyHostToDevice));
+  SCU(cudaMemcpy(t.Y, Y, (size_t)n * 4, cudaMemcpyHostToDevice));
+  SCU(cudaMemsetAsync(t.M, 0, 2 * kMlpPad * 4));  // M and V
+  AdamState st{t.P, t.M, t.V, lr, 1.0f, 1.0f};
   for (int it = 0; it < iters; ++it) {
-    b1t *= 0.9f;
-    b2t *= 0.999f;
-    batch_index_kernel<<<(batch + 255) / 256, 256>>>(I.as<long long>(), batch, seed, it, n);
-    SCU(cudaMemsetAsync(G.p, 0, kMlpParams * 4));
-    mlp_grad_kernel<<<(batch + kTrainBlock - 1) / kTrainBlock, kTrainBlock>>>(
-        P.as<float>(), Xd.as<float>(), Yd.as<float>(), I.as<long long>(), batch, 1.0f / (float)batch, G.as<float>(),
-        L.as<double>() + it);
-    adam_kernel<<<(kMlpParams + 255) / 256, 256>>>(P.as<float>(), M.as<float>(), V.as<float>(), G.as<float>(), lr,
-                                                   b1t, b2t);
+    st.b1t *= 0.9f;
+    st.b2t *= 0.999f;
+    SCU(launch_train_step(t, BatchRows{seed, (unsigned long long)n, ~0ull / (unsigned long long)n, it}, batch, nullptr, st, t.loss + it));
   }
-  SCU(cudaGetLastError());
   SCU(cudaDeviceSynchronize());
-  SCU(cudaMemcpy(params, P.p, kMlpParams * 4, cudaMemcpyDeviceToHost));
+  SCU(cudaMemcpy(params, t.P, kMlpParams * 4, cudaMemcpyDeviceToHost));
   if (loss_curve && iters > 0) {
     std::vector<double> l(iters);
-    SCU(cudaMemcpy(l.data(), L.p, (size_t)iters * 8, cudaMemcpyDeviceToHost));
+    SCU(cudaMemcpy(l.data(), t.loss, (size_t)iters * 8, cudaMemcpyDeviceToHost));
     for (int i = 0; i < iters; ++i) loss_curve[i] = (float)l[i];
   }
   return AEROSIM_OK;
