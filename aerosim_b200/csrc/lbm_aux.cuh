@@ -259,53 +259,80 @@ __global__ void slice_kernel(const float* __restrict__ mux, const float* __restr
 // reference's operation order (-fmad=false), float outputs, 0 at solid cells (flags may be
 // null); the maxima (starting at 1e-6) as the bit patterns of non-negative doubles, so an
 // unsigned max is exact and order-free.
-__global__ void q_criterion_kernel(int nx, int ny, int nz, double dx, const float* __restrict__ ux,
+// A CTA reduces its maxima and issues one atomic each: two per thread, all on the same two
+// words, took most of the 432 us the kernel needed at 192x96x96 (32 us now).  The spacings
+// (n - p) dx take two values only, so their reciprocals are formed once per thread by the
+// operations the reference forms them with.  Index is uint32_t below 2^31 cells (64-bit
+// divisions per cell otherwise).
+template <class Index>
+__global__ void __launch_bounds__(256) q_criterion_kernel(int nx, int ny, int nz, double dx, const float* __restrict__ ux,
                                    const float* __restrict__ uy, const float* __restrict__ uz,
                                    const uint8_t* __restrict__ flags, float* __restrict__ q,
                                    float* __restrict__ om, float* __restrict__ omv,
                                    unsigned long long* __restrict__ maxima) {
-  const long long N = (long long)nx * ny * nz;
-  const double inv2dx = 1.0 / (2.0 * dx);
+  const Index N = (Index)nx * (Index)ny * (Index)nz;
+  const double inv2dx = 1.0 / (2.0 * dx), inv1dx = 1.0 / (1.0 * dx);
   double mq = 0.0, mo = 0.0;
-  auto at = [&](int x, int y, int z) { return x + (long long)nx * (y + (long long)ny * z); };
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-    const int ix = (int)(i % nx);
-    const long long r = i / nx;
-    const int iy = (int)(r % ny), iz = (int)(r / ny);
-    if (flags && flags[i] == CELL_SOLID) {
-      q[i] = 0.0f; om[i] = 0.0f; omv[3 * i] = 0.0f; omv[3 * i + 1] = 0.0f; omv[3 * i + 2] = 0.0f;
-      continue;
+  for (Index i = (Index)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (Index)gridDim.x * blockDim.x) {
+    const Index r = i / (Index)nx;
+    const int ix = (int)(i - r * (Index)nx);
+    const int iz = (int)(r / (Index)ny);
+    const int iy = (int)(r - (Index)iz * (Index)ny);
+    float qf = 0.0f, mf = 0.0f, wx = 0.0f, wy = 0.0f, wz = 0.0f;
+    if (!(flags && flags[i] == CELL_SOLID)) {
+      const Index px = (Index)nx, pz = (Index)nx * (Index)ny;
+      const Index xp = ix > 0 ? i - 1 : i, xn = ix + 1 < nx ? i + 1 : i;
+      const Index yp = iy > 0 ? i - px : i, yn = iy + 1 < ny ? i + px : i;
+      const Index zp = iz > 0 ? i - pz : i, zn = iz + 1 < nz ? i + pz : i;
+      // 1 / ((n - p) dx): both neighbours, one, or (a single cell across) none
+      const double sx = (ix > 0) != (ix + 1 < nx) ? inv1dx : inv2dx;
+      const double sy = (iy > 0) != (iy + 1 < ny) ? inv1dx : inv2dx;
+      const double sz = (iz > 0) != (iz + 1 < nz) ? inv1dx : inv2dx;
+      const double a = ((double)ux[xn] - (double)ux[xp]) * sx;
+      const double b = ((double)ux[yn] - (double)ux[yp]) * sy;
+      const double c = ((double)ux[zn] - (double)ux[zp]) * sz;
+      const double d = ((double)uy[xn] - (double)uy[xp]) * sx;
+      const double e = ((double)uy[yn] - (double)uy[yp]) * sy;
+      const double f = ((double)uy[zn] - (double)uy[zp]) * sz;
+      const double g = ((double)uz[xn] - (double)uz[xp]) * sx;
+      const double h = ((double)uz[yn] - (double)uz[yp]) * sy;
+      const double k = ((double)uz[zn] - (double)uz[zp]) * sz;
+      const double S12 = 0.5 * (b + d), S13 = 0.5 * (c + g), S23 = 0.5 * (f + h);
+      const double nS = a * a + e * e + k * k + 2.0 * (S12 * S12 + S13 * S13 + S23 * S23);
+      const double O12 = 0.5 * (b - d), O13 = 0.5 * (c - g), O23 = 0.5 * (f - h);
+      const double nO = 2.0 * (O12 * O12 + O13 * O13 + O23 * O23);
+      const double qv = 0.5 * (nO - nS);
+      if (qv > mq) mq = qv;
+      const double ox = h - f, oy = c - g, oz = d - b;
+      const double m = sqrt(ox * ox + oy * oy + oz * oz);
+      if (m > mo) mo = m;
+      qf = (float)qv;
+      mf = (float)m;
+      wx = (float)ox; wy = (float)oy; wz = (float)oz;
     }
-    const int xp = ix > 0 ? ix - 1 : 0, xn = ix + 1 < nx ? ix + 1 : nx - 1;
-    const int yp = iy > 0 ? iy - 1 : 0, yn = iy + 1 < ny ? iy + 1 : ny - 1;
-    const int zp = iz > 0 ? iz - 1 : 0, zn = iz + 1 < nz ? iz + 1 : nz - 1;
-    const double sx = xn > xp ? 1.0 / ((xn - xp) * dx) : inv2dx;
-    const double sy = yn > yp ? 1.0 / ((yn - yp) * dx) : inv2dx;
-    const double sz = zn > zp ? 1.0 / ((zn - zp) * dx) : inv2dx;
-    const double a = ((double)ux[at(xn, iy, iz)] - (double)ux[at(xp, iy, iz)]) * sx;
-    const double b = ((double)ux[at(ix, yn, iz)] - (double)ux[at(ix, yp, iz)]) * sy;
-    const double c = ((double)ux[at(ix, iy, zn)] - (double)ux[at(ix, iy, zp)]) * sz;
-    const double d = ((double)uy[at(xn, iy, iz)] - (double)uy[at(xp, iy, iz)]) * sx;
-    const double e = ((double)uy[at(ix, yn, iz)] - (double)uy[at(ix, yp, iz)]) * sy;
-    const double f = ((double)uy[at(ix, iy, zn)] - (double)uy[at(ix, iy, zp)]) * sz;
-    const double g = ((double)uz[at(xn, iy, iz)] - (double)uz[at(xp, iy, iz)]) * sx;
-    const double h = ((double)uz[at(ix, yn, iz)] - (double)uz[at(ix, yp, iz)]) * sy;
-    const double k = ((double)uz[at(ix, iy, zn)] - (double)uz[at(ix, iy, zp)]) * sz;
-    const double S12 = 0.5 * (b + d), S13 = 0.5 * (c + g), S23 = 0.5 * (f + h);
-    const double nS = a * a + e * e + k * k + 2.0 * (S12 * S12 + S13 * S13 + S23 * S23);
-    const double O12 = 0.5 * (b - d), O13 = 0.5 * (c - g), O23 = 0.5 * (f - h);
-    const double nO = 2.0 * (O12 * O12 + O13 * O13 + O23 * O23);
-    const double qv = 0.5 * (nO - nS);
-    q[i] = (float)qv;
-    if (qv > mq) mq = qv;
-    const double ox = h - f, oy = c - g, oz = d - b;
-    const double m = sqrt(ox * ox + oy * oy + oz * oz);
-    omv[3 * i] = (float)ox; omv[3 * i + 1] = (float)oy; omv[3 * i + 2] = (float)oz;
-    om[i] = (float)m;
-    if (m > mo) mo = m;
+    q[i] = qf;
+    om[i] = mf;
+    float* const w = omv + 3 * (size_t)i;
+    w[0] = wx; w[1] = wy; w[2] = wz;
   }
-  atomicMax(&maxima[0], (unsigned long long)__double_as_longlong(mq));
-  atomicMax(&maxima[1], (unsigned long long)__double_as_longlong(mo));
+  // maxima of non-negative numbers (a NaN never enters: the comparisons above are false)
+  __shared__ double s_q[8], s_o[8];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    mq = fmax(mq, __shfl_down_sync(0xffffffffu, mq, o));
+    mo = fmax(mo, __shfl_down_sync(0xffffffffu, mo, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    s_q[threadIdx.x >> 5] = mq;
+    s_o[threadIdx.x >> 5] = mo;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    const double* const s = threadIdx.x ? s_o : s_q;
+    double m = s[0];
+    for (int w = 1; w < 8; ++w) m = fmax(m, s[w]);
+    atomicMax(&maxima[threadIdx.x], (unsigned long long)__double_as_longlong(m));
+  }
 }
 
 }  // namespace aerosim

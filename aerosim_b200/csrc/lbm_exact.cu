@@ -175,7 +175,10 @@ cudaError_t launch_q_criterion(int nx, int ny, int nz, double dx, const float* u
   cudaError_t e = cudaMemsetAsync(maxima, 0, 2 * sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
   const int grid = (int)std::min<long long>((N + 255) / 256, 148 * 8);
-  q_criterion_kernel<<<grid, 256, 0, s>>>(nx, ny, nz, dx, ux, uy, uz, flags, q, om, omv, maxima);
+  if (N < (1LL << 31))  // the grid stride stays far below 2^31, so a 32-bit index cannot wrap
+    q_criterion_kernel<uint32_t><<<grid, 256, 0, s>>>(nx, ny, nz, dx, ux, uy, uz, flags, q, om, omv, maxima);
+  else
+    q_criterion_kernel<unsigned long long><<<grid, 256, 0, s>>>(nx, ny, nz, dx, ux, uy, uz, flags, q, om, omv, maxima);
   return cudaGetLastError();
 }
 
