@@ -7,6 +7,7 @@ Translation units and their floating-point contracts:
   lbm_fast_<s>.cu  FP32-arithmetic step kernels per storage type, FMA contraction allowed
   lbm_exact.cu  FP64 kernels mirroring the reference's rounding: -fmad=false
   voxelize.cu   FP64 BVH voxelizer, bit-exact flags and links: -fmad=false
+  near_links.cu near-wall cells of a voxel grid and their link tables, grid memory: -fmad=false
   engine.cu     C-ABI host layer
   noalloc.cu    allocation-free force reduction entry point: -fmad=false
   sgs.cu        learned SGS closure: MLP training, wall distance, training samples
@@ -39,6 +40,7 @@ UNITS = {
     "lbm_fast_f16c.cu": [],
     "lbm_exact.cu": ["-fmad=false"],
     "voxelize.cu": ["-fmad=false"],
+    "near_links.cu": ["-fmad=false"],
     "engine.cu": [],
     "noalloc.cu": ["-fmad=false"],
     "sgs.cu": [],

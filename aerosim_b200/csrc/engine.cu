@@ -45,10 +45,13 @@ struct aerosim_engine {
   int occupancy = 0;
   int num_sms = 148;
   float *mux = nullptr, *muy = nullptr, *muz = nullptr, *mrho = nullptr;
-  int32_t* near_cells = nullptr;  // near-wall cells and their link table
-  NearLink* links = nullptr;
-  NearLinkF* links_f = nullptr;  // compact table of the FP32-arithmetic kernels
-  long long n_near = 0;
+  NearTable near;                 // near-wall cells and their link tables
+  // The arrays of the grid before the current one, of the same lattice size: the next
+  // voxelization (a body turned or moved in its tunnel) builds into them instead of
+  // allocating (6 bytes a cell against 152 of FP32 populations).  Given back when the
+  // lattice changes, when memory runs out and with the engine.
+  DevGrid spare;
+  VoxScratch vox;
   double* abl = nullptr;
   double* sin_tab = nullptr;
   int tab_ny = 0;
@@ -101,9 +104,18 @@ int fail(aerosim_engine* h, int code, const std::string& msg) {
                   std::string(#x) + ": " + cudaGetErrorString(e_));                       \
   } while (0)
 
-void free_grid(DevGrid& g) {
-  cudaFree(g.flags); cudaFree(g.cls); cudaFree(g.bmap); cudaFree(g.bcells);
-  cudaFree(g.q); cudaFree(g.minq);
+// A grid to build into: the spare arrays, if there are any.
+DevGrid take_spare(aerosim_engine* h) {
+  DevGrid g;
+  std::swap(g, h->spare);
+  return g;
+}
+void give_spare(aerosim_engine* h, DevGrid& g) {
+  grid_free(&h->spare);
+  h->spare.cell_mem = g.cell_mem;
+  h->spare.cell_cap = g.cell_cap;
+  h->spare.list_mem = g.list_mem;
+  h->spare.list_cap = g.list_cap;
   g = DevGrid();
 }
 
@@ -220,19 +232,32 @@ int configure_step(aerosim_engine* h) {
   return AEROSIM_OK;
 }
 
+cudaError_t alloc_pops(aerosim_engine* h) {
+  const size_t N = (size_t)h->g.N, eb = precision_bytes(h->cfg.precision);
+  cudaError_t e = cudaMalloc(&h->f[0], 19 * (size_t)h->L.plane * eb);
+  if (e == cudaSuccess) e = cudaMalloc(&h->f[1], 19 * (size_t)h->L.plane * eb);
+  if (e == cudaSuccess) e = cudaMalloc(&h->mux, N * sizeof(float));
+  if (e == cudaSuccess) e = cudaMalloc(&h->muy, N * sizeof(float));
+  if (e == cudaSuccess) e = cudaMalloc(&h->muz, N * sizeof(float));
+  if (e == cudaSuccess) e = cudaMalloc(&h->mrho, N * sizeof(float));
+  return e;
+}
+
 // Allocates population and macro buffers for the current grid and precision.
 int ensure_pops(aerosim_engine* h, bool* reallocated) {
   *reallocated = false;
   const long long N = h->g.N;
   if (h->f[0] && h->f_prec == h->cfg.precision && h->f_cells == N) return configure_step(h);
   free_pops(h);
-  const size_t eb = precision_bytes(h->cfg.precision);
-  CU(h, cudaMalloc(&h->f[0], 19 * (size_t)h->L.plane * eb));
-  CU(h, cudaMalloc(&h->f[1], 19 * (size_t)h->L.plane * eb));
-  CU(h, cudaMalloc(&h->mux, N * sizeof(float)));
-  CU(h, cudaMalloc(&h->muy, N * sizeof(float)));
-  CU(h, cudaMalloc(&h->muz, N * sizeof(float)));
-  CU(h, cudaMalloc(&h->mrho, N * sizeof(float)));
+  cudaError_t e = alloc_pops(h);
+  if (e == cudaErrorMemoryAllocation && (h->spare.cell_mem || h->vox.dev)) {  // once more without what is kept for later
+    cudaGetLastError();
+    free_pops(h);
+    grid_free(&h->spare);
+    h->vox.release();
+    e = alloc_pops(h);
+  }
+  CU(h, e);
   h->f_prec = h->cfg.precision;
   h->f_cells = N;
   *reallocated = true;
@@ -283,97 +308,20 @@ int install_grid(aerosim_engine* h, DevGrid& ng, double dx, const double origin[
     if (rc) return rc;
   }
   const Layout nl = make_layout(ng.nx, ng.ny, ng.nz);
-  CU(h, cudaMalloc(&ng.cls, std::max<long long>((long long)ng.ny * ng.nz * nl.pitch, 1)));
+  if ((long long)19 * nl.plane >= (1LL << 32))
+    return fail(h, AEROSIM_ERR_ARG, "lattice too large for 32-bit population offsets");
   CU(h, cudaMemsetAsync(ng.cls, CELL_SOLID, (size_t)ng.ny * ng.nz * nl.pitch, h->stream));
   CU(h, launch_classify(ng.flags, ng.cls, nl, h->stream));
-  CU(h, cudaStreamSynchronize(h->stream));
-  {
-    // Near-wall cells (x faces excluded: the inlet and outlet overwrite them) and
-    // their link table: for each direction, how the reference's pull obtains the
-    // value (lbmCpuReference.ts:189-224), resolved once per voxel grid.
-    const long long N = ng.N;
-    std::vector<uint8_t> cls((size_t)ng.ny * ng.nz * nl.pitch);
-    std::vector<int32_t> bmap(N);
-    std::vector<float> q((size_t)std::max<long long>(ng.B, 1) * 18);
-    // (the table is rebuilt with every voxel grid; the layout nl decides the offsets)
-    CU(h, cudaMemcpy(cls.data(), ng.cls, cls.size(), cudaMemcpyDeviceToHost));
-    CU(h, cudaMemcpy(bmap.data(), ng.bmap, N * 4, cudaMemcpyDeviceToHost));
-    if (ng.B > 0) CU(h, cudaMemcpy(q.data(), ng.q, ng.B * 18 * 4, cudaMemcpyDeviceToHost));
-    auto flag_at = [&](int x, int y, int z) {
-      return cls[((size_t)y + (size_t)ng.ny * z) * nl.pitch + x] & CLS_FLAG_MASK;
-    };
-    auto clampi_h = [](int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); };
-    std::vector<int32_t> nearv;
-    for (int iz = 0; iz < ng.nz; ++iz)
-      for (int iy = 0; iy < ng.ny; ++iy) {
-        const long long row = iy + (long long)ng.ny * iz;
-        for (int ix = 1; ix < ng.nx - 1; ++ix)
-          if (cls[row * nl.pitch + ix] & CLS_NEAR) nearv.push_back((int32_t)(row * ng.nx + ix));
-      }
-    const long long nn = (long long)nearv.size();
-    if ((long long)19 * nl.plane >= (1LL << 32))
-      return fail(h, AEROSIM_ERR_ARG, "lattice too large for 32-bit population offsets");
-    auto off = [&](int d, long long c) -> uint32_t { return (uint32_t)nl.at(d, c); };
-    std::vector<NearLink> links(19 * std::max<long long>(nn, 1));
-    for (long long t = 0; t < nn; ++t) {
-      const long long cell = nearv[t];
-      const int ix = (int)(cell % ng.nx);
-      const long long row = cell / ng.nx;
-      const int iy = (int)(row % ng.ny), iz = (int)(row / ng.ny);
-      const int flag = flag_at(ix, iy, iz);
-      const int bi = flag == CELL_BOUNDARY ? bmap[cell] : -1;
-      for (int d = 0; d < 19; ++d) {
-        NearLink& L = links[(size_t)d * nn + t];
-        const int sx = clampi_h(ix - cx_of(d), 0, ng.nx - 1), sy = clampi_h(iy - cy_of(d), 0, ng.ny - 1),
-                  sz = clampi_h(iz - cz_of(d), 0, ng.nz - 1);
-        const long long src = sx + (long long)ng.nx * (sy + (long long)ng.ny * sz);
-        L.A = 1.0; L.B = 0.0;
-        if (d > 0 && flag_at(sx, sy, sz) == CELL_SOLID) {
-          // Bouzidi in the pull, lbmCpuReference.ts:196-221
-          const int wd = opp_of(d);
-          const double qv = bi >= 0 ? (double)q[(size_t)bi * 18 + (wd - 1)] : 0.5;
-          const double qe = qv > 0.0 ? qv : 0.5;
-          const int fx = clampi_h(ix + cx_of(d), 0, ng.nx - 1), fy = clampi_h(iy + cy_of(d), 0, ng.ny - 1),
-                    fz = clampi_h(iz + cz_of(d), 0, ng.nz - 1);
-          const long long ff = fx + (long long)ng.nx * (fy + (long long)ng.ny * fz);
-          L.o1 = off(wd, cell); L.d1 = wd;
-          L.o2 = L.o1; L.d2 = wd;
-          if (flag_at(fx, fy, fz) != CELL_SOLID) {
-            if (qe < 0.5) {
-              L.A = 2.0 * qe; L.B = 1.0 - 2.0 * qe;
-              L.o2 = off(wd, ff); L.d2 = wd;
-            } else {
-              const double inv2q = 1.0 / (2.0 * qe);
-              L.A = inv2q; L.B = 1.0 - inv2q;
-              L.o2 = off(d, cell); L.d2 = d;
-            }
-          }
-        } else {
-          L.o1 = off(d, src); L.d1 = d;
-          L.o2 = L.o1; L.d2 = d;
-        }
-      }
-    }
-    std::vector<NearLinkF> links_f(links.size());
-    for (size_t i = 0; i < links.size(); ++i)
-      links_f[i] = NearLinkF{links[i].o1, links[i].o2, (float)links[i].A, (float)links[i].B};
-    cudaFree(h->near_cells); cudaFree(h->links); cudaFree(h->links_f);
-    h->near_cells = nullptr; h->links = nullptr; h->links_f = nullptr;
-    h->n_near = nn;
-    CU(h, cudaMalloc(&h->near_cells, std::max<long long>(nn, 1) * 4));
-    CU(h, cudaMalloc(&h->links, links.size() * sizeof(NearLink)));
-    CU(h, cudaMalloc(&h->links_f, links_f.size() * sizeof(NearLinkF)));
-    if (nn) CU(h, cudaMemcpy(h->near_cells, nearv.data(), nn * 4, cudaMemcpyHostToDevice));
-    CU(h, cudaMemcpy(h->links, links.data(), links.size() * sizeof(NearLink), cudaMemcpyHostToDevice));
-    CU(h, cudaMemcpy(h->links_f, links_f.data(), links_f.size() * sizeof(NearLinkF), cudaMemcpyHostToDevice));
-  }
+  CU(h, build_near_table(ng, nl, &h->vox, h->stream, &h->near));
   h->wall_ready = false;
   if (h->mlp_frag) {  // the learned closure reads wall distances from the class bytes
     CU(h, compute_wall_distance(ng.flags, ng.nx, ng.ny, ng.nz, nullptr, ng.cls, nl.pitch, h->stream));
     h->wall_ready = true;
   }
+  const bool same = h->have_grid && nl.nx == h->L.nx && nl.ny == h->L.ny && nl.nz == h->L.nz;
   if (h->f[0] && (nl.pitch != h->L.pitch || nl.plane != h->L.plane)) free_pops(h);
-  free_grid(h->g);
+  if (same) give_spare(h, h->g);
+  else grid_free(&h->g);
   h->g = ng;
   h->L = nl;
   ng = DevGrid();
@@ -480,10 +428,13 @@ int aerosim_destroy(aerosim_engine* h) {
   if (!h) return AEROSIM_OK;
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
-  free_grid(h->g);
+  grid_free(&h->g);
+  grid_free(&h->spare);
+  h->vox.release();
+  if (h->vox.host) cudaFreeHost(h->vox.host);
+  near_free(&h->near);
   free_pops(h);
   cudaFree(h->abl); cudaFree(h->sin_tab); cudaFree(h->st);
-  cudaFree(h->near_cells); cudaFree(h->links); cudaFree(h->links_f);
   cudaFree(h->force_partials); cudaFree(h->force_ticket); cudaFree(h->force_out);
   cudaFree(h->stats_buf); cudaFree(h->staging);
   if (h->frame_host) cudaFreeHost(h->frame_host);
@@ -512,18 +463,19 @@ int aerosim_voxelize(aerosim_engine* h, const float* positions, int64_t vertex_c
   }
   if (!(tunnel.height > 0)) return fail(h, AEROSIM_ERR_ARG, "aerosim_voxelize: tunnel height must be > 0");
   CU(h, cudaSetDevice(h->device));
-  DevGrid ng;
+  DevGrid ng = take_spare(h);
   std::string e;
   const int rc = run_voxelizer(positions, vertex_count, indices, index_count, world16, tunnel.height, nx, ny,
-                               nz, h->stream, &ng, &e);
+                               nz, h->stream, &h->vox, &ng, &e);
   if (rc) {
-    free_grid(ng);
+    grid_free(&ng);
     return fail(h, rc == -4 ? AEROSIM_ERR_DEVICE : AEROSIM_ERR_CUDA, e);
   }
   const double origin[3] = {ng.ox, ng.oy, ng.oz};
   const double dx = ng.h;
   const int r2 = install_grid(h, ng, dx, origin, reset_flow);
-  free_grid(ng);
+  grid_free(&ng);
+  h->vox.trim();
   if (r2) return r2;
   h->cfg.tunnel = tunnel;
   return aerosim_get_voxel_info(h, out);
@@ -589,22 +541,19 @@ int aerosim_set_voxel_grid(aerosim_engine* h, int32_t nx, int32_t ny, int32_t nz
   for (int64_t b = 0; b < B; ++b)
     if (bcells[b] < 0 || bcells[b] >= N) return fail(h, AEROSIM_ERR_ARG, "set_voxel_grid: boundary cell out of range");
   CU(h, cudaSetDevice(h->device));
-  DevGrid ng;
+  DevGrid ng = take_spare(h);
   ng.nx = nx; ng.ny = ny; ng.nz = nz; ng.N = N; ng.h = dx;
   ng.ox = origin ? origin[0] : -nx * dx * 0.5;
   ng.oy = origin ? origin[1] : -ny * dx * 0.5;
   ng.oz = origin ? origin[2] : -nz * dx * 0.5;
   ng.B = B; ng.solid = solid;
   auto bad = [&](cudaError_t e) {
-    free_grid(ng);
+    grid_free(&ng);
     return fail(h, AEROSIM_ERR_CUDA, std::string("set_voxel_grid: ") + cudaGetErrorString(e));
   };
   cudaError_t e;
-  if ((e = cudaMalloc(&ng.flags, N)) != cudaSuccess) return bad(e);
-  if ((e = cudaMalloc(&ng.bmap, N * 4)) != cudaSuccess) return bad(e);
-  if ((e = cudaMalloc(&ng.bcells, std::max<int64_t>(B, 1) * 4)) != cudaSuccess) return bad(e);
-  if ((e = cudaMalloc(&ng.q, std::max<int64_t>(B, 1) * 18 * 4)) != cudaSuccess) return bad(e);
-  if ((e = cudaMalloc(&ng.minq, std::max<int64_t>(B, 1) * 4)) != cudaSuccess) return bad(e);
+  if ((e = grid_cells(&ng, N, (size_t)make_layout(nx, ny, nz).plane)) != cudaSuccess) return bad(e);
+  if ((e = grid_lists(&ng, B)) != cudaSuccess) return bad(e);
   std::vector<float> mq(std::max<int64_t>(B, 1), 1.0f);
   for (int64_t b = 0; b < B; ++b)
     for (int k = 0; k < 18; ++k) {
@@ -620,7 +569,7 @@ int aerosim_set_voxel_grid(aerosim_engine* h, int32_t nx, int32_t ny, int32_t nz
   }
   const double org[3] = {ng.ox, ng.oy, ng.oz};
   const int rc = install_grid(h, ng, dx, org, reset_flow);
-  free_grid(ng);
+  grid_free(&ng);
   return rc;
 }
 
@@ -669,9 +618,9 @@ int enqueue_steps(aerosim_engine* h, int32_t n) {
   a.mux = h->mux; a.muy = h->muy; a.muz = h->muz; a.mrho = h->mrho;
   a.abl = h->abl; a.sin_tab = h->sin_tab; a.st = h->st;
   a.L = h->L; a.fluid_count = h->fluid_count;
-  a.near_cells = h->near_cells; a.n_near = h->n_near;
-  a.links = h->links;
-  a.links_f = h->links_f;
+  a.near_cells = h->near.cells; a.n_near = h->near.n;
+  a.links = h->near.links;
+  a.links_f = h->near.links_f;
   a.stages = h->stages;
   a.ground_no_slip = h->cfg.ground_no_slip;
   a.u_inlet = h->cfg.u_inlet_lattice;
@@ -1293,7 +1242,7 @@ int batch_upload_table(aerosim_batch* b) {
     a.mux = e->mux; a.muy = e->muy; a.muz = e->muz; a.mrho = e->mrho;
     a.abl = e->abl; a.sin_tab = e->sin_tab; a.st = e->st;
     a.L = e->L; a.fluid_count = e->fluid_count;
-    a.near_cells = e->near_cells; a.n_near = e->n_near; a.links = e->links; a.links_f = e->links_f;
+    a.near_cells = e->near.cells; a.n_near = e->near.n; a.links = e->near.links; a.links_f = e->near.links_f;
     a.ground_no_slip = e->cfg.ground_no_slip;
     a.u_inlet = e->cfg.u_inlet_lattice;
     a.tau0 = 3.0 * e->cfg.nu_lattice + 0.5;
@@ -1500,7 +1449,7 @@ int aerosim_batch_create(aerosim_engine* const* engines, int32_t n, aerosim_batc
   for (int k = 0; k < n; ++k) {
     const aerosim_engine* en = engines[k];
     const Layout& L = en->L;
-    near_begin[k + 1] = near_begin[k] + en->n_near;
+    near_begin[k + 1] = near_begin[k] + en->near.n;
     bufs[2 * k] = en->f[0];
     bufs[2 * k + 1] = en->f[1];
     b->cells += en->g.N;

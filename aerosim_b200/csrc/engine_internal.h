@@ -11,7 +11,9 @@ struct StepArgs;
 struct ForceArgs;
 struct BatchArgs;
 
-// A voxel grid resident on the device (VoxelGridResult, voxelizer.ts:19-59).
+// A voxel grid resident on the device (VoxelGridResult, voxelizer.ts:19-59).  The arrays of
+// one size class share an allocation: flags, cls and bmap (per cell), bcells, q and minq
+// (per boundary cell); a grid built into arrays that are large enough allocates nothing.
 struct DevGrid {
   int nx = 0, ny = 0, nz = 0;
   long long N = 0;
@@ -25,12 +27,48 @@ struct DevGrid {
   long long B = 0, solid = 0;
   int window[6] = {0, 0, 0, 0, 0, 0};
   double vox_ms = 0;
+  void *cell_mem = nullptr, *list_mem = nullptr;
+  size_t cell_cap = 0, list_cap = 0;
 };
+// Arrays for N cells (cls_bytes of classes), and lists for B boundary cells.
+cudaError_t grid_cells(DevGrid* g, long long N, size_t cls_bytes);
+cudaError_t grid_lists(DevGrid* g, long long B);
+void grid_free(DevGrid* g);
+
+// Scratch of a voxelization, kept by the engine between calls: device memory, and a few
+// words of pinned memory that results come back through.
+struct VoxScratch {
+  void* dev = nullptr;
+  size_t bytes = 0;
+  unsigned long long* host = nullptr;  // pinned [32]
+  cudaError_t device(size_t n);        // at least n bytes
+  cudaError_t pinned();
+  void trim();     // gives back device memory above 64 MB
+  void release();
+};
+
+// Near-wall cells of a grid (x faces excluded: the inlet and outlet overwrite them) and
+// their link tables, in one allocation that is reused while it is large enough.
+struct NearLink;
+struct NearLinkF;
+struct NearTable {
+  int32_t* cells = nullptr;
+  NearLink* links = nullptr;
+  NearLinkF* links_f = nullptr;
+  long long n = 0;
+  void* mem = nullptr;
+  size_t cap = 0;
+};
+cudaError_t build_near_table(const DevGrid& g, const Layout& L, VoxScratch* w, cudaStream_t s, NearTable* t);
+void near_free(NearTable* t);
+
+// Exclusive scan of n row counts in place; the total to *total (device or mapped).
+cudaError_t launch_scan_rows(uint32_t* counts, long long n, unsigned long long* total, cudaStream_t s);
 
 // voxelize.cu
 int run_voxelizer(const float* pos, int64_t nverts, const int32_t* idx, int64_t nidx,
                   const double* world16, double tunnel_height, int nx, int ny, int nz,
-                  cudaStream_t s, DevGrid* g, std::string* err);
+                  cudaStream_t s, VoxScratch* w, DevGrid* g, std::string* err);
 
 // Message returned by aerosim_last_error(NULL) (calls that take no engine handle).
 void set_global_error(const std::string& msg);
