@@ -135,7 +135,7 @@ struct StoreBF16S {
 // FP16 shifted storage with mass-compensated rounding: the values are those of StoreF16S,
 // but wherever a step kernel stores a cell it rounds the 18 moving populations first and
 // gives the rest population what their rounded values leave of the cell's deviation sum
-// (compensate_cell and its lane form below, and the pair path of pair_segment), i.e. the
+// (compensate_cell and its lane form below, and compensate_pair), i.e. the
 // rest population absorbs their rounding errors before it rounds itself.  The stored
 // deviations of a cell then sum to the computed ones up to the single rounding of f_0,
 // whose half-precision ulp is 4-8 times finer than the moving populations' near

@@ -15,6 +15,7 @@
 #include "engine_internal.h"
 #include "lbm_kernels.cuh"
 #include "lbm_batch.cuh"
+#include "lbm_pair_step.cuh"
 #include "sgs_mlp.cuh"
 
 using namespace aerosim;
@@ -41,6 +42,7 @@ struct aerosim_engine {
   int stages = 3;
   int item_groups = 1;  // row groups per work item of the step kernel
   int cells_per_thread = 1;  // consumer cells per thread of the step kernel (1 or 2)
+  int item_rows = 1;         // two cells per thread: x-rows per work item
   int dynamic_items = 1;     // work items from a device counter (1) or dealt round-robin (0)
   int occupancy = 0;
   int num_sms = 148;
@@ -166,7 +168,6 @@ const uint4* closure_umma(const aerosim_engine* h) {
 int configure_step(aerosim_engine* h) {
   const Layout& L = h->L;
   const size_t eb = precision_bytes(h->cfg.precision);
-  const dim3 block(kStepThreads, 1, 1);
   StepArgs dummy{};
   dummy.L = L;  // the kernel instance depends on the row pitch and the closure
   dummy.mlp_frag = h->mlp_frag;
@@ -188,24 +189,38 @@ int configure_step(aerosim_engine* h) {
     if (want == 2 && fast && pairs_fit) cpt = 2;
   }
   dummy.cells_per_thread = cpt;
+  const dim3 block(cpt == 2 ? kPairThreads : kStepThreads, 1, 1);
   const bool grouped = !mlp && half;
-  int groups = grouped ? item_groups_for(L.nx, cpt) : 1;
+  int groups = grouped ? item_groups_for(L.nx) : 1;
   if (const char* genv = getenv("AEROSIM_ITEM_GROUPS")) {  // override of the row groups per item (1..4)
     const int want = atoi(genv);
     if (grouped && want >= 1 && want <= 4) groups = want;
   }
+  // two cells per thread: items of about 384 pairs with 16-bit storage and 192 with FP32, in
+  // up to 3 and 4 ring slots (256x128x128 F16S: 256 pairs 61.1-63.2 us per step, 384 60.3, 512
+  // 60.6; 128x64x64 FP32: 128 pairs 17.8, 192 16.5, 256 16.8)
+  const long long all_rows = (long long)L.ny * L.nz;
+  int item_rows = 1;
+  if (cpt == 2) {
+    item_rows = pair_rows(L.nx, all_rows, half ? 384 : 192, 2LL * h->num_sms);
+    if (const char* ienv = getenv("AEROSIM_ITEM_GROUPS"))  // rows per item by hand, in units of 256 cells
+      item_rows = std::min(kMaxPairRows, std::max(1, atoi(ienv) * 256 / L.nx));
+  }
+  auto smem_for = [&](int S) {
+    return cpt == 2 ? pair_smem_bytes(L.pitch, L.ny, item_rows, S, eb) : step_smem_bytes(L, S, eb, mlp, groups);
+  };
   const char* env = getenv("AEROSIM_STAGES");
   const int forced = env ? atoi(env) : 0;
   int best_s = 0, best_occ = 0;
   for (int S = 2; S <= 8; ++S) {
     if (forced && S != forced) continue;
-    const size_t smem = step_smem_bytes(L, S, eb, mlp, groups, cpt);
+    const size_t smem = smem_for(S);
     if (smem > 227 * 1024) break;
     int occ = 0;
     cudaError_t e = launch_step(h->cfg.precision, dummy, block, 0, smem, h->stream, &occ, nullptr);
     if (e != cudaSuccess || occ < 1) break;
     // keep deepening the ring while the residency does not drop
-    if (best_s == 0 || (occ >= best_occ && S <= 4)) {
+    if (best_s == 0 || (occ >= best_occ && S <= (cpt == 2 && half ? 3 : 4))) {
       best_s = S;
       best_occ = occ;
     }
@@ -213,7 +228,8 @@ int configure_step(aerosim_engine* h) {
   if (best_s == 0) return fail(h, AEROSIM_ERR_ARG, "step kernel: no launch configuration fits shared memory");
   h->block = block;
   h->stages = best_s;
-  h->smem = step_smem_bytes(L, best_s, eb, mlp, groups, cpt);
+  h->smem = smem_for(best_s);
+  h->item_rows = item_rows;
   h->item_groups = groups;
   h->cells_per_thread = cpt;
   // work items from the step's counter (108.8 vs 115.8 us FP32 with one cell per thread):
@@ -222,8 +238,8 @@ int configure_step(aerosim_engine* h) {
   // the occupancy of the chosen configuration
   CU(h, launch_step(h->cfg.precision, dummy, block, 0, h->smem, h->stream, &best_occ, nullptr));
   h->occupancy = best_occ;
-  const long long item_rows = (long long)rows_per_item(L.nx, cpt) * groups;
-  const long long items = ((long long)L.ny * L.nz + item_rows - 1) / item_rows;
+  const long long per_item = cpt == 2 ? item_rows : (long long)rows_per_item(L.nx) * groups;
+  const long long items = (all_rows + per_item - 1) / per_item;
   long long grid = (long long)best_occ * h->num_sms;
   const char* genv = getenv("AEROSIM_CTAS_PER_SM");
   if (genv && atoi(genv) > 0 && atoi(genv) <= best_occ) grid = (long long)atoi(genv) * h->num_sms;
@@ -634,6 +650,8 @@ int enqueue_steps(aerosim_engine* h, int32_t n) {
   a.item_groups = h->item_groups;
   a.cells_per_thread = h->cells_per_thread;
   a.dynamic_items = h->dynamic_items;
+  a.item_rows = h->item_rows;
+  a.pair_magic = pair_magic(std::max(1, h->L.nx / 2));
   a.wait_limit = h->wait_limit;
   long long launches = 0;
   CU(h, cudaEventRecord(h->ev0, h->stream));
@@ -1184,12 +1202,15 @@ struct aerosim_batch {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   StepArgs* d_inst = nullptr;
+  PairInst* d_pair = nullptr;
   void** d_bufs = nullptr;
   long long* d_item_begin = nullptr;
   long long* d_near_begin = nullptr;
   int4* d_geo = nullptr;
   unsigned long long* d_partials = nullptr;
-  unsigned int* d_ticket = nullptr;  // [2]
+  unsigned int* d_ticket = nullptr;  // [4]: CTAs done, then next item, per step parity
+  std::vector<long long> item_begin;  // the flat item list: first item and rows per item of each instance
+  std::vector<int> item_rows;
   int* d_step = nullptr;
   int* d_error = nullptr;
   long long n_items = 0, n_near = 0, cells = 0;
@@ -1206,7 +1227,7 @@ struct aerosim_batch {
   double last_ms = 0;
   long long last_launches = 0;
   int wait_limit = kWaitLimit;  // polls of a ring wait before the batched step gives up
-  int cells_per_thread = 1;     // 2 when every instance has an even nx (pair_segment)
+  int cells_per_thread = 1;     // 2 when every instance has an even nx (batch_pair_kernel)
 };
 
 namespace {
@@ -1223,7 +1244,7 @@ void batch_free(aerosim_batch* b) {
   cudaSetDevice(b->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
   if (b->graph) cudaGraphExecDestroy(b->graph);
-  cudaFree(b->d_inst); cudaFree(b->d_bufs); cudaFree(b->d_item_begin); cudaFree(b->d_near_begin);
+  cudaFree(b->d_inst); cudaFree(b->d_pair); cudaFree(b->d_bufs); cudaFree(b->d_item_begin); cudaFree(b->d_near_begin);
   cudaFree(b->d_geo);
   cudaFree(b->d_partials); cudaFree(b->d_ticket); cudaFree(b->d_step); cudaFree(b->d_error);
   if (b->ev0) cudaEventDestroy(b->ev0);
@@ -1249,12 +1270,21 @@ int batch_upload_table(aerosim_batch* b) {
     a.k_smag = 18.0 * M_SQRT2 * e->cfg.smagorinsky_cs * e->cfg.smagorinsky_cs;
   }
   BCU(cudaMemcpyAsync(b->d_inst, t.data(), t.size() * sizeof(StepArgs), cudaMemcpyHostToDevice, b->stream));
+  if (b->cells_per_thread == 2) {
+    std::vector<PairInst> p(b->eng.size());
+    for (size_t k = 0; k < b->eng.size(); ++k) {
+      const aerosim_engine* e = b->eng[k];
+      p[k] = PairInst{{e->f[0], e->f[1]}, e->g.cls, e->st, e->L.nx, e->L.nx / 2, e->L.pitch, e->L.ny, e->L.nz, b->item_rows[k],
+                      e->cfg.ground_no_slip, pair_magic(e->L.nx / 2), (float)t[k].tau0, (float)t[k].k_smag, b->item_begin[k]};
+    }
+    BCU(cudaMemcpyAsync(b->d_pair, p.data(), p.size() * sizeof(PairInst), cudaMemcpyHostToDevice, b->stream));
+  }
   return AEROSIM_OK;
 }
 
 BatchArgs batch_args(const aerosim_batch* b, int write_macro) {
   BatchArgs a{};
-  a.inst = b->d_inst; a.bufs = b->d_bufs; a.item_begin = b->d_item_begin; a.near_begin = b->d_near_begin;
+  a.inst = b->d_inst; a.pair = b->d_pair; a.bufs = b->d_bufs; a.item_begin = b->d_item_begin; a.near_begin = b->d_near_begin;
   a.partials = b->d_partials; a.ticket = b->d_ticket; a.step = b->d_step; a.error = b->d_error;
   a.geo = b->d_geo;
   a.n_items = b->n_items; a.n_near = b->n_near; a.slot_elems = b->slot_elems; a.slot_cls = b->slot_cls;
@@ -1279,20 +1309,23 @@ int batch_build_items(aerosim_batch* b, int item_cells) {
   const int n = (int)b->eng.size();
   std::vector<long long> item_begin(n + 1, 0);
   std::vector<int4> geo(n);
+  std::vector<int> rows_of(n);
   long long slot_elems = 0, slot_cls = 0;
   for (int k = 0; k < n; ++k) {
     const Layout& L = b->eng[k]->L;
     const int RY = batch_rows_per_item(L, item_cells);
     const long long rows = (long long)L.ny * L.nz;
     item_begin[k + 1] = item_begin[k] + (rows + RY - 1) / RY;
-    geo[k] = b->cells_per_thread == 2 ? make_int4(RY, (L.nx + 63) / 64, 0, 0)  // 64-cell pair segments
-                                      : make_int4(RY, (L.nx + row_shift(L.nx) + 31) / 32, row_shift(L.nx), 0);
+    geo[k] = make_int4(RY, (L.nx + row_shift(L.nx) + 31) / 32, row_shift(L.nx), 0);
+    rows_of[k] = RY;
     slot_elems = std::max<long long>(slot_elems, (long long)RY * 19 * L.pitch);
     slot_cls = std::max<long long>(slot_cls, (long long)RY * L.pitch);
   }
   BCU(cudaMemcpy(b->d_item_begin, item_begin.data(), item_begin.size() * sizeof(long long), cudaMemcpyHostToDevice));
   BCU(cudaMemcpy(b->d_geo, geo.data(), geo.size() * sizeof(int4), cudaMemcpyHostToDevice));
   b->n_items = item_begin[n];
+  b->item_begin = item_begin;
+  b->item_rows = rows_of;
   b->slot_elems = slot_elems;
   b->slot_cls = slot_cls;
   b->item_cells = item_cells;
@@ -1309,7 +1342,8 @@ int batch_configure(aerosim_batch* b, const aerosim_batch_tuning& t, unsigned* g
     if (rc) return rc;
   }
   const size_t eb = precision_bytes(b->precision);
-  const size_t sm = batch_smem_bytes(b->slot_elems, b->slot_cls, t.stages, eb);
+  const size_t sm = b->cells_per_thread == 2 ? batch_pair_smem_bytes(b->slot_elems, b->slot_cls, t.stages, eb)
+                                             : batch_smem_bytes(b->slot_elems, b->slot_cls, t.stages, eb);
   if (sm > 227 * 1024) return bfail(AEROSIM_ERR_ARG, "batch: the ring does not fit shared memory");
   BatchArgs a = batch_args(b, 0);
   a.stages = t.stages;
@@ -1354,7 +1388,7 @@ int batch_reset(aerosim_batch* b) {
   }
   BCU(cudaSetDevice(b->device));
   BCU(cudaMemsetAsync(b->d_step, 0, sizeof(int), b->stream));
-  BCU(cudaMemsetAsync(b->d_ticket, 0, 2 * sizeof(unsigned int), b->stream));
+  BCU(cudaMemsetAsync(b->d_ticket, 0, 4 * sizeof(unsigned int), b->stream));
   BCU(cudaMemsetAsync(b->d_error, 0, sizeof(int), b->stream));
   BCU(cudaStreamSynchronize(b->stream));
   b->step = 0;
@@ -1462,12 +1496,13 @@ int aerosim_batch_create(aerosim_engine* const* engines, int32_t n, aerosim_batc
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
   if (e == cudaSuccess) e = cudaMalloc(&b->d_inst, n * sizeof(StepArgs));
+  if (e == cudaSuccess) e = cudaMalloc(&b->d_pair, n * sizeof(PairInst));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_bufs, 2 * n * sizeof(void*));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_item_begin, (n + 1) * sizeof(long long));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_near_begin, (n + 1) * sizeof(long long));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_geo, n * sizeof(int4));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_partials, part * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_ticket, 2 * sizeof(unsigned int));
+  if (e == cudaSuccess) e = cudaMalloc(&b->d_ticket, 4 * sizeof(unsigned int));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_step, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_error, sizeof(int));
   if (e == cudaSuccess)

@@ -1,4 +1,4 @@
-// Batched step kernel: many wind-tunnel instances of uneven lattice sizes advance one
+// Batched step kernels: many wind-tunnel instances of uneven lattice sizes advance one
 // time step in ONE persistent launch.  The items (x-row groups) of all instances form
 // one flat work list; a CTA walks it with the producer / consumer / near-wall warp
 // roles of main_kernel, switching the instance's arguments per item and dealing the
@@ -9,8 +9,22 @@
 // launches can be replayed without changing a kernel argument.
 #pragma once
 #include "lbm_kernels.cuh"
+#include "lbm_pair_step.cuh"
 
 namespace aerosim {
+
+// What the pair kernel needs of an instance, in one place (the step's argument block is
+// spread over 300 bytes): read by the producer and the consumers once per item.
+struct __align__(16) PairInst {
+  void* buf[2];            // populations, by step parity
+  const uint8_t* cls;
+  StepState* st;
+  int nx, np, pitch, ny;
+  int nz, rows_per_item, ground_no_slip;
+  uint32_t magic;
+  float tau0, k_smag;
+  long long item_begin;    // first item in the flat list
+};
 
 constexpr int kMaxBatch = 64;  // instances per batch
 constexpr int kMaxRowsPerItem = kConsumerWarps;
@@ -22,7 +36,8 @@ struct BatchArgs {
   const long long* item_begin;   // [n_inst + 1] first item of each instance in the flat list
   const long long* near_begin;   // [n_inst + 1] first near-wall cell of each instance
   unsigned long long* partials;  // [gridDim.x * n_inst] per-CTA fixed-point density sums
-  unsigned int* ticket;          // [2] CTAs done, per step parity
+  unsigned int* ticket;          // [2] CTAs done, per step parity, then [2] next item (pair kernel)
+  const PairInst* pair;          // [n_inst], for the pair kernel
   const int4* geo;               // [n_inst] rows per item, 32-cell segments per row, row shift
   int* step;                     // step counter shared by all instances
   int* error;                    // pipeline timeout flag of the batch
@@ -53,9 +68,9 @@ __host__ __device__ inline size_t batch_smem_bytes(long long slot_elems, long lo
          kConsumerWarps * 24 * sizeof(float) + 16 + 19 * sizeof(float4) + 19 * sizeof(int);
 }
 
-// CPT: consumer cells per thread, 1 or 2 (pair_segment; every instance with an even nx).
-template <class S, int P, int CPT = 1>
-__global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE_FAST, MLP_NONE, CPT>())
+// One cell per thread: batches with an instance of an odd nx.
+template <class S, int P>
+__global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE_FAST, MLP_NONE>())
     batch_kernel(const __grid_constant__ BatchArgs b) {
   using T = typename S::T;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -242,42 +257,6 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE_FAST, ML
         return make_float2((float)u.x, (float)u.y);
       };
       for (int sg = first; sg < total; sg += kConsumerWarps) {
-        if constexpr (CPT == 2) {
-          // two adjacent cells per lane, 64-cell segments (every instance has an even nx)
-          const int cell_lo = sr * 64;
-          const int2 yz = s_row[s * kMaxRowsPerItem + ry];
-          const int iy = yz.x, iz = yz.y;
-          const T* sp = spop + (size_t)s * b.slot_elems + (size_t)ry * 19 * pitch;
-          const uint8_t* sc = scls + (size_t)s * b.slot_cls + (size_t)ry * pitch;
-          const int x0 = cell_lo + 2 * lane;
-          const bool active = x0 < nx;
-          const int lx = active ? x0 : 0;  // lanes outside the row read cells 0 and 1
-          const uint32_t cls2 = *reinterpret_cast<const uint16_t*>(sc + lx);
-          float2 v[19];
-#pragma unroll
-          for (int d = 0; d < 19; ++d) {
-            const T* q = sp + slot_of(d) * pitch + lx;
-            if (cx_of(d) == 0) v[d] = load_pair<S>(q);
-            else v[d] = make_float2(S::raw(q[-cx_of(d)]), S::raw(q[1 - cx_of(d)]));
-          }
-          if (sg + kConsumerWarps >= total) {  // this warp's last segment of the slot
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[s]);
-          }
-          PairGeom g;
-          g.row = row0 + ry; g.nx = nx; g.ny = ny; g.nz = nz; g.pitch = pitch;
-          g.iy = iy; g.iz = iz; g.x0 = x0; g.cell_lo = cell_lo; g.active = active;
-          g.has_lo = cell_lo == 0;
-          g.has_hi = cell_lo <= nx - 2 && nx - 2 < cell_lo + 64;
-          g.wall_row = (iy == 0 || iy == ny - 1 || (nz > 4 && (iz == 0 || iz == nz - 1)));
-          g.ground_no_slip = ia.ground_no_slip; g.write_macro = b.write_macro;
-          g.c0 = (uint8_t)(cls2 & 0xffu);
-          g.c1 = (uint8_t)(cls2 >> 8);
-          pair_segment<S>(v, fd, g, tau0f, ksmagf, dec, inlet, ia, s_xo + warp * 24, s_dcw, s_dslot, lane,
-                          item_sum, my_nan);
-          for (sr += kConsumerWarps; sr >= segs; sr -= segs) ++ry;
-          continue;
-        }
         const int cell_lo = sr * 32 - shift;
         const int2 yz = s_row[s * kMaxRowsPerItem + ry];
         const int iy = yz.x, iz = yz.y;
@@ -354,6 +333,213 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE_FAST, ML
   __syncthreads();
   if (threadIdx.x == 0) {
     b.ticket[slot ^ 1] = 0u;
+    *b.step = step + 1;
+  }
+}
+
+// Shared memory of the pair kernel's batch form: as pair_smem_bytes, with slots for the
+// largest item, an instance index per slot and no inlet tables.
+__host__ __device__ inline size_t batch_pair_smem_bytes(long long slot_elems, long long slot_cls, int stages, size_t elem) {
+  return kSmemGuard + (size_t)stages * ((size_t)slot_elems * elem + (size_t)slot_cls) + kSmemGuard + 16 * (size_t)stages +
+         19 * sizeof(float4) + kPairWarps * kEndScratch * sizeof(float) + 19 + (size_t)stages * kMaxRowsPerItem + 32;
+}
+
+// One step of a batch with two cells per thread (every instance of an even nx): pair_kernel's
+// roles over the flat item list of all instances.  Items come from a device counter, as in the
+// single lattice; density sums go to the instances' own state, and the last CTA takes every
+// instance's decision.  Launched as a programmatic dependent of the step before it (inside the
+// captured graphs too), so a step's prologue runs while the last CTAs of the step before finish.
+// 12 tunnels of 128x64x64 .. 172x86x86 (8.6 M cells, mixed row pitches): F16S 269 -> 219 us per
+// step, FP32 333 -> 298.  The run-time pitch costs about a quarter of the instructions.
+template <class S, int P>
+__global__ void __launch_bounds__(kPairThreads, 2) batch_pair_kernel(const __grid_constant__ BatchArgs b) {
+  using T = typename S::T;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ unsigned long long s_sum[kMaxBatch];  // this CTA's density sum per instance
+  __shared__ int s_inst[8], s_first[8], s_rows[8];  // item of ring slot s: instance (-1: none left), first row, rows
+  __shared__ int is_last;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int S_ = b.stages;
+  T* const spop = reinterpret_cast<T*>(smem_raw + kSmemGuard);
+  uint8_t* const scls = smem_raw + kSmemGuard + (size_t)S_ * b.slot_elems * sizeof(T);
+  uint64_t* const full = reinterpret_cast<uint64_t*>(scls + (size_t)S_ * b.slot_cls + kSmemGuard);
+  uint64_t* const empty = full + S_;
+  float4* const s_dcw = reinterpret_cast<float4*>((reinterpret_cast<uintptr_t>(empty + S_) + 15) & ~uintptr_t(15));
+  float* const s_xo = reinterpret_cast<float*>(s_dcw + 19);
+  uint8_t* const s_dslot = reinterpret_cast<uint8_t*>(s_xo + kPairWarps * kEndScratch);
+  uint8_t* const s_wall = s_dslot + 19;  // [S_][kMaxRowsPerItem]
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S_; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], kPairWarps);
+    }
+    mbar_fence_init();
+  }
+  for (int k = threadIdx.x; k < b.n_inst; k += blockDim.x) s_sum[k] = 0ull;
+  fill_end_tables(s_dcw, s_dslot);
+  __syncthreads();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+  const int step = *b.step;  // every CTA reads it before the last CTA advances it
+  const int cur = step & 1;  // buffer parity of this step's source populations
+  const int pslot = (step + 1) & 1;
+  const bool reverse = cur != 0;  // odd steps take the items last to first (pair_kernel)
+  bool failed = false;
+
+  if (warp == kPairProducer) {
+    int issued = 0, end_slot = -1, s = 0;
+    uint32_t ph = 0;
+    int k = reverse ? b.n_inst - 1 : 0;  // instance of the last item: the items come in order
+    for (int j = 0;; ++j) {
+      unsigned int t = 0;
+      if (lane == 0) t = atomicAdd(&b.ticket[2 + cur], 1u);
+      t = __shfl_sync(0xffffffffu, t, 0);
+      const bool none = t >= (unsigned long long)b.n_items;
+      if (j >= S_) {
+        const bool ok = mbar_wait(&empty[s], ph ^ 1u, b.wait_limit);
+        if (!__any_sync(0xffffffffu, ok)) {
+          failed = true;
+          break;
+        }
+      }
+      if (none) {
+        if (lane == 0) {
+          s_inst[s] = -1;
+          mbar_arrive(&full[s]);
+        }
+        end_slot = s;
+        break;
+      }
+      const long long gi = reverse ? b.n_items - 1 - t : t;
+      if (reverse) while (gi < b.pair[k].item_begin) --k;
+      else while (k + 1 < b.n_inst && gi >= b.pair[k + 1].item_begin) ++k;
+      const PairInst& in = b.pair[k];
+      const int ny = in.ny, nz = in.nz, RY = in.rows_per_item;
+      const int pitch = P ? P : in.pitch;
+      const int r0 = (int)(gi - in.item_begin) * RY, nr = min(ny * nz - r0, RY);
+      pair_fill(lane, static_cast<const T*>(in.buf[cur]), in.cls, r0, nr, ny, nz, pitch, spop + (size_t)s * b.slot_elems,
+                scls + (size_t)s * b.slot_cls, s_wall + s * kMaxRowsPerItem, &full[s], [&] {
+                  s_inst[s] = k;
+                  s_first[s] = r0;
+                  s_rows[s] = nr;
+                });
+      issued = j + 1;
+      if (++s == S_) { s = 0; ph ^= 1u; }
+    }
+    if (failed && lane == 0) atomicOr(b.error, STEP_ERR_PIPELINE_TIMEOUT);
+    if (lane == 0) {  // no copy may still be in flight when the CTA exits (see main_kernel)
+      for (int q = 0; q < S_ && q < issued; ++q) {
+        if (q == end_slot) continue;
+        const int last = q + ((issued - 1 - q) / S_) * S_;
+        mbar_wait(&full[q], (uint32_t)((last / S_) & 1), kWaitLimit);
+      }
+    }
+  } else {
+    // inlet velocity of row y of an instance (:334-342) at this step
+    auto inlet_of = [&](const StepArgs& ia, int y) -> double2 {
+      double ux = ia.u_inlet;
+      if (ia.ground_no_slip) ux = ia.u_inlet * ia.abl[y];
+      double uy = 0.0;
+      if (step < 120) uy = 0.015 * ia.u_inlet * ia.sin_tab[(long long)step * ia.L.ny + y];
+      return make_double2(ux, uy);
+    };
+    // near-wall cells of all instances, while the first slots fill
+    for (long long t = ((long long)warp * gridDim.x + blockIdx.x) * 32 + lane; t < b.n_near;
+         t += (long long)gridDim.x * (kPairWarps * 32)) {
+      const int k = find_instance(b.near_begin, b.n_inst, t);
+      const StepArgs& ia = b.inst[k];
+      const double corr = ia.st->apply[pslot] ? ia.st->corr[pslot] : 1.0;
+      int nan = 0;
+      const long long add = near_cell<S, MODE_FAST, P>(ia, b.bufs[2 * k + cur], b.bufs[2 * k + (cur ^ 1)], b.write_macro,
+                                                       t - b.near_begin[k], corr, [&](int y) { return inlet_of(ia, y); },
+                                                       &nan);
+      atomicAdd(&s_sum[k], (unsigned long long)add);
+      if (nan) ia.st->nan_seen = 1;
+    }
+    const EndTables ends{s_dcw, s_dslot, s_xo + warp * kEndScratch};
+    int s = 0;
+    uint32_t ph = 0;
+    int deal = warp;
+    for (;;) {
+      const bool ok = mbar_wait(&full[s], ph, b.wait_limit);
+      if (!__any_sync(0xffffffffu, ok)) {
+        failed = true;
+        break;
+      }
+      const int k = s_inst[s];
+      if (k < 0) break;
+      const PairInst& in = b.pair[k];
+      PairItem<T> it;
+      it.r0 = s_first[s];
+      it.nr = s_rows[s];
+      it.np = in.np;
+      const int chunks = (it.nr * it.np + 31) >> 5;
+      if (deal < chunks) {
+        it.nx = in.nx; it.pitch = in.pitch; it.magic = in.magic;
+        it.ny = in.ny; it.nz = in.nz; it.ground_no_slip = in.ground_no_slip; it.write_macro = b.write_macro;
+        it.tau0 = in.tau0; it.k_smag = in.k_smag;
+        const float corrf = in.st->apply[pslot] ? (float)in.st->corr[pslot] : 1.0f;
+        it.dec = make_float2(corrf * S::kRawScale, corrf - 1.0f);  // raw-moment decode
+        const int pitch = P ? P : it.pitch;
+        it.dst = static_cast<T*>(in.buf[cur ^ 1]) + (long long)it.r0 * (19 * pitch);
+        const StepArgs& ia = b.inst[k];
+        long long sum = 0;
+        int nan = 0;
+        pair_item<S, P>(it, ia, spop + (size_t)s * b.slot_elems, scls + (size_t)s * b.slot_cls, s_wall + s * kMaxRowsPerItem,
+                        deal, &empty[s], ends, [&](int y) { return inlet_of(ia, y); }, lane, sum, nan);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+        if (lane == 0 && sum) atomicAdd(&s_sum[k], (unsigned long long)sum);
+        if (__any_sync(0xffffffffu, nan) && lane == 0) in.st->nan_seen = 1;
+      } else {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[s]);
+      }
+      deal -= chunks % kPairWarps;
+      if (deal < 0) deal += kPairWarps;
+      if (++s == S_) { s = 0; ph ^= 1u; }
+    }
+    if (failed && lane == 0) atomicOr(b.error, STEP_ERR_PIPELINE_TIMEOUT);
+  }
+
+  __syncthreads();
+  const int slot = step & 1;
+  for (int k = threadIdx.x; k < b.n_inst; k += blockDim.x)
+    if (s_sum[k]) atomicAdd(&b.pair[k].st->rho_sum[slot], s_sum[k]);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned int tk = atomicAdd(&b.ticket[slot], 1u);
+    is_last = (tk == gridDim.x - 1);
+  }
+  __syncthreads();
+  if (!is_last) return;
+  // ---- the last CTA: mean-density rescale decision of every instance (:431-455) ----
+  __threadfence();
+  for (int k = threadIdx.x; k < b.n_inst; k += blockDim.x) {
+    const StepArgs& ia = b.inst[k];
+    StepState* const st = ia.st;
+    const long long total = (long long)atomicAdd(&st->rho_sum[slot], 0ull);
+    int ap = 0;
+    double cr = 1.0;
+    if (ia.fluid_count > 0) {
+      const double mean = rho_unfixed(total, 0.0f) / (double)ia.fluid_count;
+      cr = 1.0 / mean;
+      ap = fabs(mean - 1.0) > 1e-4 ? 1 : 0;
+    }
+    st->corr[slot] = cr;
+    st->apply[slot] = ap;
+    if (ap) {
+      st->cumulative_rescale *= cr;
+      st->rescale_count += 1;
+    }
+    st->rho_sum[slot ^ 1] = 0ull;
+  }
+  if (threadIdx.x == 0) {
+    b.ticket[slot ^ 1] = 0u;
+    b.ticket[2 + (slot ^ 1)] = 0u;
     *b.step = step + 1;
   }
 }

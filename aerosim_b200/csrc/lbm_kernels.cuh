@@ -35,10 +35,9 @@ enum { MODE_FAST = 0, MODE_MIRROR = 1, MODE_F64 = 2 };
 // MLP: 0 Smagorinsky, 1 the closure as warp-level mma.sync tiles, 2 the closure as
 // 128-cell tcgen05 tiles (groups of four consumer warps, TMEM accumulators).
 enum { MLP_NONE = 0, MLP_WARP = 1, MLP_TCGEN05 = 2 };
-// Two cells per thread (CPT = 2) hold twice the values: two CTAs for every storage.
-template <class S, int MODE, int MLP = MLP_NONE, int CPT = 1>
+template <class S, int MODE, int MLP = MLP_NONE>
 constexpr int step_min_blocks() {
-  return MODE != MODE_FAST ? 1 : ((MLP || CPT == 2) ? 2 : (sizeof(typename S::T) == 4 ? 3 : 2));
+  return MODE != MODE_FAST ? 1 : (MLP ? 2 : (sizeof(typename S::T) == 4 ? 3 : 2));
 }
 // Row groups per work item of the step kernel: a work item holds item_groups x
 // rows_per_item(nx) x-rows and every consumer warp takes its segment of each group, so
@@ -91,6 +90,8 @@ struct StepArgs {
   int cells_per_thread;   // consumer cells per thread: 1, or 2 (pair kernels, even nx)
   int dynamic_items;      // 1: CTAs take work items from a device counter (StepState::next_item)
                           //   instead of the static round-robin deal
+  int item_rows;          // two cells per thread: x-rows per work item, and the multiplier of a
+  uint32_t pair_magic;    //   division by the pairs per row (pair_magic)
 };
 
 struct ForceArgs {
@@ -224,6 +225,11 @@ __device__ __forceinline__ void collide_f64(double (&v)[19], double& r, double& 
 // 7 +-(y+z), 8 +-(y-z), matching lbmConstants.ts:10-32.
 __device__ __forceinline__ float frcp(float x) { return __frcp_rn(x); }
 
+// YY: the sum of squares of the stress with its roundings spelled out, starting from xx (the
+// compiler starts its FMA chain from yy otherwise): a last-bit difference of tau that a 16-bit
+// store shows about once in 10^7 values, kept apart so that each kernel gives the bits it gave
+// whatever it is inlined into.
+template <bool YY = false>
 __device__ __forceinline__ void collide_f32(float (&h)[19], float& r, float& ux, float& uy,
                                             float& uz, float tau0, float k_smag) {
   float s[9], t[9];
@@ -260,8 +266,10 @@ __device__ __forceinline__ void collide_f32(float (&h)[19], float& r, float& ux,
   const float pxy = fmaf(-rux, uy, sxy);
   const float pxz = fmaf(-rux, uz, sxz);
   const float pyz = fmaf(-ruy, uz, syz);
-  const float off = pxy * pxy + pxz * pxz + pyz * pyz;
-  const float pn = sqrtf(pxx * pxx + pyy * pyy + pzz * pzz + 2.0f * off);
+const float off = YY ? fmaf(pyz, pyz, fmaf(pxy, pxy, __fmul_rn(pxz, pxz))) : pxy * pxy + pxz * pxz + pyz * pyz;
+  const float sq = YY ? fmaf(2.0f, off, fmaf(pzz, pzz, fmaf(pyy, pyy, __fmul_rn(pxx, pxx))))
+                      : pxx * pxx + pyy * pyy + pzz * pzz + 2.0f * off;
+  const float pn = sqrtf(sq);
   const float tau = 0.5f * (tau0 + sqrtf(fmaf(tau0, tau0, k_smag * pn * ir)));
   const float om = frcp(fmaxf(0.5015f, fminf(1.95f, tau)));
   const float g = (1.0f - om) * 4.5f;
@@ -484,24 +492,19 @@ constexpr int kHelperWarp = kConsumerWarps + 1;        // warp 9: near-wall cell
 constexpr int kStepThreads = (kConsumerWarps + 2) * 32;
 enum { STEP_ERR_PIPELINE_TIMEOUT = 1 };
 
-// Thread -> cell mapping of a row.  One cell per thread (cpt = 1): cell ix = slot - shift
-// with slot = lane + 32 * warp + tx_span * chunk; shift = 1 when nx = 1 (mod 32) keeps
-// the cell pairs (0, 1) and (nx-2, nx-1) inside one warp, so the inlet and outlet
-// exchange stays warp-local.  Two cells per thread (cpt = 2, rows of an even cell count):
-// thread slot holds cells 2 slot and 2 slot + 1, so each row end sits in one thread with
-// the neighbour its boundary condition reads, and no shift is needed.
-__host__ __device__ inline int row_shift(int nx, int cpt = 1) { return (cpt == 1 && nx % 32 == 1) ? 1 : 0; }
-__host__ __device__ inline int row_span(int nx, int cpt = 1) {  // threads along x (multiple of 32, <= 256)
-  const int t = ((nx + row_shift(nx, cpt) + cpt - 1) / cpt + 31) / 32 * 32;
+// Thread -> cell mapping of a row: cell ix = slot - shift with slot = lane + 32 * warp +
+// tx_span * chunk; shift = 1 when nx = 1 (mod 32) keeps the cell pairs (0, 1) and (nx-2, nx-1)
+// inside one warp, so the inlet and outlet exchange stays warp-local.
+__host__ __device__ inline int row_shift(int nx) { return nx % 32 == 1 ? 1 : 0; }
+__host__ __device__ inline int row_span(int nx) {  // threads along x (multiple of 32, <= 256)
+  const int t = (nx + row_shift(nx) + 31) / 32 * 32;
   return t > kConsumerWarps * 32 ? kConsumerWarps * 32 : t;
 }
-__host__ __device__ inline int rows_per_item(int nx, int cpt = 1) {
-  return (kConsumerWarps * 32) / row_span(nx, cpt);
-}
+__host__ __device__ inline int rows_per_item(int nx) { return (kConsumerWarps * 32) / row_span(nx); }
 // Row groups per work item for about 1024 cells per item (1..4).
-__host__ __device__ inline int item_groups_for(int nx, int cpt = 1) {
-  const int span = row_span(nx, cpt) * cpt, chunks = (nx + row_shift(nx, cpt) + span - 1) / span;
-  const int cells = rows_per_item(nx, cpt) * chunks * span;
+__host__ __device__ inline int item_groups_for(int nx) {
+  const int span = row_span(nx), chunks = (nx + row_shift(nx) + span - 1) / span;
+  const int cells = rows_per_item(nx) * chunks * span;
   return cells >= 1024 ? 1 : (1024 / cells > 4 ? 4 : 1024 / cells);
 }
 
@@ -511,17 +514,17 @@ __host__ __device__ inline int item_groups_for(int nx, int cpt = 1) {
 // slots' destination rows; a guard; a full and an empty mbarrier per slot; the inlet
 // tables ux_in[ny], uy_in[ny]; the row coordinates [stages][groups x RY]; per consumer warp an outlet scratch row of 20
 // floats; the per-lane direction table (c_x, c_y, c_z, w; slot) of the row-end cells.
-__host__ __device__ inline size_t step_stage_bytes(const Layout& L, size_t elem, int groups = 1, int cpt = 1) {
-  return (size_t)rows_per_item(L.nx, cpt) * groups * (19 * (size_t)L.pitch * elem + (size_t)L.pitch);
+__host__ __device__ inline size_t step_stage_bytes(const Layout& L, size_t elem, int groups = 1) {
+  return (size_t)rows_per_item(L.nx) * groups * (19 * (size_t)L.pitch * elem + (size_t)L.pitch);
 }
 constexpr size_t kSmemGuard = 64;
 // With the learned closure (mlp = MLP_WARP or MLP_TCGEN05): its weight fragments, biases
 // and per-warp staging blocks; with MLP_TCGEN05 also the tcgen05 operands (sgs_umma.cuh).
 __host__ __device__ inline size_t step_smem_bytes(const Layout& L, int stages, size_t elem, int mlp = 0,
-                                                   int groups = 1, int cpt = 1) {
-  return kSmemGuard + (size_t)stages * step_stage_bytes(L, elem, groups, cpt) + kSmemGuard + 16 +
+                                                   int groups = 1) {
+  return kSmemGuard + (size_t)stages * step_stage_bytes(L, elem, groups) + kSmemGuard + 16 +
          16 * (size_t)stages + 2 * (size_t)L.ny * sizeof(double) +
-         (size_t)stages * rows_per_item(L.nx, cpt) * groups * sizeof(int2) +
+         (size_t)stages * rows_per_item(L.nx) * groups * sizeof(int2) +
          kConsumerWarps * 24 * sizeof(float) + 16 + 19 * sizeof(float4) + 19 * sizeof(int) +
          (mlp ? (kMlpFragWords * 32 + kMlpBias + 3 + kConsumerWarps * 128) * 4 : 0) +
          (mlp == 2 ? kStepUmmaBytes : 0);
@@ -535,11 +538,9 @@ __host__ __device__ inline size_t step_smem_bytes(const Layout& L, int stages, s
 // outlet (:323-373), store.  Meanwhile the helper warp takes the CTA's share of the
 // near-wall cells (Bouzidi, :196-221; one lane per cell from a link table built with
 // the voxel grid).  A near-wall cell at ix = 1 or nx-2 carries its row's inlet or
-// outlet, which need its post-collision values.  With 16-bit storage and two cells per
-// thread the helper warp also takes, from every ring slot, the two pairs of each row
-// that hold its ends (end_pair; the consumers leave them out), and a batch of near-wall
-// cells after each slot.  The last CTA takes the step's mean-density rescale decision
-// (:431-455).
+// outlet, which need its post-collision values.  The last CTA takes the step's mean-density
+// rescale decision (:431-455).  Rows of an even cell count, in the FP32 arithmetic without the
+// closure, step two cells per thread instead (pair_kernel, lbm_pair_step.cuh).
 //
 // P is the row pitch when it is a compile-time constant (0: L.pitch at run time):
 // with a constant pitch every shared-memory load and global store of a cell is an
@@ -584,7 +585,7 @@ __device__ __forceinline__ void wall_feq(typename std::conditional<MODE == MODE_
 // fsrc / fdst are the step's population buffers, inlet_u(iy) the inlet velocity
 // (double2) of row iy.  Returns the fixed-point density added to the step's sum; sets
 // *nan on a NaN.
-template <class S, int MODE, int P, class InletFn>
+template <class S, int MODE, int P, bool YY = false, class InletFn>
 __device__ __forceinline__ long long near_cell(const StepArgs& a, const void* fsrc, void* fdst, int write_macro,
                                                long long t, double corr, InletFn inlet_u, int* nan) {
   using T = typename S::T;
@@ -629,7 +630,7 @@ __device__ __forceinline__ long long near_cell(const StepArgs& a, const void* fs
   Mac mr, mx, my, mz;
   {
     Real r, ux, uy, uz;
-    if constexpr (MODE == MODE_FAST) collide_f32(v, r, ux, uy, uz, (float)a.tau0, (float)a.k_smag);
+    if constexpr (MODE == MODE_FAST) collide_f32<YY>(v, r, ux, uy, uz, (float)a.tau0, (float)a.k_smag);
     else collide_f64<MODE == MODE_MIRROR>(v, r, ux, uy, uz, a.tau0, a.k_smag);
     mr = (Mac)r; mx = (Mac)ux; my = (Mac)uy; mz = (Mac)uz;
   }
@@ -843,9 +844,8 @@ __device__ __forceinline__ long long general_cells(const StepArgs& a, double (&v
   return add;
 }
 
-// The row ends' equilibria round every operation explicitly (FMA forms), so that the
-// lane-transposed row ends (a run-time direction per lane) and the helper warp's end
-// pairs (end_pair, unrolled directions) give the same bits: in the storage domain
+// The row ends' equilibria round every operation explicitly (FMA forms), so that every kernel
+// gives the same bits: in the storage domain
 // OS w_d h + OW w_d with h = A + rho (cu + cu^2 / 2), cu = 3 c_d . u and
 // A = (rho - 1) - 1.5 rho u^2 shared by the cell's directions.  The run-time dot product
 // adds the zero products c_a u_a = +-0 that dotc leaves out, which changes no sum but the
@@ -871,21 +871,6 @@ __device__ __forceinline__ float end_rho(float r) { return __fmaf_rn(0.85f, r, 0
 // equilibrium q of its moments (:361-368), both in the storage domain.
 __device__ __forceinline__ float outlet_blend(float prev, float q) {
   return __fmaf_rn(0.75f, prev, __fmul_rn(0.25f, q));
-}
-
-// compensate_lanes' correction as lane 0 sums it (the butterfly's order), for a cell whose
-// 19 values one thread holds: the rounding errors of directions 1..18.
-template <class S>
-__device__ __forceinline__ float lane_order_errors(const float (&q)[19]) {
-  float e[32];
-#pragma unroll
-  for (int l = 0; l < 32; ++l) e[l] = (l >= 1 && l < 19) ? q[l] - S::raw(S::store(q[l])) : 0.0f;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-    for (int l = 0; l < o; ++l) e[l] = e[l] + e[l + o];
-  }
-  return e[0];
 }
 
 // One FP32-arithmetic consumer segment (32 cells of an x-row), shared by the
@@ -1043,349 +1028,55 @@ __device__ __forceinline__ void store_pair(typename S::T* p, float2 v) {
   }
 }
 
-// Geometry of a two-cells-per-thread segment: 64 cells of an x-row with an even cell
-// count, lane l holding cells x0 = cell_lo + 2 l and x0 + 1.
-struct PairGeom {
-  long long row;
-  int nx, ny, nz, pitch;
-  int iy, iz, x0;
-  int cell_lo;           // first cell of lane 0
-  bool active;           // both cells lie in the row (nx even: x0 < nx implies x0 + 1 < nx)
-  bool has_lo, has_hi;   // the segment holds cell 0 / cell nx-1 (warp-uniform)
-  bool wall_row, ground_no_slip, write_macro;
-  uint8_t c0, c1;        // class bytes of the two cells
-};
-
-// The consumer work of a two-cells-per-thread segment: the same per-cell semantics as
-// fast_segment (pull values in v, collision, inlet and outlet of the row, wall rows,
-// stores, density sum, macro outputs).  The thread that holds cell 0 holds cell 1 too, and
-// the thread that holds cell nx-1 holds nx-2, so the boundary conditions' sources
-// (lbmCpuReference.ts:323-373) sit with the row end: the outlet's (cell nx-2 after the
-// collision, before any wall condition: 19 values and the moments) are parked in the
-// warp's scratch row xo[24].  After the cells' own stores the warp holding a row end writes
-// it lane-transposed (lane d writes direction d), so the row-end work is one equilibrium
-// per lane and not 19 per thread, whether the compiler branches around it or predicates it.
-// ENDS = false: the two pairs of the row that hold its ends, (0, 1) and (nx-2, nx-1), are
-// left out altogether (no stores, density sums or macros) -- the helper warp computes
-// them from the same ring slot (end_pair) -- and the segment carries no row-end code.
-template <class S, class InletFn, bool ENDS = true>
-__device__ __forceinline__ void pair_segment(float2 (&v)[19], typename S::T* __restrict__ fd, const PairGeom g,
-                                             float tau0, float k_smag, float2 dec, InletFn inlet_u,
-                                             const StepArgs& m, float* xo, const float4* s_dcw,
-                                             const int* s_dslot, int lane, long long& my_sum, int& my_nan) {
-  using T = typename S::T;
-  constexpr float OS = S::kOutScale, OW = S::kOutW;
-  const int nx = g.nx, ny = g.ny, nz = g.nz, pitch = g.pitch, x0 = g.x0;
-  const long long row = g.row;
-  T* const blk = fd + row * 19 * pitch;
-  float2 r, ux, uy, uz;
-  collide_fast2<S>(v, r, ux, uy, uz, tau0, k_smag, dec);  // v: storage domain
-  const int f0 = g.c0 & CLS_FLAG_MASK, f1 = g.c1 & CLS_FLAG_MASK;
-  const bool mine = ENDS || (x0 != 0 && x0 + 2 != nx);  // not a pair of the helper warp
-  const bool own0 = mine && g.active && f0 != CELL_SOLID && !(g.c0 & CLS_NEAR) && x0 != 0;
-  const bool own1 = mine && g.active && f1 != CELL_SOLID && !(g.c1 & CLS_NEAR) && x0 + 1 != nx - 1;
-  if (ENDS && g.has_hi && x0 == nx - 2) {  // the outlet's sources
-#pragma unroll
-    for (int d = 0; d < 19; ++d) xo[slot_of(d)] = v[d].x;
-    xo[19] = r.x; xo[20] = ux.x; xo[21] = uy.x; xo[22] = uz.x;
-  }
-  if (g.wall_row) {  // floor, ceiling, then sides (:375-429), fluid cells only
-    if (g.iy == 0) {
-      if (g.ground_no_slip) { ux = f2(0.0f); uz = f2(0.0f); }
-      uy = f2(0.0f);
-    }
-    if (g.iy == ny - 1) uy = f2(0.0f);
-    if (nz > 4 && (g.iz == 0 || g.iz == nz - 1)) uz = f2(0.0f);
-    heq_pair<S>(v, r, ux, uy, uz);
-  }
-  T* out = blk + x0;
-  // A row end (cell 0 or nx-1) that this warp rewrites below -- the inlet or the outlet,
-  // after a __syncwarp that orders the warp's global stores -- takes the pair store with
-  // its neighbour, so the lanes of a row-end segment all store pairs instead of
-  // diverging into per-cell stores.  Not for a solid row end (never written) nor with a
-  // near-wall neighbour (the near-wall pass writes the row end then).
-  const bool pair_st = (own0 && own1) || (own1 && x0 == 0 && f0 != CELL_SOLID) ||
-                       (own0 && x0 + 1 == nx - 1 && f1 != CELL_SOLID);
-  if constexpr (S::kCompensate) {
-    // mass-compensated rounding (compensate_cell) of both cells: the moving directions
-    // round first, as packed half2 that are kept for the stores, and direction 0 takes
-    // what their rounded values leave of the cell's deviation sum.  The collision and the
-    // wall equilibrium both conserve the density, so the 19 values sum to
-    // kOutScale (r - 1) (kOutW is 0 for the shifted codecs): direction 0 is formed from
-    // that sum rather than from its own value plus the rounding errors, which needs no
-    // second copy of the 18 values
-    static_assert(std::is_same<T, __half>::value && OW == 0.0f, "compensated rounding is a shifted FP16 codec");
-    __half2 hv[19];
-    float2 sr = f2(0.0f);
-#pragma unroll
-    for (int d = 1; d < 19; ++d) {
-      hv[d] = __float22half2_rn(v[d]);
-      sr = f2add(sr, __half22float2(hv[d]));
-    }
-    hv[0] = __float22half2_rn(f2sub(f2mul(f2(OS), f2sub(r, f2(1.0f))), sr));
-    if (pair_st) {
-#pragma unroll
-      for (int d = 0; d < 19; ++d) *reinterpret_cast<__half2*>(out + slot_of(d) * pitch) = hv[d];
-    } else if (own0 || own1) {
-#pragma unroll
-      for (int d = 0; d < 19; ++d) {
-        if (own0) out[slot_of(d) * pitch] = __low2half(hv[d]);
-        if (own1) out[slot_of(d) * pitch + 1] = __high2half(hv[d]);
-      }
-    }
-  } else if (pair_st) {
-#pragma unroll
-    for (int d = 0; d < 19; ++d) store_pair<S>(out + slot_of(d) * pitch, v[d]);
-  } else if (own0 || own1) {
-#pragma unroll
-    for (int d = 0; d < 19; ++d) {
-      if (own0) out[slot_of(d) * pitch] = S::store(v[d].x);
-      if (own1) out[slot_of(d) * pitch + 1] = S::store(v[d].y);
-    }
-  }
-  if (own0) {
-    if (r.x == r.x) my_sum += rho_fixed(r.x);
-    else my_nan = 1;
-  }
-  if (own1) {
-    if (r.y == r.y) my_sum += rho_fixed(r.y);
-    else my_nan = 1;
-  }
-  if (g.write_macro && g.active && mine) {
-    const long long di = row * nx + x0;
-    if (f0 == CELL_SOLID) {  // solid macro (:173-179)
-      m.mux[di] = 0.0f; m.muy[di] = 0.0f; m.muz[di] = 0.0f; m.mrho[di] = 1.0f;
-    } else if (own0) {
-      m.mux[di] = ux.x; m.muy[di] = uy.x; m.muz[di] = uz.x; m.mrho[di] = r.x;
-    }
-    if (f1 == CELL_SOLID) {
-      m.mux[di + 1] = 0.0f; m.muy[di + 1] = 0.0f; m.muz[di + 1] = 0.0f; m.mrho[di + 1] = 1.0f;
-    } else if (own1) {
-      m.mux[di + 1] = ux.y; m.muy[di + 1] = uy.y; m.muz[di + 1] = uz.y; m.mrho[di + 1] = r.y;
-    }
-  }
-  if constexpr (!ENDS) return;
-  if (g.has_lo) {
-    // inlet (:328-352) from the density of cell 1 (1 for a solid, :177; the walls leave
-    // the density as it is), both held by lane 0; a near-wall cell 1 defers it to the
-    // near-wall pass, a solid cell 0 has none
-    const int c0 = __shfl_sync(0xffffffffu, (int)g.c0, 0), c1 = __shfl_sync(0xffffffffu, (int)g.c1, 0);
-    const float r1 = __shfl_sync(0xffffffffu, r.y, 0);
-    const bool solid1 = (c1 & CLS_FLAG_MASK) == CELL_SOLID;
-    if ((c0 & CLS_FLAG_MASK) != CELL_SOLID && !((c1 & CLS_NEAR) && !solid1)) {
-      const float ri = end_rho(solid1 ? 1.0f : r1);
-      const float2 ui = inlet_u(g.iy);
-      float q = 0.0f;
-      if (lane < 19) {
-        const float4 cw = s_dcw[lane];
-        q = end_eq<S>(dot_lane(cw, ui.x, ui.y, 0.0f), cw.w, ri, end_A(ri, ui.x, ui.y, 0.0f));
-      }
-      q = compensate_lanes<S>(q, lane);
-      __syncwarp();  // after lane 0's pair store of cells 0 and 1
-      if (lane < 19) blk[s_dslot[lane] * pitch] = S::store(q);
-      if (lane == 0) {
-        if (ri == ri) my_sum += rho_fixed(ri);
-        else my_nan = 1;
-        if (g.write_macro) {
-          const long long ic = row * nx;
-          m.mux[ic] = ui.x; m.muy[ic] = ui.y; m.muz[ic] = 0.0f; m.mrho[ic] = ri;
-        }
-      }
-    }
-  }
-  if (g.has_hi) {
-    // outlet (:354-371) from the parked cell nx-2, or from what fDst holds there when
-    // nx-2 is solid; a near-wall nx-2 defers it
-    const int src = (nx - 2 - g.cell_lo) >> 1;
-    const int c2 = __shfl_sync(0xffffffffu, (int)g.c0, src), c3 = __shfl_sync(0xffffffffu, (int)g.c1, src);
-    const bool stale = (c2 & CLS_FLAG_MASK) == CELL_SOLID;
-    if ((c3 & CLS_FLAG_MASK) != CELL_SOLID && !((c2 & CLS_NEAR) && !stale)) {
-      __syncwarp();  // the parked row xo, and the pair store of cells nx-2 and nx-1 before ours
-      const float ro = end_rho(stale ? 1.0f : xo[19]);
-      const float mx = stale ? 0.0f : xo[20], my = stale ? 0.0f : xo[21], mz = stale ? 0.0f : xo[22];
-      float q = 0.0f;
-      const int sl = lane < 19 ? s_dslot[lane] : 0;
-      if (lane < 19) {
-        const float prev = stale ? S::raw(blk[sl * pitch + nx - 2]) : xo[sl];
-        const float4 cw = s_dcw[lane];
-        q = outlet_blend(prev, end_eq<S>(dot_lane(cw, mx, my, mz), cw.w, ro, end_A(ro, mx, my, mz)));
-      }
-      q = compensate_lanes<S>(q, lane);
-      if (lane < 19) blk[sl * pitch + nx - 1] = S::store(q);
-      __syncwarp();  // the scratch row is free for the next segment
-      if (lane == 0) {
-        if (ro == ro) my_sum += rho_fixed(ro);
-        else my_nan = 1;
-        if (g.write_macro) {
-          const long long oc = row * nx + nx - 1;
-          m.mux[oc] = mx; m.muy[oc] = my; m.muz[oc] = mz; m.mrho[oc] = ro;
-        }
-      }
-    }
-  }
-}
-
-// One component of heq_pair with the same operations, so that a cell's equilibrium
-// rounds as it would in the pair form: OS (feq_d - w_d) + OW w_d.
+// Mass-compensated rounding (compensate_cell) of both cells of a pair: the moving directions
+// round first, as packed half2 that are kept for the stores, and direction 0 takes what their
+// rounded values leave of the cell's deviation sum.  The collision and the wall equilibrium
+// both conserve the density, so the 19 values sum to kOutScale (r - 1) (kOutW is 0 for the
+// shifted codecs): direction 0 is formed from that sum rather than from its own value plus
+// the rounding errors, which needs no second copy of the 18 values.
 template <class S>
-__device__ __forceinline__ float heq_one(int d, float r, float ux, float uy, float uz) {
-  constexpr float OS = S::kOutScale, OW = S::kOutW;
-  const float u2 = __fmaf_rn(ux, ux, __fmaf_rn(uy, uy, __fmul_rn(uz, uz)));
-  const float A = __fmaf_rn(__fmul_rn(-1.5f, r), u2, __fsub_rn(r, 1.0f));
-  const float cu = __fmul_rn(3.0f, dotc(d, ux, uy, uz));
-  const float h = __fmaf_rn(r, __fmaf_rn(__fmul_rn(0.5f, cu), cu, cu), A);
-  return __fmaf_rn(OS * wf_of(d), h, OW * wf_of(d));
+__device__ __forceinline__ void compensate_pair(const float2 (&v)[19], float2 r, __half2 (&hv)[19]) {
+  static_assert(std::is_same<typename S::T, __half>::value && S::kOutW == 0.0f, "compensated rounding is a shifted FP16 codec");
+  float2 sr = f2(0.0f);
+#pragma unroll
+  for (int d = 1; d < 19; ++d) {
+    hv[d] = __float22half2_rn(v[d]);
+    sr = f2add(sr, __half22float2(hv[d]));
+  }
+  hv[0] = __float22half2_rn(f2sub(f2mul(f2(S::kOutScale), f2sub(r, f2(1.0f))), sr));
 }
 
-// A pair of an x-row that holds one of its ends: cells (0, 1) (x0 = 0) or (nx-2, nx-1).
-struct EndGeom {
-  long long row;
-  int nx, ny, nz, pitch;
-  int iy, iz, x0;
-  bool wall_row, ground_no_slip, write_macro;
-  uint8_t c0, c1;  // class bytes of the two cells
-};
-
-// The helper warp's share of a two-cells-per-thread step: one lane per row-end pair,
-// pulled from the ring slot like a consumer pair, with pair_segment's semantics for
-// both cells -- the collision of both, the inlet of cell 0 from the density of cell 1
-// (:328-352) or the outlet of cell nx-1 from the post-collision, pre-wall values of
-// cell nx-2 (:354-371), the wall condition of the pair's interior cell (:375-429), the
-// stores, the density sum and the macro outputs -- with the row end's 19 equilibria
-// evaluated in the lane itself.  A near-wall interior cell defers the row end to the
-// near-wall pass (near_cell writes both), a solid row end is never written.  Returns
-// the fixed-point density added to the step's sum.
-template <class S, class InletFn>
-__device__ __forceinline__ long long end_pair(float2 (&v)[19], typename S::T* __restrict__ fd, const EndGeom g,
-                                              float tau0, float k_smag, float2 dec, InletFn inlet_u,
-                                              const StepArgs& m, int& my_nan) {
-  using T = typename S::T;
-  constexpr float OS = S::kOutScale;
-  const int pitch = g.pitch;
-  const bool lo = g.x0 == 0;
-  T* const out = fd + g.row * 19 * pitch + g.x0;
-  float2 r, ux, uy, uz;
-  collide_fast2<S>(v, r, ux, uy, uz, tau0, k_smag, dec);  // v: storage domain
-  const int f0 = g.c0 & CLS_FLAG_MASK, f1 = g.c1 & CLS_FLAG_MASK;
-  // the interior cell (1 or nx-2), unless solid or near-wall
-  const bool own = lo ? (f1 != CELL_SOLID && !(g.c1 & CLS_NEAR)) : (f0 != CELL_SOLID && !(g.c0 & CLS_NEAR));
-  bool end = false;                              // the row end is written here
-  float er = 0.0f, eu = 0.0f, ev = 0.0f, ew = 0.0f;  // its density and velocity
-  if (lo) {
-    if (f0 != CELL_SOLID && !((g.c1 & CLS_NEAR) && f1 != CELL_SOLID)) {
-      er = end_rho(f1 == CELL_SOLID ? 1.0f : r.y);
-      const float2 ui = inlet_u(g.iy);
-      eu = ui.x;
-      ev = ui.y;
-      const float A = end_A(er, eu, ev, 0.0f);
-#pragma unroll
-      for (int d = 0; d < 19; ++d) v[d].x = end_eq<S>(dotc(d, eu, ev, 0.0f), wf_of(d), er, A);
-      end = true;
-    }
-  } else {
-    const bool stale = f0 == CELL_SOLID;  // fDst's values of a solid nx-2 (never written)
-    if (f1 != CELL_SOLID && !((g.c0 & CLS_NEAR) && !stale)) {
-      er = end_rho(stale ? 1.0f : r.x);
-      eu = stale ? 0.0f : ux.x;
-      ev = stale ? 0.0f : uy.x;
-      ew = stale ? 0.0f : uz.x;
-      const float A = end_A(er, eu, ev, ew);
-#pragma unroll
-      for (int d = 0; d < 19; ++d) {
-        const float prev = stale ? S::raw(out[slot_of(d) * pitch]) : v[d].x;
-        v[d].y = outlet_blend(prev, end_eq<S>(dotc(d, eu, ev, ew), wf_of(d), er, A));
-      }
-      end = true;
-    }
+// The end of a step for one CTA (thread 0): its density sum and, in the last CTA, the
+// mean-density rescale (:431-455) and the next step's counters.
+__device__ __forceinline__ void finish_step(const StepArgs& a, long long sum) {
+  const int slot = a.step_index & 1;
+  if (sum) atomicAdd(&a.st->rho_sum[slot], (unsigned long long)sum);
+  __threadfence();
+  const unsigned int tk = atomicAdd(&a.st->ticket[slot], 1u);
+  if (tk != gridDim.x - 1) return;
+  __threadfence();
+  const long long total = (long long)atomicAdd(&a.st->rho_sum[slot], 0ull);
+  int ap = 0;
+  double cr = 1.0;
+  if (a.fluid_count > 0) {
+    const double mean = rho_unfixed(total, 0.0f) / (double)a.fluid_count;
+    cr = 1.0 / mean;
+    ap = fabs(mean - 1.0) > 1e-4 ? 1 : 0;
   }
-  if (g.wall_row) {  // floor, ceiling, then sides, on the interior cell
-    if (g.iy == 0) {
-      if (g.ground_no_slip) { ux = f2(0.0f); uz = f2(0.0f); }
-      uy = f2(0.0f);
-    }
-    if (g.iy == g.ny - 1) uy = f2(0.0f);
-    if (g.nz > 4 && (g.iz == 0 || g.iz == g.nz - 1)) uz = f2(0.0f);
-    if (lo) {
-#pragma unroll
-      for (int d = 0; d < 19; ++d) v[d].y = heq_one<S>(d, r.y, ux.y, uy.y, uz.y);
-    } else {
-#pragma unroll
-      for (int d = 0; d < 19; ++d) v[d].x = heq_one<S>(d, r.x, ux.x, uy.x, uz.x);
-    }
+  a.st->corr[slot] = cr;
+  a.st->apply[slot] = ap;
+  if (ap) {
+    a.st->cumulative_rescale *= cr;
+    a.st->rescale_count += 1;
   }
-  const bool s0 = lo ? end : own, s1 = lo ? own : end;
-  if constexpr (S::kCompensate) {
-    // the interior cell's direction 0 from its deviation sum OS (r - 1) as in
-    // pair_segment, the row end's from its own value plus the moving directions'
-    // rounding errors, summed in compensate_lanes' order
-    static_assert(std::is_same<T, __half>::value, "compensated rounding is a shifted FP16 codec");
-    float q[19];
-#pragma unroll
-    for (int d = 0; d < 19; ++d) q[d] = lo ? v[d].x : v[d].y;
-    const float q0 = q[0] + lane_order_errors<S>(q);
-    __half2 hv[19];
-    float2 sr = f2(0.0f);
-#pragma unroll
-    for (int d = 1; d < 19; ++d) {
-      hv[d] = __float22half2_rn(v[d]);
-      sr = f2add(sr, __half22float2(hv[d]));
-    }
-    const float ix = OS * (r.x - 1.0f) - sr.x, iy_ = OS * (r.y - 1.0f) - sr.y;
-    hv[0] = __floats2half2_rn(lo ? q0 : ix, lo ? iy_ : q0);
-    if (s0 && s1) {
-#pragma unroll
-      for (int d = 0; d < 19; ++d) *reinterpret_cast<__half2*>(out + slot_of(d) * pitch) = hv[d];
-    } else if (s0) {
-#pragma unroll
-      for (int d = 0; d < 19; ++d) out[slot_of(d) * pitch] = __low2half(hv[d]);
-    } else if (s1) {
-#pragma unroll
-      for (int d = 0; d < 19; ++d) out[slot_of(d) * pitch + 1] = __high2half(hv[d]);
-    }
-  } else if (s0 && s1) {
-#pragma unroll
-    for (int d = 0; d < 19; ++d) store_pair<S>(out + slot_of(d) * pitch, v[d]);
-  } else if (s0) {
-#pragma unroll
-    for (int d = 0; d < 19; ++d) out[slot_of(d) * pitch] = S::store(v[d].x);
-  } else if (s1) {
-#pragma unroll
-    for (int d = 0; d < 19; ++d) out[slot_of(d) * pitch + 1] = S::store(v[d].y);
-  }
-  long long add = 0;
-  const float ri = lo ? r.y : r.x;
-  if (own) {
-    if (ri == ri) add += rho_fixed(ri);
-    else my_nan = 1;
-  }
-  if (end) {
-    if (er == er) add += rho_fixed(er);
-    else my_nan = 1;
-  }
-  if (g.write_macro) {
-    const long long di = g.row * g.nx + g.x0;
-    const float ru = lo ? ux.y : ux.x, rv = lo ? uy.y : uy.x, rw = lo ? uz.y : uz.x;
-    if (f0 == CELL_SOLID) {  // solid macro (:173-179)
-      m.mux[di] = 0.0f; m.muy[di] = 0.0f; m.muz[di] = 0.0f; m.mrho[di] = 1.0f;
-    } else if (s0) {
-      m.mux[di] = lo ? eu : ru; m.muy[di] = lo ? ev : rv; m.muz[di] = lo ? ew : rw; m.mrho[di] = lo ? er : ri;
-    }
-    if (f1 == CELL_SOLID) {
-      m.mux[di + 1] = 0.0f; m.muy[di + 1] = 0.0f; m.muz[di + 1] = 0.0f; m.mrho[di + 1] = 1.0f;
-    } else if (s1) {
-      m.mux[di + 1] = lo ? ru : eu; m.muy[di + 1] = lo ? rv : ev; m.muz[di + 1] = lo ? rw : ew;
-      m.mrho[di + 1] = lo ? ri : er;
-    }
-  }
-  return add;
+  a.st->rho_sum[slot ^ 1] = 0ull;
+  a.st->ticket[slot ^ 1] = 0u;
+  a.st->next_item[slot ^ 1] = 0u;
 }
 
-// CPT: consumer cells per thread, 1 or 2 (MODE_FAST without the closure, even nx; the
-// host chooses, pair_segment does the work).
-template <class S, int MODE, int P, int MLP = MLP_NONE, int CPT = 1>
-__global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE, MLP, CPT>())
+template <class S, int MODE, int P, int MLP = MLP_NONE>
+__global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE, MLP>())
     main_kernel(const __grid_constant__ StepArgs a) {
-  static_assert(CPT == 1 || (MODE == MODE_FAST && MLP == MLP_NONE), "two cells per thread: fast mode only");
   using T = typename S::T;
   using Real = typename std::conditional<MODE == MODE_FAST, float, double>::type;
   using Mac = typename MacroOf<T>::type;
@@ -1400,7 +1091,7 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE, MLP, CP
   const int pitch = P ? P : L.pitch;
   const int S_ = a.stages;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int shift = row_shift(nx, CPT), span = row_span(nx, CPT), RY = rows_per_item(nx, CPT);
+  const int shift = row_shift(nx), span = row_span(nx), RY = rows_per_item(nx);
   const int wpr = span / 32;
   const long long rows = (long long)ny * nz;
   const int G = step_item_grouped<S, MODE, MLP>() && a.item_groups > 1 ? a.item_groups : 1;
@@ -1450,11 +1141,6 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE, MLP, CP
   // divide the 8 consumer warps (row spans of 96, 160, 192, 224 threads) the
   // remaining warps take no rows.
   const int n_cons = RY * wpr;
-  // Two cells per thread: the helper warp takes the row-end pairs of every item from the
-  // ring (end_pair) and releases each slot with the consumers.
-  // (16-bit storage only: the FP32 steps, bound by bandwidth, lose more to the helper's
-  // slot releases than they gain: 101.4 -> 106.9 us at 256x128x128.)
-  constexpr bool kHelperEnds = CPT == 2 && sizeof(T) == 2;
   // the tcgen05 closure needs all 8 consumer warps busy on every item (two full groups);
   // the host launches it only then, and a lattice where that does not hold steps nothing
   // and reports an error instead of leaving a group barrier short of a warp
@@ -1468,7 +1154,7 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE, MLP, CP
   if (threadIdx.x == 0) {
     for (int s = 0; s < S_; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], n_cons + (kHelperEnds ? 1 : 0));
+      mbar_init(&empty[s], n_cons);
     }
     nan_flag = 0;
     if (!groups_ok) atomicOr(&a.st->error, STEP_ERR_PIPELINE_TIMEOUT);
@@ -1531,70 +1217,12 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE, MLP, CP
 
   if (warp == kHelperWarp) {
     // ---------------- helper warp: this CTA's share of the near-wall cells ----------------
-    // (two cells per thread: and the row-end pairs of every item, one batch of near-wall
-    // cells after each item's pairs)
     const int pslot = (a.step_index + 1) & 1;
     const double corr = a.st->apply[pslot] ? a.st->corr[pslot] : 1.0;
     int my_nan = 0;
     auto inlet_d = [&](int y) { return make_double2(s_uxi[y], s_uyi[y]); };
     long long t = (long long)blockIdx.x * 32 + lane;
     const long long t_step = (long long)gridDim.x * 32;
-    if constexpr (kHelperEnds) {
-      const float corrf = (float)corr;
-      const float2 dec = make_float2(corrf * S::kRawScale, corrf - 1.0f);
-      auto inlet_f = [&](int y) { return make_float2((float)s_uxi[y], (float)s_uyi[y]); };
-      int s = 0;
-      uint32_t ph = 0;
-      long long r0 = item_row0;
-      for (int j = 0; dyn || j < count; ++j, r0 += item_step) {
-        const bool ok = mbar_wait(&full[s], ph, a.wait_limit);
-        if (!__any_sync(0xffffffffu, ok)) {
-          failed = true;
-          break;
-        }
-        if (dyn) {  // the item the producer took for this slot
-          const long long first = s_first[s];
-          if (first < 0) break;
-          r0 = first;
-        }
-        const int nr = (int)(rows - r0 < RYG ? rows - r0 : RYG);
-        for (int e0 = 0; e0 < 2 * nr; e0 += 32) {  // lane e: row e / 2 of the item, end e % 2
-          const int e = e0 + lane;
-          const bool act = e < 2 * nr;
-          const int yy = act ? e >> 1 : 0;
-          const int x0 = act && (e & 1) ? nx - 2 : 0;
-          const T* sp = spop + (size_t)(s * RYG + yy) * 19 * pitch + x0;
-          float2 v[19];
-#pragma unroll
-          for (int d = 0; d < 19; ++d) {
-            const T* q = sp + slot_of(d) * pitch;
-            if (cx_of(d) == 0) v[d] = load_pair<S>(q);
-            else v[d] = make_float2(S::raw(q[-cx_of(d)]), S::raw(q[1 - cx_of(d)]));
-          }
-          const uint32_t cls2 = *reinterpret_cast<const uint16_t*>(scls + (size_t)(s * RYG + yy) * pitch + x0);
-          const int2 yz = s_row[s * RYG + yy];
-          if (e0 + 32 >= 2 * nr) {  // the item's last pull: release the slot
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[s]);
-          }
-          if (act) {
-            EndGeom g;
-            g.row = r0 + yy; g.nx = nx; g.ny = ny; g.nz = nz; g.pitch = pitch;
-            g.iy = yz.x; g.iz = yz.y; g.x0 = x0;
-            g.wall_row = yz.x == 0 || yz.x == ny - 1 || (nz > 4 && (yz.y == 0 || yz.y == nz - 1));
-            g.ground_no_slip = a.ground_no_slip; g.write_macro = a.write_macro;
-            g.c0 = (uint8_t)(cls2 & 0xffu);
-            g.c1 = (uint8_t)(cls2 >> 8);
-            my_sum += end_pair<S>(v, fd, g, (float)a.tau0, (float)a.k_smag, dec, inlet_f, a, my_nan);
-          }
-        }
-        if (t < a.n_near) {
-          my_sum += near_cell<S, MODE, P>(a, a.fsrc, a.fdst, a.write_macro, t, corr, inlet_d, &my_nan);
-          t += t_step;
-        }
-        if (++s == S_) { s = 0; ph ^= 1u; }
-      }
-    }
     for (; t < a.n_near; t += t_step)
       my_sum += near_cell<S, MODE, P>(a, a.fsrc, a.fdst, a.write_macro, t, corr, inlet_d, &my_nan);
     if (__any_sync(0xffffffffu, my_nan) && lane == 0) nan_flag = 1;
@@ -1681,7 +1309,7 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE, MLP, CP
     const float corrf = (float)corr;
     const float2 dec = make_float2(corrf * S::kRawScale, corrf - 1.0f);  // raw-moment decode
     const int ry = warp / wpr;
-    const int nchunks = (nx + shift + span * CPT - 1) / (span * CPT);
+    const int nchunks = (nx + shift + span - 1) / span;
     int my_nan = 0;
     int s = 0;
     uint32_t ph = 0;
@@ -1742,41 +1370,6 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE, MLP, CP
         const uint8_t* sc = scls + (size_t)(s * RYG + gq * RY + ry) * pitch;
         const bool wall_row = (iy == 0 || iy == ny - 1 || (nz > 4 && (iz == 0 || iz == nz - 1)));
 
-        if constexpr (CPT == 2) {
-          // two adjacent cells per lane: 64 cells per segment, no row shift (nx even)
-          auto inlet = [&](int y) { return make_float2((float)s_uxi[y], (float)s_uyi[y]); };
-          for (int c = 0; c < nchunks; ++c) {
-            const int cell_lo = c * span * 2 + seg * 64;  // first cell of lane 0
-            const int x0 = cell_lo + 2 * lane;
-            const bool active = row_ok && x0 < nx;
-            const int lx = active ? x0 : 0;  // lanes outside the row read cells 0 and 1
-            const uint32_t cls2 = *reinterpret_cast<const uint16_t*>(sc + lx);
-            float2 v[19];
-            // ---- pull-stream (lbmCpuReference.ts:189-231) from the staged rows: a pair
-            // load where the two sources are adjacent and aligned (c_x = 0) ----
-#pragma unroll
-            for (int d = 0; d < 19; ++d) {
-              const T* q = sp + slot_of(d) * pitch + lx;
-              if (cx_of(d) == 0) v[d] = load_pair<S>(q);
-              else v[d] = make_float2(S::raw(q[-cx_of(d)]), S::raw(q[1 - cx_of(d)]));
-            }
-            if (gq == G - 1 && c == nchunks - 1) {  // every value of this slot is in registers: release it
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&empty[s]);
-            }
-            PairGeom g;
-            g.row = row; g.nx = nx; g.ny = ny; g.nz = nz; g.pitch = pitch;
-            g.iy = iy; g.iz = iz; g.x0 = x0; g.cell_lo = cell_lo; g.active = active;
-            g.has_lo = row_ok && cell_lo == 0;
-            g.has_hi = row_ok && cell_lo <= nx - 2 && nx - 2 < cell_lo + 64;
-            g.wall_row = wall_row; g.ground_no_slip = a.ground_no_slip; g.write_macro = a.write_macro;
-            g.c0 = (uint8_t)(cls2 & 0xffu);
-            g.c1 = (uint8_t)(cls2 >> 8);
-            pair_segment<S, decltype(inlet), !kHelperEnds>(v, fd, g, (float)a.tau0, (float)a.k_smag, dec, inlet, a,
-                                                           s_xo + warp * 24, s_dcw,
-                            s_dslot, lane, my_sum, my_nan);
-          }
-        } else
         for (int c = 0; c < nchunks; ++c) {
           const int cell_lo = c * span + seg * 32 - shift;  // cell of lane 0
           const int ix = cell_lo + lane;

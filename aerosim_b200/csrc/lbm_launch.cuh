@@ -4,6 +4,7 @@
 #pragma once
 #include "lbm_kernels.cuh"
 #include "lbm_batch.cuh"
+#include "lbm_pair_step.cuh"
 
 namespace aerosim {
 
@@ -28,7 +29,10 @@ cudaError_t raise_smem_limit(K k) {
 template <class S, int MODE, int P, int MLP = MLP_NONE, int CPT = 1>
 cudaError_t step_entry(const StepArgs& a, dim3 block, unsigned grid, size_t smem, cudaStream_t s, int* occ,
                        int* launches) {
-  auto k = main_kernel<S, MODE, P, MLP, CPT>;
+  auto k = [] {
+    if constexpr (CPT == 2) return pair_kernel<S, P>;
+    else return main_kernel<S, MODE, P, MLP>;
+  }();
   if (occ) {
     cudaError_t e = raise_smem_limit(k);
     if (e != cudaSuccess) return e;
@@ -103,11 +107,32 @@ cudaError_t step_dispatch(const StepArgs& a, dim3 block, unsigned grid, size_t s
   return step_entry<S, MODE, 0>(a, block, grid, smem, s, occ, launches);
 }
 
-// One step of a batch (batch_kernel) for a row pitch P (0: run time) and CPT cells per
-// consumer thread.
-template <class S, int P, int CPT>
+// One step of a batch for a row pitch P (0: run time): two cells per thread
+// (batch_pair_kernel, a programmatic dependent of the step before it, inside a captured graph
+// too) or one (batch_kernel).
+template <class S, int P>
 cudaError_t batch_entry(const BatchArgs& b, unsigned grid, size_t smem, cudaStream_t s, int* occ) {
-  auto k = batch_kernel<S, P, CPT>;
+  if (b.cells_per_thread == 2) {
+    auto k = batch_pair_kernel<S, P>;
+    if (occ) {
+      cudaError_t e = raise_smem_limit(k);
+      if (e != cudaSuccess) return e;
+      return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, kPairThreads, smem);
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kPairThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k, b);
+    return e != cudaSuccess ? e : cudaGetLastError();
+  }
+  auto k = batch_kernel<S, P>;
   if (occ) {
     cudaError_t e = raise_smem_limit(k);
     if (e != cudaSuccess) return e;
@@ -117,23 +142,17 @@ cudaError_t batch_entry(const BatchArgs& b, unsigned grid, size_t smem, cudaStre
   return cudaGetLastError();
 }
 
-template <class S, int CPT>
-cudaError_t batch_dispatch_cpt(const BatchArgs& b, int pitch, unsigned grid, size_t smem, cudaStream_t s, int* occ) {
-  switch (pitch) {
-    case 64: return batch_entry<S, 64, CPT>(b, grid, smem, s, occ);
-    case 128: return batch_entry<S, 128, CPT>(b, grid, smem, s, occ);
-    case 192: return batch_entry<S, 192, CPT>(b, grid, smem, s, occ);
-    case 256: return batch_entry<S, 256, CPT>(b, grid, smem, s, occ);
-    default: return batch_entry<S, 0, CPT>(b, grid, smem, s, occ);
-  }
-}
-
-// One step of a batch (batch_kernel).  pitch: the row pitch shared by every instance,
-// or 0 when the instances differ (the kernel then reads each instance's pitch).
+// pitch: the row pitch shared by every instance, or 0 when the instances differ (the kernel
+// then reads each instance's pitch).
 template <class S>
 cudaError_t batch_dispatch(const BatchArgs& b, int pitch, unsigned grid, size_t smem, cudaStream_t s, int* occ) {
-  return b.cells_per_thread == 2 ? batch_dispatch_cpt<S, 2>(b, pitch, grid, smem, s, occ)
-                                 : batch_dispatch_cpt<S, 1>(b, pitch, grid, smem, s, occ);
+  switch (pitch) {
+    case 64: return batch_entry<S, 64>(b, grid, smem, s, occ);
+    case 128: return batch_entry<S, 128>(b, grid, smem, s, occ);
+    case 192: return batch_entry<S, 192>(b, grid, smem, s, occ);
+    case 256: return batch_entry<S, 256>(b, grid, smem, s, occ);
+    default: return batch_entry<S, 0>(b, grid, smem, s, occ);
+  }
 }
 
 }  // namespace aerosim
