@@ -35,9 +35,12 @@ enum { MODE_FAST = 0, MODE_MIRROR = 1, MODE_F64 = 2 };
 // MLP: 0 Smagorinsky, 1 the closure as warp-level mma.sync tiles, 2 the closure as
 // 128-cell tcgen05 tiles (groups of four consumer warps, TMEM accumulators).
 enum { MLP_NONE = 0, MLP_WARP = 1, MLP_TCGEN05 = 2 };
+// Double modes: the mirror's FP64 chains want the second CTA more than the registers (43.0 ->
+// 39.0 us per step at 128x64x64 with 96 registers and spills, before the shared opposite pairs
+// 48.2); with 8-byte populations two CTAs leave two ring slots and lose (38.2 -> 43.0).
 template <class S, int MODE, int MLP = MLP_NONE>
 constexpr int step_min_blocks() {
-  return MODE != MODE_FAST ? 1 : (MLP ? 2 : (sizeof(typename S::T) == 4 ? 3 : 2));
+  return MODE == MODE_MIRROR ? 2 : MODE != MODE_FAST ? 1 : (MLP ? 2 : (sizeof(typename S::T) == 4 ? 3 : 2));
 }
 // Row groups per work item of the step kernel: a work item holds item_groups x
 // rows_per_item(nx) x-rows and every consumer warp takes its segment of each group, so
@@ -155,19 +158,22 @@ __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? l
 // the deviation h = f - w) and the moments (rho, u) with the reference's clamps.
 // ---------------------------------------------------------------------------
 
-// Double modes, lbmCpuReference.ts:226-309, evaluated in the reference's order.
-// MIRROR additionally rounds fLocal and feq to float exactly where the reference
-// stores them in Float32Arrays and uses the float-rounded weights.
-template <bool MIRROR>
+// Double modes, lbmCpuReference.ts:226-309, every operation rounded as the reference rounds
+// it.  MIRROR additionally rounds fLocal and feq to float exactly where the reference stores
+// them in Float32Arrays and uses the float-rounded weights.  What the reference evaluates per
+// direction and that cannot change a result is left out or shared: products with a zero
+// lattice component (they add a signed zero to a sum that is not one, or reach a NaN that is
+// there anyway), and between opposite directions, whose c.u are exact negatives, the square of
+// c.u and the non-equilibrium term.  That halves the FP64 operations (617 -> about 330 a cell);
+// FLOAT_IN (values that are floats already) spares the two conversions of fLocal.  Bound by
+// FP64 latency and conversions: 128x64x64 F64 42.9 -> 38.2 us per step, F32_MIRROR 48.2 -> 39.0.
+template <bool MIRROR, bool FLOAT_IN>
 __device__ __forceinline__ void collide_f64(double (&v)[19], double& r, double& ux, double& uy,
                                             double& uz, double tau0, double k_smag) {
-  double fl[19];
+  using Fe = typename std::conditional<MIRROR, float, double>::type;  // feq as the reference holds it
   r = 0.0; ux = 0.0; uy = 0.0; uz = 0.0;
-  // Terms with a zero lattice component only add a signed zero to these sums, which
-  // leaves every value the reference can produce unchanged, so they are skipped.
 #pragma unroll
   for (int d = 0; d < 19; ++d) {
-    fl[d] = MIRROR ? (double)(float)v[d] : v[d];
     r += v[d];
     if (cx_of(d)) ux += (double)cx_of(d) * v[d];
     if (cy_of(d)) uy += (double)cy_of(d) * v[d];
@@ -182,33 +188,54 @@ __device__ __forceinline__ void collide_f64(double (&v)[19], double& r, double& 
     ux *= s; uy *= s; uz *= s;
   }
   const double uSq = ux * ux + uy * uy + uz * uz;
+  const double u15 = 1.5 * uSq;
   double pxx = 0, pyy = 0, pzz = 0, pxy = 0, pxz = 0, pyz = 0;
-  double fe[19];
-#pragma unroll
-  for (int d = 0; d < 19; ++d) {
+  Fe fe[19];
+  const double wr[3] = {w32_of(0) * r, w32_of(1) * r, w32_of(7) * r};
+  // feq of direction d from the bracket 1 + cu + cu^2 / 2 - 1.5 u^2, and its share of the stress
+  auto take = [&](int d, double bracket) {
+    const double eq = wr[d == 0 ? 0 : d <= 6 ? 1 : 2] * bracket;
+    fe[d] = (Fe)eq;
+    const double fn = (MIRROR && !FLOAT_IN ? (double)(float)v[d] : v[d]) - eq;
     const double cx = cx_of(d), cy = cy_of(d), cz = cz_of(d);
-    const double cu = 3.0 * (cx * ux + cy * uy + cz * uz);
-    const double eq = w32_of(d) * r * (1.0 + cu + 0.5 * cu * cu - 1.5 * uSq);
-    fe[d] = MIRROR ? (double)(float)eq : eq;
-    const double fn = fl[d] - eq;
     if (cx_of(d)) pxx += cx * cx * fn;
     if (cy_of(d)) pyy += cy * cy * fn;
     if (cz_of(d)) pzz += cz * cz * fn;
     if (cx_of(d) * cy_of(d)) pxy += cx * cy * fn;
     if (cx_of(d) * cz_of(d)) pxz += cx * cz * fn;
     if (cy_of(d) * cz_of(d)) pyz += cy * cz * fn;
+  };
+  take(0, 1.0 - u15);
+#pragma unroll
+  for (int d = 1; d < 19; d += 2) {  // the pair d, d + 1 of opposite directions, in this order
+    const int a = cx_of(d), b = cy_of(d), c = cz_of(d);
+    double s = a ? ux : (b ? uy : uz);  // the first component of d is always positive
+    if (a && b) s = b > 0 ? s + uy : s - uy;
+    if ((a || b) && c) s = c > 0 ? s + uz : s - uz;
+    const double cu = 3.0 * s;
+    const double h = 0.5 * cu * cu;
+    take(d, 1.0 + cu + h - u15);
+    take(d + 1, 1.0 - cu + h - u15);
   }
   const double pn = sqrt(pxx * pxx + pyy * pyy + pzz * pzz + 2.0 * (pxy * pxy + pxz * pxz + pyz * pyz));
   const double tau = 0.5 * (tau0 + sqrt(tau0 * tau0 + (k_smag * pn) / r));
   const double om = 1.0 / js_max(0.5015, js_min(1.95, tau));
+  const double rest = 1.0 - om;
+  // Q:Pi from products with c^2 - 1/3, which is 1 - 1/3 or -1/3
+  constexpr double q1 = 1.0 - 1.0 / 3.0, q0 = 0.0 - 1.0 / 3.0;
+  const double x1 = q1 * pxx, x0 = q0 * pxx, y1 = q1 * pyy, y0 = q0 * pyy, z1 = q1 * pzz, z0 = q0 * pzz;
+  const double xy = 2.0 * pxy, xz = 2.0 * pxz, yz = 2.0 * pyz;
+  v[0] = (double)fe[0] + rest * (4.5 * w32_of(0) * (x0 + y0 + z0));
 #pragma unroll
-  for (int d = 0; d < 19; ++d) {
-    const double cx = cx_of(d), cy = cy_of(d), cz = cz_of(d);
-    const double qxx = cx * cx - 1.0 / 3.0, qyy = cy * cy - 1.0 / 3.0, qzz = cz * cz - 1.0 / 3.0;
-    const double qxy = cx * cy, qxz = cx * cz, qyz = cy * cz;
-    const double f1 = 4.5 * w32_of(d) *
-                      (qxx * pxx + qyy * pyy + qzz * pzz + 2.0 * (qxy * pxy + qxz * pxz + qyz * pyz));
-    v[d] = fe[d] + (1.0 - om) * f1;
+  for (int d = 1; d < 19; d += 2) {
+    const int a = cx_of(d), b = cy_of(d), c = cz_of(d);
+    double q = (a ? x1 : x0) + (b ? y1 : y0) + (c ? z1 : z0);
+    if (a * b) q = a * b > 0 ? q + xy : q - xy;
+    if (a * c) q = a * c > 0 ? q + xz : q - xz;
+    if (b * c) q = b * c > 0 ? q + yz : q - yz;
+    const double f1 = rest * (4.5 * w32_of(d) * q);
+    v[d] = (double)fe[d] + f1;
+    v[d + 1] = (double)fe[d + 1] + f1;
   }
 }
 
@@ -631,7 +658,7 @@ __device__ __forceinline__ long long near_cell(const StepArgs& a, const void* fs
   {
     Real r, ux, uy, uz;
     if constexpr (MODE == MODE_FAST) collide_f32<YY>(v, r, ux, uy, uz, (float)a.tau0, (float)a.k_smag);
-    else collide_f64<MODE == MODE_MIRROR>(v, r, ux, uy, uz, a.tau0, a.k_smag);
+    else collide_f64<MODE == MODE_MIRROR, false>(v, r, ux, uy, uz, a.tau0, a.k_smag);
     mr = (Mac)r; mx = (Mac)ux; my = (Mac)uy; mz = (Mac)uz;
   }
   if (ix == 1 && (a.cls[cls_row] & CLS_FLAG_MASK) != CELL_SOLID) {
@@ -766,7 +793,7 @@ __device__ __forceinline__ long long general_cells(const StepArgs& a, double (&v
   Mac mr, mx, my, mz;
   {
     double r, ux, uy, uz;
-    collide_f64<MODE == MODE_MIRROR>(v, r, ux, uy, uz, a.tau0, a.k_smag);
+    collide_f64<MODE == MODE_MIRROR, true>(v, r, ux, uy, uz, a.tau0, a.k_smag);  // the pull rounds to float
     mr = (Mac)r; mx = (Mac)ux; my = (Mac)uy; mz = (Mac)uz;
   }
   bool done = active && !solid && !xface && !near;  // this lane stores its cell
@@ -1384,8 +1411,16 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE, MLP>())
           for (int d = 0; d < 19; ++d) {
             const T raw = sp[slot_of(d) * pitch + lx - cx_of(d)];
             if constexpr (MODE == MODE_FAST) v[d] = S::raw(raw);  // decoded in the moments
-            else if constexpr (MODE == MODE_MIRROR) v[d] = (double)(float)(S::f_of(raw, d) * corr);
-            else v[d] = S::f_of(raw, d) * corr;
+            else v[d] = S::f_of(raw, d);
+          }
+          if constexpr (MODE != MODE_FAST) {
+            if (corr != 1.0) {  // a pending rescale (a factor of 1 changes nothing)
+#pragma unroll
+              for (int d = 0; d < 19; ++d) {
+                v[d] *= corr;
+                if constexpr (MODE == MODE_MIRROR) v[d] = (double)(float)v[d];
+              }
+            }
           }
           if (gq == G - 1 && c == nchunks - 1) {  // every value of this slot is in registers: release it
             __syncwarp();
