@@ -90,7 +90,7 @@ struct StepArgs {
   int item_groups;        // row groups per work item (16-bit storage kernels; 1 elsewhere)
   int wait_limit;         // polls of a ring wait before the step gives up (kWaitLimit;
                           //   0 gives up at once: the failure path's test)
-  int cells_per_thread;   // consumer cells per thread: 1, or 2 (pair kernels, even nx)
+  int cells_per_thread;   // consumer cells per thread: 1, or 2 (pair kernels)
   int dynamic_items;      // 1: CTAs take work items from a device counter (StepState::next_item)
                           //   instead of the static round-robin deal
   int item_rows;          // two cells per thread: x-rows per work item, and the multiplier of a
@@ -1060,17 +1060,19 @@ __device__ __forceinline__ void store_pair(typename S::T* p, float2 v) {
 // rounded values leave of the cell's deviation sum.  The collision and the wall equilibrium
 // both conserve the density, so the 19 values sum to kOutScale (r - 1) (kOutW is 0 for the
 // shifted codecs): direction 0 is formed from that sum rather than from its own value plus
-// the rounding errors, which needs no second copy of the 18 values.
-template <class S>
+// the rounding errors, which needs no second copy of the 18 values.  With FUSE as
+// compensate_cell does it: direction 0 plus the rounding errors in direction order.
+template <class S, bool FUSE = false>
 __device__ __forceinline__ void compensate_pair(const float2 (&v)[19], float2 r, __half2 (&hv)[19]) {
   static_assert(std::is_same<typename S::T, __half>::value && S::kOutW == 0.0f, "compensated rounding is a shifted FP16 codec");
   float2 sr = f2(0.0f);
 #pragma unroll
   for (int d = 1; d < 19; ++d) {
     hv[d] = __float22half2_rn(v[d]);
-    sr = f2add(sr, __half22float2(hv[d]));
+    sr = f2add(sr, FUSE ? f2sub(v[d], __half22float2(hv[d])) : __half22float2(hv[d]));
   }
-  hv[0] = __float22half2_rn(f2sub(f2mul(f2(S::kOutScale), f2sub(r, f2(1.0f))), sr));
+  if constexpr (FUSE) hv[0] = __float22half2_rn(f2add(v[0], sr));
+  else hv[0] = __float22half2_rn(f2sub(f2mul(f2(S::kOutScale), f2sub(r, f2(1.0f))), sr));
 }
 
 // The end of a step for one CTA (thread 0): its density sum and, in the last CTA, the

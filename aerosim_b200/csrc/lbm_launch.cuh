@@ -24,13 +24,15 @@ cudaError_t raise_smem_limit(K k) {
   return e;
 }
 
-// One time step: a single main_kernel launch.  Returns the number of launches in
+// One time step: a single launch, main_kernel (CPT 1), pair_kernel (2) or its form for rows
+// of an odd cell count (3).  Returns the number of launches in
 // *launches.
 template <class S, int MODE, int P, int MLP = MLP_NONE, int CPT = 1>
 cudaError_t step_entry(const StepArgs& a, dim3 block, unsigned grid, size_t smem, cudaStream_t s, int* occ,
                        int* launches) {
   auto k = [] {
-    if constexpr (CPT == 2) return pair_kernel<S, P>;
+    if constexpr (CPT == 3) return pair_kernel<S, P, true>;
+    else if constexpr (CPT == 2) return pair_kernel<S, P>;
     else return main_kernel<S, MODE, P, MLP>;
   }();
   if (occ) {
@@ -79,7 +81,20 @@ cudaError_t step_dispatch(const StepArgs& a, dim3 block, unsigned grid, size_t s
         default: return step_entry<S, MODE, 0, MLP_WARP>(a, block, grid, smem, s, occ, launches);
       }
     }
-    if (a.cells_per_thread == 2) {  // two cells per thread (even nx)
+    if (a.cells_per_thread == 2 && a.L.nx % 2) {  // two cells per thread, a single outlet cell (odd nx)
+      switch (a.L.pitch) {
+        case 32: return step_entry<S, MODE, 32, MLP_NONE, 3>(a, block, grid, smem, s, occ, launches);
+        case 64: return step_entry<S, MODE, 64, MLP_NONE, 3>(a, block, grid, smem, s, occ, launches);
+        case 96: return step_entry<S, MODE, 96, MLP_NONE, 3>(a, block, grid, smem, s, occ, launches);
+        case 128: return step_entry<S, MODE, 128, MLP_NONE, 3>(a, block, grid, smem, s, occ, launches);
+        case 160: return step_entry<S, MODE, 160, MLP_NONE, 3>(a, block, grid, smem, s, occ, launches);
+        case 192: return step_entry<S, MODE, 192, MLP_NONE, 3>(a, block, grid, smem, s, occ, launches);
+        case 224: return step_entry<S, MODE, 224, MLP_NONE, 3>(a, block, grid, smem, s, occ, launches);
+        case 256: return step_entry<S, MODE, 256, MLP_NONE, 3>(a, block, grid, smem, s, occ, launches);
+        default: return step_entry<S, MODE, 0, MLP_NONE, 3>(a, block, grid, smem, s, occ, launches);
+      }
+    }
+    if (a.cells_per_thread == 2) {  // two cells per thread, even nx
       switch (a.L.pitch) {
         case 32: return step_entry<S, MODE, 32, MLP_NONE, 2>(a, block, grid, smem, s, occ, launches);
         case 64: return step_entry<S, MODE, 64, MLP_NONE, 2>(a, block, grid, smem, s, occ, launches);

@@ -3,8 +3,10 @@
 // instruction, so a thread that owns two adjacent cells of an x-row issues about half
 // the floating-point instructions per cell.  Clamps, comparisons and the approximate
 // reciprocal and square roots stay per component.  Same operations and order as
-// collide_fast (lbm_kernels.cuh), so each component rounds exactly as collide_fast would
-// for that cell, up to the compiler's FMA contraction.
+// collide_fast (lbm_kernels.cuh), up to the compiler's FMA contraction.  With FUSE the sums
+// that the compiler contracts there are spelled out as FMAs, so each component rounds exactly
+// as collide_fast does: lattices of an odd nx keep the 16-bit populations of the
+// one-cell-per-thread step (tests/test_gpu_pair_items.py).
 #pragma once
 #include "common.cuh"
 
@@ -45,9 +47,21 @@ __device__ __forceinline__ float2 dotc2(int d, float2 x, float2 y, float2 z) {
 
 // Equilibrium of a pair in the storage domain, OS (feq_d - w_d) + OW w_d, with
 // feq_d - w_d = w_d ((rho - 1) - 1.5 rho u^2 + rho (cu + cu^2 / 2)), cu = 3 c_d . u.
-template <class S>
+template <class S, bool FUSE = false>
 __device__ __forceinline__ void heq_pair(float2 (&v)[19], float2 r, float2 ux, float2 uy, float2 uz) {
   constexpr float OS = S::kOutScale, OW = S::kOutW;
+  if constexpr (FUSE) {  // heq32's form
+    const float2 u2 = f2fma(uz, uz, f2fma(uy, uy, f2mul(ux, ux)));
+    const float2 r1 = f2sub(r, f2(1.0f));
+#pragma unroll
+    for (int d = 0; d < 19; ++d) {
+      const float2 cu = f2mul(f2(3.0f), dotc2(d, ux, uy, uz));
+      const float2 b = f2fma(f2(-1.5f), u2, f2fma(f2mul(f2(0.5f), cu), cu, cu));
+      const float2 h = f2mul(f2(wf_of(d)), f2fma(r, b, r1));
+      v[d] = OS == 1.0f && OW == 0.0f ? h : f2fma(f2(OS), h, f2(OW * wf_of(d)));
+    }
+    return;
+  }
   const float2 u2 = f2fma(ux, ux, f2fma(uy, uy, f2mul(uz, uz)));
   const float2 A = f2fma(f2mul(f2(-1.5f), r), u2, f2sub(r, f2(1.0f)));
 #pragma unroll
@@ -61,7 +75,7 @@ __device__ __forceinline__ void heq_pair(float2 (&v)[19], float2 r, float2 ux, f
 // h: the raw stored values of the two cells (x: first cell, y: second), replaced by the
 // post-collision values in the storage domain; r, u: the clamped, Mach-limited moments.
 // dec = (storage scale x pending rescale, rescale - 1) as in collide_fast.
-template <class S>
+template <class S, bool FUSE = false>
 __device__ __forceinline__ void collide_fast2(float2 (&h)[19], float2& r, float2& ux, float2& uy, float2& uz,
                                               float tau0, float k_smag, float2 dec) {
   static_assert(S::kRawMoments, "the FP32 collision runs on stored deviations");
@@ -73,8 +87,8 @@ __device__ __forceinline__ void collide_fast2(float2 (&h)[19], float2& r, float2
     s[p] = f2add(h[2 * p + 1], h[2 * p + 2]);
     t[p] = f2sub(h[2 * p + 1], h[2 * p + 2]);
   }
-  float2 dr = f2add(h[0], f2add(f2add(f2add(s[0], s[1]), f2add(s[2], s[3])),
-                                f2add(f2add(f2add(s[4], s[5]), f2add(s[6], s[7])), s[8])));
+  const float2 da = f2add(f2add(s[0], s[1]), f2add(s[2], s[3])), db = f2add(f2add(s[4], s[5]), f2add(s[6], s[7]));
+  float2 dr = f2add(h[0], FUSE ? f2add(f2add(da, db), s[8]) : f2add(da, f2add(db, s[8])));
   float2 jx = f2add(f2add(f2add(t[0], t[3]), f2add(t[4], t[5])), t[6]);
   float2 jy = f2add(f2sub(f2add(t[1], t[3]), t[4]), f2add(t[7], t[8]));
   float2 jz = f2add(f2sub(f2add(t[2], t[5]), t[6]), f2sub(t[7], t[8]));
@@ -96,7 +110,7 @@ __device__ __forceinline__ void collide_fast2(float2 (&h)[19], float2& r, float2
   const float2 ir = make_float2(rcp_approx_(r.x), rcp_approx_(r.y));
   ux = f2mul(jx, ir); uy = f2mul(jy, ir); uz = f2mul(jz, ir);
   {
-    const float2 u2 = f2fma(ux, ux, f2fma(uy, uy, f2mul(uz, uz)));
+    const float2 u2 = FUSE ? f2fma(uz, uz, f2fma(uy, uy, f2mul(ux, ux))) : f2fma(ux, ux, f2fma(uy, uy, f2mul(uz, uz)));
     // Mach limiter |u| <= 0.22: a factor of exactly 1 leaves the other cell unchanged
     const float2 sc = make_float2(u2.x > 0.0484f ? 0.22f * rsqrtf(u2.x) : 1.0f,
                                   u2.y > 0.0484f ? 0.22f * rsqrtf(u2.y) : 1.0f);
@@ -105,7 +119,9 @@ __device__ __forceinline__ void collide_fast2(float2 (&h)[19], float2& r, float2
   const float2 drc = f2sub(r, f2(1.0f));
   const float2 d3 = f2mul(drc, f2(1.0f / 3.0f));
   const float2 jcx = f2mul(r, ux), jcy = f2mul(r, uy), jcz = f2mul(r, uz);
-  const float2 dxx = f2sub(sxx, d3), dyy = f2sub(syy, d3), dzz = f2sub(szz, d3);
+  const float2 m3 = f2(-1.0f / 3.0f);
+  const float2 dxx = FUSE ? f2fma(m3, drc, sxx) : f2sub(sxx, d3), dyy = FUSE ? f2fma(m3, drc, syy) : f2sub(syy, d3),
+               dzz = FUSE ? f2fma(m3, drc, szz) : f2sub(szz, d3);
   const float2 pxx = f2fma(f2neg(jcx), ux, dxx), pyy = f2fma(f2neg(jcy), uy, dyy), pzz = f2fma(f2neg(jcz), uz, dzz);
   const float2 pxy = f2fma(f2neg(jcx), uy, sxy), pxz = f2fma(f2neg(jcx), uz, sxz), pyz = f2fma(f2neg(jcy), uz, syz);
   const float2 off = f2fma(pxy, pxy, f2fma(pxz, pxz, f2mul(pyz, pyz)));
@@ -125,15 +141,15 @@ __device__ __forceinline__ void collide_fast2(float2 (&h)[19], float2& r, float2
   constexpr float kf = OS * 4.5f * w1, of = OS * 3.0f * w1;
   {
     const float2 E = f2fma(f2(kf), xxx, b1), O = f2mul(f2(of), jcx);
-    h[1] = f2add(E, O); h[2] = f2sub(E, O);
+    h[1] = FUSE ? f2fma(f2(of), jcx, E) : f2add(E, O); h[2] = FUSE ? f2fma(f2(-of), jcx, E) : f2sub(E, O);
   }
   {
     const float2 E = f2fma(f2(kf), xyy, b1), O = f2mul(f2(of), jcy);
-    h[3] = f2add(E, O); h[4] = f2sub(E, O);
+    h[3] = FUSE ? f2fma(f2(of), jcy, E) : f2add(E, O); h[4] = FUSE ? f2fma(f2(-of), jcy, E) : f2sub(E, O);
   }
   {
     const float2 E = f2fma(f2(kf), xzz, b1), O = f2mul(f2(of), jcz);
-    h[5] = f2add(E, O); h[6] = f2sub(E, O);
+    h[5] = FUSE ? f2fma(f2(of), jcz, E) : f2add(E, O); h[6] = FUSE ? f2fma(f2(-of), jcz, E) : f2sub(E, O);
   }
   const float2 b2 = f2mul(f2(w2), b);
   constexpr float ke = OS * 4.5f * w2, ke2 = OS * 9.0f * w2, oe = OS * 3.0f * w2;
@@ -141,19 +157,22 @@ __device__ __forceinline__ void collide_fast2(float2 (&h)[19], float2& r, float2
   {
     const float2 base = f2fma(f2(ke), f2add(xxx, xyy), b2);
     const float2 Ep = f2fma(f2(ke2), xxy, base), Em = f2fma(f2(-ke2), xxy, base);
-    const float2 Op = f2add(qx, qy), Om = f2sub(qx, qy);
+    const float2 Op = FUSE ? f2fma(f2(oe), jcy, qx) : f2add(qx, qy);
+    const float2 Om = FUSE ? f2fma(f2(-oe), jcy, qx) : f2sub(qx, qy);
     h[7] = f2add(Ep, Op); h[8] = f2sub(Ep, Op); h[9] = f2add(Em, Om); h[10] = f2sub(Em, Om);
   }
   {
     const float2 base = f2fma(f2(ke), f2add(xxx, xzz), b2);
     const float2 Ep = f2fma(f2(ke2), xxz, base), Em = f2fma(f2(-ke2), xxz, base);
-    const float2 Op = f2add(qx, qz), Om = f2sub(qx, qz);
+    const float2 Op = FUSE ? f2fma(f2(oe), jcz, qx) : f2add(qx, qz);
+    const float2 Om = FUSE ? f2fma(f2(-oe), jcz, qx) : f2sub(qx, qz);
     h[11] = f2add(Ep, Op); h[12] = f2sub(Ep, Op); h[13] = f2add(Em, Om); h[14] = f2sub(Em, Om);
   }
   {
     const float2 base = f2fma(f2(ke), f2add(xyy, xzz), b2);
     const float2 Ep = f2fma(f2(ke2), xyz, base), Em = f2fma(f2(-ke2), xyz, base);
-    const float2 Op = f2add(qy, qz), Om = f2sub(qy, qz);
+    const float2 Op = FUSE ? f2fma(f2(oe), jcz, qy) : f2add(qy, qz);
+    const float2 Om = FUSE ? f2fma(f2(-oe), jcz, qy) : f2sub(qy, qz);
     h[15] = f2add(Ep, Op); h[16] = f2sub(Ep, Op); h[17] = f2add(Em, Om); h[18] = f2sub(Em, Om);
   }
 }

@@ -1,5 +1,7 @@
 // The two-cells-per-thread step of a single lattice (pair_kernel) and the item loop it
-// shares with the batched step: rows of an even cell count, FP32 arithmetic, no closure.
+// shares with the batched step: FP32 arithmetic, no closure, rows of 4 and more cells (a batch:
+// of an even count).  With ODD the pairs cover cells 0 .. nx-2 and the outlet cell nx-1 follows
+// the last of them.
 //
 // A work item is R consecutive x-rows; its pairs of cells form one list, and each consumer
 // warp takes chunks of 32 consecutive pairs of it, across row ends, dealt cyclically (the
@@ -15,7 +17,8 @@
 // 0.95 of the copy peak in a run of steps).  Microseconds per step, before -> with this kernel:
 // 256x128x128 F16S 68.5 -> 60.3, BF16S 69.5 -> 59.6, F16C 73.1 -> 64, FP32 101.6 -> 101.4;
 // 160x80x80 F16S 28.2 -> 22.1; 200x100x96 F16S 43.1 -> 37.1; 128x64x64 FP32 20.3 -> 16.5;
-// 64x32x32 FP32 11.4 -> 9.6.  What made the difference: the bulk copies issued by one elected
+// 64x32x32 FP32 11.4 -> 9.6; 191x95x97 (one cell per thread before) BF16S 43.8 -> 33.8, FP32
+// 58.4 -> 50.1.  What made the difference: the bulk copies issued by one elected
 // lane from uniform registers, 37 an item of 4 rows (by 32 lanes they are replayed one by one,
 // about 20 instructions each, and the producer warp was the limit: 63.5 us), the flat pair
 // list (the helper warp's row ends were 6 M of 46 M instructions, on the critical path) and
@@ -76,18 +79,20 @@ struct EndTables {
   const uint8_t* dslot;
   float* xo;            // the warp's scratch row
 };
-template <class S, class InletFn>
+template <class S, bool ODD, class InletFn>
 __device__ __forceinline__ void chunk_ends(const float2 (&v)[19], float2 r, float2 ux, float2 uy, float2 uz, bool lo, bool hi,
-                                           uint32_t cls2, int yy, typename S::T* dst, int pitch, int nx, int ny, int r0,
-                                           bool write_macro, const StepArgs& m, const EndTables& e, InletFn inlet, int lane,
+                                           uint32_t cls2 /* of the pair and, nx odd, of cell nx-1 */, int yy,
+                                           typename S::T* dst, int pitch, int nx, int ny, int r0, bool write_macro,
+                                           const StepArgs& m, const EndTables& e, InletFn inlet, int lane,
                                            long long& my_sum, int& my_nan) {
   using T = typename S::T;
   for (unsigned left = __ballot_sync(0xffffffffu, lo || hi); left; left &= left - 1) {
     const int src = __ffs(left) - 1;
     const bool is_hi = __shfl_sync(0xffffffffu, (int)hi, src) != 0;
-    const int c2 = __shfl_sync(0xffffffffu, (int)cls2, src), ry = __shfl_sync(0xffffffffu, yy, src);
+    const int cls3 = __shfl_sync(0xffffffffu, (int)cls2, src), ry = __shfl_sync(0xffffffffu, yy, src);
     // the end's class and its neighbour's
-    const int ce = is_hi ? c2 >> 8 : c2 & 0xff, cn = is_hi ? c2 & 0xff : c2 >> 8;
+    const int ce = (is_hi ? (ODD ? cls3 >> 16 : cls3 >> 8) : cls3) & 0xff,
+              cn = (is_hi ? (ODD ? cls3 >> 8 : cls3) : cls3 >> 8) & 0xff;
     const bool solid_n = (cn & CLS_FLAG_MASK) == CELL_SOLID;
     if ((ce & CLS_FLAG_MASK) == CELL_SOLID || ((cn & CLS_NEAR) && !solid_n)) continue;
     T* const blk = dst + ry * (19 * pitch);
@@ -97,8 +102,9 @@ __device__ __forceinline__ void chunk_ends(const float2 (&v)[19], float2 r, floa
     if (is_hi) {  // outlet (:354-371); a solid nx-2 gives what fDst holds there
       if (lane == src) {
 #pragma unroll
-        for (int d = 0; d < 19; ++d) e.xo[slot_of(d)] = v[d].x;
-        e.xo[19] = r.x; e.xo[20] = ux.x; e.xo[21] = uy.x; e.xo[22] = uz.x;
+        for (int d = 0; d < 19; ++d) e.xo[slot_of(d)] = ODD ? v[d].y : v[d].x;
+        e.xo[19] = ODD ? r.y : r.x; e.xo[20] = ODD ? ux.y : ux.x;
+        e.xo[21] = ODD ? uy.y : uy.x; e.xo[22] = ODD ? uz.y : uz.x;
       }
       __syncwarp();
       rho = end_rho(solid_n ? 1.0f : e.xo[19]);
@@ -134,7 +140,7 @@ __device__ __forceinline__ void chunk_ends(const float2 (&v)[19], float2 r, floa
 // collision, stores, density sum, row ends.  (After the release only registers may be used:
 // the next fill overwrites the slot and the rows' flags.)  Near-wall cells are left to the
 // near-wall pass, solids are never written.
-template <class S, int P, class InletFn>
+template <class S, int P, bool ODD = false, class InletFn>
 __device__ __forceinline__ void pair_item(const PairItem<typename S::T>& it, const StepArgs& m, const typename S::T* slot,
                                           const uint8_t* cls, const uint8_t* wall, int first, uint64_t* empty,
                                           const EndTables& ends, InletFn inlet, int lane, long long& my_sum,
@@ -151,6 +157,10 @@ __device__ __forceinline__ void pair_item(const PairItem<typename S::T>& it, con
     const T* const sp = slot + off;
     const uint32_t cls2 = *reinterpret_cast<const uint16_t*>(cls + yy * pitch + x0);
     const bool wall_row = wall[yy] != 0;
+    // the row ends: cell 0 in its pair; cell nx-1 in its pair (nx even) or after the last
+    // pair, which then ends with its source nx-2 (nx odd)
+    const bool lo = act && x0 == 0, hi = act && x0 + (ODD ? 3 : 2) == it.nx;
+    const uint32_t end_cls = ODD ? cls[yy * pitch + it.nx - 1] : 0u;
     float2 v[19];
 #pragma unroll
     for (int d = 0; d < 19; ++d) {  // pull-stream (lbmCpuReference.ts:189-231)
@@ -163,14 +173,13 @@ __device__ __forceinline__ void pair_item(const PairItem<typename S::T>& it, con
       if (lane == 0) mbar_arrive(empty);
     }
     float2 r, ux, uy, uz;
-    collide_fast2<S>(v, r, ux, uy, uz, it.tau0, it.k_smag, it.dec);  // v: storage domain
-    const bool lo = act && x0 == 0, hi = act && x0 + 2 == it.nx;
+    collide_fast2<S, ODD>(v, r, ux, uy, uz, it.tau0, it.k_smag, it.dec);  // v: storage domain
     T* const out = it.dst + off;
     if (!__any_sync(0xffffffffu, act && ((cls2 & 0x0707u) != 0u || wall_row)) && !it.write_macro) {
       if (act) {
         if constexpr (S::kCompensate) {
           __half2 hv[19];
-          compensate_pair<S>(v, r, hv);
+          compensate_pair<S, ODD>(v, r, hv);
 #pragma unroll
           for (int d = 0; d < 19; ++d) *reinterpret_cast<__half2*>(out + slot_of(d) * pitch) = hv[d];
         } else {
@@ -178,22 +187,23 @@ __device__ __forceinline__ void pair_item(const PairItem<typename S::T>& it, con
           for (int d = 0; d < 19; ++d) store_pair<S>(out + slot_of(d) * pitch, v[d]);
         }
         // a NaN density counts 0 in the sum (the conversion's result) and sets the flag
-        my_sum += (lo ? 0 : __float2int_rn(r.x * 33554432.0f)) + (hi ? 0 : __float2int_rn(r.y * 33554432.0f));
-        const float t = (lo ? 1.0f : r.x) + (hi ? 1.0f : r.y);
+        const bool end1 = !ODD && hi;  // the pair's second cell is the outlet
+        my_sum += (lo ? 0 : __float2int_rn(r.x * 33554432.0f)) + (end1 ? 0 : __float2int_rn(r.y * 33554432.0f));
+        const float t = (lo ? 1.0f : r.x) + (end1 ? 1.0f : r.y);
         if (t != t) my_nan = 1;
       }
       if (__any_sync(0xffffffffu, lo || hi))
-        chunk_ends<S>(v, r, ux, uy, uz, lo, hi, cls2, yy, it.dst, pitch, it.nx, it.ny, it.r0, false, m, ends, inlet, lane,
-                      my_sum, my_nan);
+        chunk_ends<S, ODD>(v, r, ux, uy, uz, lo, hi, cls2 | (end_cls << 16), yy, it.dst, pitch, it.nx, it.ny, it.r0,
+                           false, m, ends, inlet, lane, my_sum, my_nan);
       continue;
     }
     // the row ends first: the outlet reads cell nx-2 before any wall condition
     if (__any_sync(0xffffffffu, lo || hi))
-      chunk_ends<S>(v, r, ux, uy, uz, lo, hi, cls2, yy, it.dst, pitch, it.nx, it.ny, it.r0, it.write_macro, m, ends, inlet,
-                    lane, my_sum, my_nan);
+      chunk_ends<S, ODD>(v, r, ux, uy, uz, lo, hi, cls2 | (end_cls << 16), yy, it.dst, pitch, it.nx, it.ny, it.r0,
+                         it.write_macro, m, ends, inlet, lane, my_sum, my_nan);
     const int f0 = cls2 & CLS_FLAG_MASK, f1 = (cls2 >> 8) & CLS_FLAG_MASK;
     const bool own0 = act && f0 != CELL_SOLID && !(cls2 & CLS_NEAR) && !lo;
-    const bool own1 = act && f1 != CELL_SOLID && !(cls2 & (CLS_NEAR << 8)) && !hi;
+    const bool own1 = act && f1 != CELL_SOLID && !(cls2 & (CLS_NEAR << 8)) && (ODD || !hi);
     if (wall_row) {  // floor, ceiling, then sides (:375-429), fluid cells only
       const int row = it.r0 + yy, iz = row / it.ny, iy = row - iz * it.ny;
       if (iy == 0) {
@@ -202,11 +212,11 @@ __device__ __forceinline__ void pair_item(const PairItem<typename S::T>& it, con
       }
       if (iy == it.ny - 1) uy = f2(0.0f);
       if (it.nz > 4 && (iz == 0 || iz == it.nz - 1)) uz = f2(0.0f);
-      heq_pair<S>(v, r, ux, uy, uz);
+      heq_pair<S, ODD>(v, r, ux, uy, uz);
     }
     if constexpr (S::kCompensate) {
       __half2 hv[19];
-      compensate_pair<S>(v, r, hv);
+      compensate_pair<S, ODD>(v, r, hv);
       if (own0 && own1) {
 #pragma unroll
         for (int d = 0; d < 19; ++d) *reinterpret_cast<__half2*>(out + slot_of(d) * pitch) = hv[d];
@@ -246,6 +256,9 @@ __device__ __forceinline__ void pair_item(const PairItem<typename S::T>& it, con
         m.mux[di + 1] = 0.0f; m.muy[di + 1] = 0.0f; m.muz[di + 1] = 0.0f; m.mrho[di + 1] = 1.0f;
       } else if (own1) {
         m.mux[di + 1] = ux.y; m.muy[di + 1] = uy.y; m.muz[di + 1] = uz.y; m.mrho[di + 1] = r.y;
+      }
+      if (ODD && hi && (end_cls & CLS_FLAG_MASK) == CELL_SOLID) {
+        m.mux[di + 2] = 0.0f; m.muy[di + 2] = 0.0f; m.muz[di + 2] = 0.0f; m.mrho[di + 2] = 1.0f;
       }
     }
   }
@@ -332,7 +345,7 @@ __device__ __forceinline__ void fill_end_tables(float4* dcw, uint8_t* dslot) {
 // One time step of one lattice: a producer warp fills the ring, the consumer warps first take
 // their near-wall cells, while the first slots fill, and then the chunks of the items; the
 // last CTA takes the rescale decision.
-template <class S, int P>
+template <class S, int P, bool ODD = false>
 __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(const __grid_constant__ StepArgs a) {
   using T = typename S::T;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -448,7 +461,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(const __grid_cons
     auto inlet = [&](int y) { return make_double2(s_uxi[y], s_uyi[y]); };
     for (long long t = ((long long)warp * gridDim.x + blockIdx.x) * 32 + lane; t < a.n_near;
          t += (long long)gridDim.x * (kPairWarps * 32))
-      my_sum += near_cell<S, MODE_FAST, P, sizeof(T) == 2>(a, a.fsrc, a.fdst, a.write_macro, t, corr, inlet, &my_nan);
+      my_sum += near_cell<S, MODE_FAST, P, sizeof(T) == 2 || ODD>(a, a.fsrc, a.fdst, a.write_macro, t, corr, inlet, &my_nan);
     const float corrf = (float)corr;
     PairItem<T> it;
     it.nx = nx; it.np = nx / 2; it.pitch = pitch; it.magic = a.pair_magic;
@@ -471,8 +484,8 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(const __grid_cons
       it.dst = fd + (long long)it.r0 * (19 * pitch);
       const int chunks = (it.nr * it.np + 31) >> 5;
       if (deal < chunks) {
-        pair_item<S, P>(it, a, spop + (size_t)s * R * 19 * pitch, scls + (size_t)s * R * pitch, s_wall + s * R, deal,
-                        &empty[s], ends, inlet, lane, my_sum, my_nan);
+        pair_item<S, P, ODD>(it, a, spop + (size_t)s * R * 19 * pitch, scls + (size_t)s * R * pitch, s_wall + s * R, deal,
+                             &empty[s], ends, inlet, lane, my_sum, my_nan);
       } else {
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);

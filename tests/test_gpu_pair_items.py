@@ -77,6 +77,27 @@ def test_items_of_a_lattice(gpu_engine_cls, monkeypatch, dims, precision):
         x.close()
 
 
+ODD = [(5, 9, 8, False), (7, 9, 300, True), (63, 44, 31, False), (65, 7, 200, True), (129, 12, 400, False),
+       (385, 6, 5, True)]
+
+
+@pytest.mark.parametrize("precision", list(ULPS))
+@pytest.mark.parametrize("dims", ODD, ids=lambda d: f"{d[0]}x{d[1]}x{d[2]}")
+def test_rows_of_an_odd_cell_count_keep_their_bits(gpu_engine_cls, monkeypatch, dims, precision):
+    e = {}
+    for cpt in (1, 2):
+        monkeypatch.setenv("AEROSIM_CELLS_PER_THREAD", str(cpt))
+        e[cpt], flags = _lattice(*dims[:3], precision, dims[3])
+        e[cpt].step(1)
+    _compare(e[2], e[1], flags, precision)
+    for x in e.values():
+        x.step(2)
+    if precision != "f32":
+        assert np.array_equal(e[1].read_populations(), e[2].read_populations())
+    for x in e.values():
+        x.close()
+
+
 @pytest.mark.parametrize("precision", list(ULPS))
 @pytest.mark.parametrize("dims", [[(4, 5, 6), (34, 9, 40), (130, 12, 30)], [(66, 31, 21), (72, 7, 50)]],
                          ids=["pitches", "one_pitch"])
