@@ -176,10 +176,11 @@ int configure_step(aerosim_engine* h) {
   const bool half = h->cfg.precision == AEROSIM_PREC_F16S || h->cfg.precision == AEROSIM_PREC_BF16S ||
                     h->cfg.precision == AEROSIM_PREC_F16C;
   const bool fast = half || h->cfg.precision == AEROSIM_PREC_F32;
-  // two cells per consumer thread (packed FP32 pairs) without the closure on rows of 4 cells
-  // and more (with 3 both row ends would hang on one pair); AEROSIM_CELLS_PER_THREAD (1 or 2)
-  // overrides the choice for any fast-mode lattice that allows it
-  const bool pairs_fit = !mlp && L.nx >= 4;
+  // two cells per consumer thread (packed FP32 pairs) without the tcgen05 closure tiles (their
+  // groups of four warps walk the rows together) on rows of 4 cells and more (with 3 both row
+  // ends would hang on one pair); AEROSIM_CELLS_PER_THREAD (1 or 2) overrides the choice for
+  // any fast-mode lattice that allows it
+  const bool pairs_fit = mlp != 2 && L.nx >= 4;
   // two cells per thread vs one, us per step: 256x128x128 FP32 101.4 vs 108.4, F16S 60.3 vs
   // 80.6, BF16S 59.6 vs 80.4; 191x95x97 FP32 50.1 vs 58.4, BF16S 33.8 vs 43.8
   int cpt = (fast && pairs_fit) ? 2 : 1;
@@ -207,7 +208,7 @@ int configure_step(aerosim_engine* h) {
       item_rows = std::min(kMaxPairRows, std::max(1, atoi(ienv) * 256 / L.nx));
   }
   auto smem_for = [&](int S) {
-    return cpt == 2 ? pair_smem_bytes(L.pitch, L.ny, item_rows, S, eb) : step_smem_bytes(L, S, eb, mlp, groups);
+    return cpt == 2 ? pair_smem_bytes(L.pitch, L.ny, item_rows, S, eb, mlp == 1) : step_smem_bytes(L, S, eb, mlp, groups);
   };
   const char* env = getenv("AEROSIM_STAGES");
   const int forced = env ? atoi(env) : 0;

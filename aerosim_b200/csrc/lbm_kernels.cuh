@@ -566,8 +566,8 @@ __host__ __device__ inline size_t step_smem_bytes(const Layout& L, int stages, s
 // near-wall cells (Bouzidi, :196-221; one lane per cell from a link table built with
 // the voxel grid).  A near-wall cell at ix = 1 or nx-2 carries its row's inlet or
 // outlet, which need its post-collision values.  The last CTA takes the step's mean-density
-// rescale decision (:431-455).  Rows of an even cell count, in the FP32 arithmetic without the
-// closure, step two cells per thread instead (pair_kernel, lbm_pair_step.cuh).
+// rescale decision (:431-455).  In the FP32 arithmetic rows of 4 and more cells step two cells
+// per thread instead (pair_kernel, lbm_pair_step.cuh), except with the tcgen05 closure tiles.
 //
 // P is the row pitch when it is a compile-time constant (0: L.pitch at run time):
 // with a constant pitch every shared-memory load and global store of a cell is an

@@ -31,8 +31,8 @@ template <class S, int MODE, int P, int MLP = MLP_NONE, int CPT = 1>
 cudaError_t step_entry(const StepArgs& a, dim3 block, unsigned grid, size_t smem, cudaStream_t s, int* occ,
                        int* launches) {
   auto k = [] {
-    if constexpr (CPT == 3) return pair_kernel<S, P, true>;
-    else if constexpr (CPT == 2) return pair_kernel<S, P>;
+    if constexpr (CPT == 3) return pair_kernel<S, P, true, MLP == MLP_WARP>;
+    else if constexpr (CPT == 2) return pair_kernel<S, P, false, MLP == MLP_WARP>;
     else return main_kernel<S, MODE, P, MLP>;
   }();
   if (occ) {
@@ -60,7 +60,8 @@ cudaError_t step_entry(const StepArgs& a, dim3 block, unsigned grid, size_t smem
 // The FP32-arithmetic kernels are compiled for every row pitch up to 256 (multiples
 // of 32) with the pitch as a constant; other pitches and the double modes take the
 // run-time pitch.  With the learned closure (a.mlp_frag set): pitches 128 and 256, or
-// the run-time pitch, as warp-level mma.sync tiles; with a.mlp_umma set as well, the
+// the run-time pitch, as warp-level mma.sync tiles, two cells per thread from 4 cells a row
+// (256x128x128 FP32 220.5 us per step with one, 189.5 with two; 160x80x80 81.3 and 60.2); with a.mlp_umma set as well, the
 // 128-cell tcgen05 tiles, for pitches 128 and 256 (rows of 97..256 cells: every item
 // keeps all 8 consumer warps busy, two full groups of four).
 template <class S, int MODE>
@@ -75,10 +76,12 @@ cudaError_t step_dispatch(const StepArgs& a, dim3 block, unsigned grid, size_t s
       }
     }
     if (a.mlp_frag) {
+      if (a.cells_per_thread != 2) return step_entry<S, MODE, 0, MLP_WARP>(a, block, grid, smem, s, occ, launches);
+      if (a.L.nx % 2) return step_entry<S, MODE, 0, MLP_WARP, 3>(a, block, grid, smem, s, occ, launches);
       switch (a.L.pitch) {
-        case 128: return step_entry<S, MODE, 128, MLP_WARP>(a, block, grid, smem, s, occ, launches);
-        case 256: return step_entry<S, MODE, 256, MLP_WARP>(a, block, grid, smem, s, occ, launches);
-        default: return step_entry<S, MODE, 0, MLP_WARP>(a, block, grid, smem, s, occ, launches);
+        case 128: return step_entry<S, MODE, 128, MLP_WARP, 2>(a, block, grid, smem, s, occ, launches);
+        case 256: return step_entry<S, MODE, 256, MLP_WARP, 2>(a, block, grid, smem, s, occ, launches);
+        default: return step_entry<S, MODE, 0, MLP_WARP, 2>(a, block, grid, smem, s, occ, launches);
       }
     }
     if (a.cells_per_thread == 2 && a.L.nx % 2) {  // two cells per thread, a single outlet cell (odd nx)

@@ -9,6 +9,7 @@
 // one-cell-per-thread step (tests/test_gpu_pair_items.py).
 #pragma once
 #include "common.cuh"
+#include "sgs_mlp.cuh"
 
 namespace aerosim {
 
@@ -74,10 +75,19 @@ __device__ __forceinline__ void heq_pair(float2 (&v)[19], float2 r, float2 ux, f
 
 // h: the raw stored values of the two cells (x: first cell, y: second), replaced by the
 // post-collision values in the storage domain; r, u: the clamped, Mach-limited moments.
-// dec = (storage scale x pending rescale, rescale - 1) as in collide_fast.
-template <class S, bool FUSE = false>
+// dec = (storage scale x pending rescale, rescale - 1) as in collide_fast.  With MLP the
+// relaxation time comes from the learned closure (all 32 lanes call together): one tile
+// evaluation for the warp's first cells and one for the second.
+struct PairMlp {
+  const uint32_t* frag;  // shared memory
+  const float* bias;
+  uint32_t* stage;       // the warp's 32 x 8 BF16 staging block
+  float nu0;
+};
+template <class S, bool FUSE = false, bool MLP = false>
 __device__ __forceinline__ void collide_fast2(float2 (&h)[19], float2& r, float2& ux, float2& uy, float2& uz,
-                                              float tau0, float k_smag, float2 dec) {
+                                              float tau0, float k_smag, float2 dec, const PairMlp* m = nullptr,
+                                              uint32_t cls2 = 0, int lane = 0) {
   static_assert(S::kRawMoments, "the FP32 collision runs on stored deviations");
   constexpr float OS = S::kOutScale, OW = S::kOutW;
   constexpr float w0 = 1.0f / 3.0f, w1 = 1.0f / 18.0f, w2 = 1.0f / 36.0f;
@@ -128,7 +138,16 @@ __device__ __forceinline__ void collide_fast2(float2 (&h)[19], float2& r, float2
   const float2 pq = f2fma(pxx, pxx, f2fma(pyy, pyy, f2fma(pzz, pzz, f2mul(f2(2.0f), off))));
   const float2 pn = make_float2(sqrt_approx_(pq.x), sqrt_approx_(pq.y));
   const float2 arg = f2fma(f2(tau0), f2(tau0), f2mul(f2mul(f2(k_smag), pn), ir));
-  const float2 tau = f2mul(f2(0.5f), f2add(f2(tau0), make_float2(sqrt_approx_(arg.x), sqrt_approx_(arg.y))));
+  float2 tau = f2mul(f2(0.5f), f2add(f2(tau0), make_float2(sqrt_approx_(arg.x), sqrt_approx_(arg.y))));
+  if constexpr (MLP) {
+    float x[kMlpIn];
+    mlp_features(pxx.x, pyy.x, pzz.x, pxy.x, pxz.x, pyz.x, r.x, tau.x, (float)((cls2 & 0xffu) >> 3), x);
+    float tm = fmaf(3.0f * m->nu0, 1.0f + mlp_nut_warp(x, m->frag, m->bias, m->stage, lane), 0.5f);
+    if (tm == tm && tm < 1.0e30f) tau.x = tm;
+    mlp_features(pxx.y, pyy.y, pzz.y, pxy.y, pxz.y, pyz.y, r.y, tau.y, (float)((cls2 & 0xffffu) >> 11), x);
+    tm = fmaf(3.0f * m->nu0, 1.0f + mlp_nut_warp(x, m->frag, m->bias, m->stage, lane), 0.5f);
+    if (tm == tm && tm < 1.0e30f) tau.y = tm;
+  }
   const float2 om = make_float2(rcp_approx_(fmaxf(0.5015f, fminf(1.95f, tau.x))),
                                 rcp_approx_(fmaxf(0.5015f, fminf(1.95f, tau.y))));
   const float2 nom = f2neg(om);

@@ -1,6 +1,6 @@
 // The two-cells-per-thread step of a single lattice (pair_kernel) and the item loop it
-// shares with the batched step: FP32 arithmetic, no closure, rows of 4 and more cells (a batch:
-// of an even count).  With ODD the pairs cover cells 0 .. nx-2 and the outlet cell nx-1 follows
+// shares with the batched step: FP32 arithmetic, with MLP the learned closure as warp tiles,
+// rows of 4 and more cells (a batch: of an even count).  With ODD the pairs cover cells 0 .. nx-2 and the outlet cell nx-1 follows
 // the last of them.
 //
 // A work item is R consecutive x-rows; its pairs of cells form one list, and each consumer
@@ -49,12 +49,13 @@ __host__ inline int pair_rows(int nx, long long rows, int pairs, long long ctas)
 // Dynamic shared memory: a guard (a pull of cell 0's or nx-1's outer neighbour reads past
 // the row); the ring slots (R row blocks, then their class bytes); a guard; the barriers; the
 // inlet tables; the direction table of the row ends, a scratch row per consumer warp, the
-// directions' slots; per slot the rows' wall flags.
+// directions' slots; per slot the rows' wall flags; the closure's weights, biases and a staging
+// block per consumer warp.
 constexpr int kEndScratch = 23;
-__host__ __device__ inline size_t pair_smem_bytes(int pitch, int ny, int rows, int stages, size_t elem) {
+__host__ __device__ inline size_t pair_smem_bytes(int pitch, int ny, int rows, int stages, size_t elem, bool mlp = false) {
   return kSmemGuard + (size_t)stages * rows * pitch * (19 * elem + 1) + kSmemGuard + 16 * (size_t)stages +
          2 * (size_t)ny * sizeof(double) + 19 * sizeof(float4) + kPairWarps * kEndScratch * sizeof(float) + 19 +
-         (size_t)stages * rows + 16;
+         (size_t)stages * rows + 16 + (mlp ? 16 + (kMlpFragWords * 32 + kMlpBias + 3 + kPairWarps * 128) * 4 : 0);
 }
 
 // What a consumer warp needs of an item beyond its slot.
@@ -140,12 +141,13 @@ __device__ __forceinline__ void chunk_ends(const float2 (&v)[19], float2 r, floa
 // collision, stores, density sum, row ends.  (After the release only registers may be used:
 // the next fill overwrites the slot and the rows' flags.)  Near-wall cells are left to the
 // near-wall pass, solids are never written.
-template <class S, int P, bool ODD = false, class InletFn>
+template <class S, int P, bool ODD = false, bool MLP = false, class InletFn>
 __device__ __forceinline__ void pair_item(const PairItem<typename S::T>& it, const StepArgs& m, const typename S::T* slot,
                                           const uint8_t* cls, const uint8_t* wall, int first, uint64_t* empty,
                                           const EndTables& ends, InletFn inlet, int lane, long long& my_sum,
-                                          int& my_nan) {
+                                          int& my_nan, const PairMlp* mlp = nullptr) {
   using T = typename S::T;
+  constexpr bool FUSE = ODD || MLP;  // the arithmetic of the one-cell kernels
   const int pitch = P ? P : it.pitch;
   const int total = it.nr * it.np;
   for (int base = first * 32; base < total; base += kPairWarps * 32) {
@@ -173,13 +175,13 @@ __device__ __forceinline__ void pair_item(const PairItem<typename S::T>& it, con
       if (lane == 0) mbar_arrive(empty);
     }
     float2 r, ux, uy, uz;
-    collide_fast2<S, ODD>(v, r, ux, uy, uz, it.tau0, it.k_smag, it.dec);  // v: storage domain
+    collide_fast2<S, FUSE, MLP>(v, r, ux, uy, uz, it.tau0, it.k_smag, it.dec, mlp, cls2, lane);  // v: storage domain
     T* const out = it.dst + off;
     if (!__any_sync(0xffffffffu, act && ((cls2 & 0x0707u) != 0u || wall_row)) && !it.write_macro) {
       if (act) {
         if constexpr (S::kCompensate) {
           __half2 hv[19];
-          compensate_pair<S, ODD>(v, r, hv);
+          compensate_pair<S, FUSE>(v, r, hv);
 #pragma unroll
           for (int d = 0; d < 19; ++d) *reinterpret_cast<__half2*>(out + slot_of(d) * pitch) = hv[d];
         } else {
@@ -212,11 +214,11 @@ __device__ __forceinline__ void pair_item(const PairItem<typename S::T>& it, con
       }
       if (iy == it.ny - 1) uy = f2(0.0f);
       if (it.nz > 4 && (iz == 0 || iz == it.nz - 1)) uz = f2(0.0f);
-      heq_pair<S, ODD>(v, r, ux, uy, uz);
+      heq_pair<S, FUSE>(v, r, ux, uy, uz);
     }
     if constexpr (S::kCompensate) {
       __half2 hv[19];
-      compensate_pair<S, ODD>(v, r, hv);
+      compensate_pair<S, FUSE>(v, r, hv);
       if (own0 && own1) {
 #pragma unroll
         for (int d = 0; d < 19; ++d) *reinterpret_cast<__half2*>(out + slot_of(d) * pitch) = hv[d];
@@ -345,7 +347,7 @@ __device__ __forceinline__ void fill_end_tables(float4* dcw, uint8_t* dslot) {
 // One time step of one lattice: a producer warp fills the ring, the consumer warps first take
 // their near-wall cells, while the first slots fill, and then the chunks of the items; the
 // last CTA takes the rescale decision.
-template <class S, int P, bool ODD = false>
+template <class S, int P, bool ODD = false, bool MLP = false>
 __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(const __grid_constant__ StepArgs a) {
   using T = typename S::T;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -375,6 +377,15 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(const __grid_cons
   float* const s_xo = reinterpret_cast<float*>(s_dcw + 19);                                // [kPairWarps][kEndScratch]
   uint8_t* const s_dslot = reinterpret_cast<uint8_t*>(s_xo + kPairWarps * kEndScratch);    // [19]
   uint8_t* const s_wall = s_dslot + 19;                                                    // [S_][R]
+
+  uint32_t* const s_mfrag =
+      reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(s_wall + S_ * R) + 15) & ~uintptr_t(15));  // [24 * 32]
+  float* const s_mbias = reinterpret_cast<float*>(s_mfrag + kMlpFragWords * 32);   // [65]
+  uint32_t* const s_mstage = reinterpret_cast<uint32_t*>(s_mbias + kMlpBias + 3);  // [kPairWarps][128]
+  if constexpr (MLP) {
+    for (int i = threadIdx.x; i < kMlpFragWords * 32; i += blockDim.x) s_mfrag[i] = a.mlp_frag[i];
+    for (int i = threadIdx.x; i < kMlpBias; i += blockDim.x) s_mbias[i] = a.mlp_bias[i];
+  }
 
   const T* const fs = static_cast<const T*>(a.fsrc);
   T* const fd = static_cast<T*>(a.fdst);
@@ -461,7 +472,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(const __grid_cons
     auto inlet = [&](int y) { return make_double2(s_uxi[y], s_uyi[y]); };
     for (long long t = ((long long)warp * gridDim.x + blockIdx.x) * 32 + lane; t < a.n_near;
          t += (long long)gridDim.x * (kPairWarps * 32))
-      my_sum += near_cell<S, MODE_FAST, P, sizeof(T) == 2 || ODD>(a, a.fsrc, a.fdst, a.write_macro, t, corr, inlet, &my_nan);
+      my_sum += near_cell<S, MODE_FAST, P, sizeof(T) == 2 || ODD || MLP>(a, a.fsrc, a.fdst, a.write_macro, t, corr, inlet, &my_nan);
     const float corrf = (float)corr;
     PairItem<T> it;
     it.nx = nx; it.np = nx / 2; it.pitch = pitch; it.magic = a.pair_magic;
@@ -469,6 +480,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(const __grid_cons
     it.tau0 = (float)a.tau0; it.k_smag = (float)a.k_smag;
     it.dec = make_float2(corrf * S::kRawScale, corrf - 1.0f);  // raw-moment decode
     const EndTables ends{s_dcw, s_dslot, s_xo + warp * kEndScratch};
+    const PairMlp mlp{s_mfrag, s_mbias, s_mstage + warp * 128, a.mlp_nu0};
     int s = 0;
     uint32_t ph = 0;
     int deal = warp;  // this warp's first chunk of the item
@@ -484,8 +496,8 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(const __grid_cons
       it.dst = fd + (long long)it.r0 * (19 * pitch);
       const int chunks = (it.nr * it.np + 31) >> 5;
       if (deal < chunks) {
-        pair_item<S, P, ODD>(it, a, spop + (size_t)s * R * 19 * pitch, scls + (size_t)s * R * pitch, s_wall + s * R, deal,
-                             &empty[s], ends, inlet, lane, my_sum, my_nan);
+        pair_item<S, P, ODD, MLP>(it, a, spop + (size_t)s * R * 19 * pitch, scls + (size_t)s * R * pitch, s_wall + s * R, deal,
+                                  &empty[s], ends, inlet, lane, my_sum, my_nan, &mlp);
       } else {
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);

@@ -57,6 +57,7 @@ __host__ __device__ inline void mlp_features(float pxx, float pyy, float pzz, fl
 //   w 0..3        layer 1, N tile t:       (W1[n][k], W1[n][k+1]),  n = 8t + l/4, k = 2(l%4)
 //   w 4..19       layer 2, (kt, t, half):  (W2[n][k], W2[n][k+1]),  k = 16kt + 2(l%4) + 8 half
 //   w 20..23      layer 3, (kt, half):     (W3[k], W3[k+1]) for l/4 == 0, else 0
+// W2 and W3 are packed as halves: their inputs are twice the GELU (gelu2_bf16x2).
 // Biases: bias[0..31] = b1, bias[32..63] = b2, bias[64] = b3.
 constexpr int kMlpFragWords = 24;
 constexpr int kMlpBias = 65;
@@ -82,12 +83,12 @@ __host__ inline void mlp_pack_fragments(const float* P, uint32_t* frag /*[24 * 3
         for (int h = 0; h < 2; ++h) {
           const int n = 8 * t + n0, k = 16 * kt + k0 + 8 * h;
           frag[(4 + (kt * 4 + t) * 2 + h) * 32 + l] =
-              pair(P[kMlpW2 + n * kMlpHidden + k], P[kMlpW2 + n * kMlpHidden + k + 1]);
+              pair(0.5f * P[kMlpW2 + n * kMlpHidden + k], 0.5f * P[kMlpW2 + n * kMlpHidden + k + 1]);
         }
     for (int kt = 0; kt < 2; ++kt)
       for (int h = 0; h < 2; ++h) {
         const int k = 16 * kt + k0 + 8 * h;
-        frag[(20 + kt * 2 + h) * 32 + l] = n0 == 0 ? pair(P[kMlpW3 + k], P[kMlpW3 + k + 1]) : 0u;
+        frag[(20 + kt * 2 + h) * 32 + l] = n0 == 0 ? pair(0.5f * P[kMlpW3 + k], 0.5f * P[kMlpW3 + k + 1]) : 0u;
       }
   }
   for (int j = 0; j < 32; ++j) {
@@ -123,6 +124,19 @@ __device__ __forceinline__ uint32_t gelu_bf16x2(float a, float b) {
   asm("tanh.approx.bf16x2 %0, %1;" : "=r"(t) : "r"(u));
   asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(u) : "r"(x), "r"(0x3f003f00u));
   asm("fma.rn.bf16x2 %0, %1, %2, %1;" : "=r"(r) : "r"(u), "r"(t));
+  return r;
+}
+
+// Twice the GELU of a pair: x (1 + tanh(...)), the factor 1/2 (an exact scaling of BF16) in the
+// weights of the next layer instead of one more multiplication per pair.
+__device__ __forceinline__ uint32_t gelu2_bf16x2(float a, float b) {
+  const uint32_t x = bf16x2_of(a, b);
+  uint32_t x2, u, t, r;
+  asm("mul.rn.bf16x2 %0, %1, %1;" : "=r"(x2) : "r"(x));
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(u) : "r"(x2), "r"(0x3d123d12u), "r"(0x3f4c3f4cu));
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(u) : "r"(u), "r"(x));
+  asm("tanh.approx.bf16x2 %0, %1;" : "=r"(t) : "r"(u));
+  asm("fma.rn.bf16x2 %0, %1, %2, %1;" : "=r"(r) : "r"(x), "r"(t));
   return r;
 }
 
@@ -163,10 +177,10 @@ __device__ __forceinline__ float mlp_nut_warp(const float (&x)[kMlpIn], const ui
     for (int kt = 0; kt < 2; ++kt) {
       const float* lo = h[mt][2 * kt];
       const float* hi = h[mt][2 * kt + 1];
-      a2[mt][kt][0] = gelu_bf16x2(lo[0], lo[1]);
-      a2[mt][kt][1] = gelu_bf16x2(lo[2], lo[3]);
-      a2[mt][kt][2] = gelu_bf16x2(hi[0], hi[1]);
-      a2[mt][kt][3] = gelu_bf16x2(hi[2], hi[3]);
+      a2[mt][kt][0] = gelu2_bf16x2(lo[0], lo[1]);
+      a2[mt][kt][1] = gelu2_bf16x2(lo[2], lo[3]);
+      a2[mt][kt][2] = gelu2_bf16x2(hi[0], hi[1]);
+      a2[mt][kt][3] = gelu2_bf16x2(hi[2], hi[3]);
     }
   // layer 2: 32 -> 32
 #pragma unroll
@@ -191,10 +205,10 @@ __device__ __forceinline__ float mlp_nut_warp(const float (&x)[kMlpIn], const ui
     for (int kt = 0; kt < 2; ++kt) {
       const float* lo = h[mt][2 * kt];
       const float* hi = h[mt][2 * kt + 1];
-      a2[mt][kt][0] = gelu_bf16x2(lo[0], lo[1]);
-      a2[mt][kt][1] = gelu_bf16x2(lo[2], lo[3]);
-      a2[mt][kt][2] = gelu_bf16x2(hi[0], hi[1]);
-      a2[mt][kt][3] = gelu_bf16x2(hi[2], hi[3]);
+      a2[mt][kt][0] = gelu2_bf16x2(lo[0], lo[1]);
+      a2[mt][kt][1] = gelu2_bf16x2(lo[2], lo[3]);
+      a2[mt][kt][2] = gelu2_bf16x2(hi[0], hi[1]);
+      a2[mt][kt][3] = gelu2_bf16x2(hi[2], hi[3]);
     }
   // layer 3: 32 -> 1 (N padded to 8; column 0 is the output)
   float o[2][4];

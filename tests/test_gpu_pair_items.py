@@ -1,7 +1,7 @@
 """The two-cells-per-thread step at the edges of its work items: rows shorter and longer than
 a warp's 32 pairs, items that cross iz planes (also several of them), up to 16 rows an item, a
 ragged last item, solid and near-wall cells at the row ends and in every chunk, macro steps,
-batches of one and of several row pitches.
+batches of one and of several row pitches, rows of an odd cell count, the learned closure.
 
 Each lattice holds random solids and random populations; one step of it is compared with the
 one-cell-per-thread kernel's.  The two round differently: about 60 FP32 operations on values
@@ -12,7 +12,7 @@ direction 0.
 import numpy as np
 import pytest
 
-from aerosim_b200 import LBMBatch, LBMEngine, VoxelGridResult
+from aerosim_b200 import LBMBatch, LBMEngine, VoxelGridResult, sgs
 
 pytestmark = pytest.mark.gpu
 
@@ -48,10 +48,10 @@ def _lattice(nx, ny, nz, precision, ground):
     return e, flags
 
 
-def _compare(two, one, flags, precision):
+def _compare(two, one, flags, precision, tol=1e-6):
     a = two.read_populations().reshape(19, -1).astype(np.float64)
     b = one.read_populations().reshape(19, -1).astype(np.float64)
-    tol = 1e-6 + ULPS[precision] * np.abs(b - W[:, None])[:, flags != 1].max()
+    tol += ULPS[precision] * np.abs(b - W[:, None])[:, flags != 1].max()
     assert np.abs(a - b)[:, flags != 1].max() <= tol
     ma, mb = two.read_macro(), one.read_macro()
     for k in ("ux", "uy", "uz", "rho"):  # read from the same source lattice by both
@@ -94,6 +94,26 @@ def test_rows_of_an_odd_cell_count_keep_their_bits(gpu_engine_cls, monkeypatch, 
         x.step(2)
     if precision != "f32":
         assert np.array_equal(e[1].read_populations(), e[2].read_populations())
+    for x in e.values():
+        x.close()
+
+
+@pytest.mark.parametrize("precision", list(ULPS))
+@pytest.mark.parametrize("dims", [(4, 7, 3, False), (62, 9, 66, True), (66, 31, 21, False), (130, 12, 100, False),
+                                  (256, 6, 7, True), (5, 9, 8, False), (65, 7, 100, True)],
+                         ids=lambda d: f"{d[0]}x{d[1]}x{d[2]}")
+def test_items_with_the_closure(gpu_engine_cls, monkeypatch, dims, precision):
+    # an input that rounds to the neighbouring BF16 value (2^-8 of the eddy viscosity) moves a
+    # population by less than 4.5/18 |Pi| 2^-8, 1e-6 for the stresses here
+    e = {}
+    for cpt in (1, 2):
+        monkeypatch.setenv("AEROSIM_CELLS_PER_THREAD", str(cpt))
+        e[cpt], flags = _lattice(*dims[:3], precision, dims[3])
+        f = e[cpt].read_populations()
+        e[cpt].set_sgs_mlp(sgs.init_params(3))
+        e[cpt].write_populations(f)
+        e[cpt].step(1)
+    _compare(e[2], e[1], flags, precision, tol=2e-6)
     for x in e.values():
         x.close()
 
