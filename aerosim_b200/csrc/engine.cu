@@ -197,13 +197,14 @@ int configure_step(aerosim_engine* h) {
     const int want = atoi(genv);
     if (grouped && want >= 1 && want <= 4) groups = want;
   }
-  // two cells per thread: items of about 384 pairs with 16-bit storage and 192 with FP32, in
-  // up to 3 and 4 ring slots (256x128x128 F16S: 256 pairs 61.1-63.2 us per step, 384 60.3, 512
-  // 60.6; 128x64x64 FP32: 128 pairs 17.8, 192 16.5, 256 16.8)
+  // two cells per thread: items of about 384 pairs with 16-bit storage and 192 with FP32, 256
+  // with the closure too, in up to 3 and 4 ring slots (256x128x128 F16S: 256 pairs 61.1-63.2 us
+  // per step, 384 60.3, 512 60.6; 128x64x64 FP32: 128 pairs 17.8, 192 16.5, 256 16.8;
+  // 256x128x128 FP32 with the closure: 192 168.3, 256 162.5)
   const long long all_rows = (long long)L.ny * L.nz;
   int item_rows = 1;
   if (cpt == 2) {
-    item_rows = pair_rows(L.nx, all_rows, half ? 384 : 192, 2LL * h->num_sms);
+    item_rows = pair_rows(L.nx, all_rows, half ? 384 : (mlp ? 256 : 192), 2LL * h->num_sms);
     if (const char* ienv = getenv("AEROSIM_ITEM_GROUPS"))  // rows per item by hand, in units of 256 cells
       item_rows = std::min(kMaxPairRows, std::max(1, atoi(ienv) * 256 / L.nx));
   }

@@ -148,6 +148,15 @@ __device__ __forceinline__ float heq32(int d, float rho, float ux, float uy, flo
   return wf_of(d) * ((rho - 1.0f) + rho * (cu + 0.5f * cu * cu - 1.5f * uSq));
 }
 
+// The same with its contractions spelled out, u^2 from the y product on (FROM_Y) or from x.
+template <bool FROM_Y>
+__device__ __forceinline__ float heq32_fused(int d, float rho, float ux, float uy, float uz) {
+  const float cu = __fmul_rn(3.0f, dotc(d, ux, uy, uz));
+  const float uSq = __fmaf_rn(uz, uz, FROM_Y ? __fmaf_rn(ux, ux, __fmul_rn(uy, uy)) : __fmaf_rn(uy, uy, __fmul_rn(ux, ux)));
+  const float b = __fmaf_rn(-1.5f, uSq, __fmaf_rn(__fmul_rn(0.5f, cu), cu, cu));
+  return __fmul_rn(wf_of(d), __fmaf_rn(rho, b, __fsub_rn(rho, 1.0f)));
+}
+
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
 
@@ -553,7 +562,7 @@ __host__ __device__ inline size_t step_smem_bytes(const Layout& L, int stages, s
          16 * (size_t)stages + 2 * (size_t)L.ny * sizeof(double) +
          (size_t)stages * rows_per_item(L.nx) * groups * sizeof(int2) +
          kConsumerWarps * 24 * sizeof(float) + 16 + 19 * sizeof(float4) + 19 * sizeof(int) +
-         (mlp ? (kMlpFragWords * 32 + kMlpBias + 3 + kConsumerWarps * 128) * 4 : 0) +
+         (mlp ? 16 + (kMlpFragWords * 32 + kMlpBias + kConsumerWarps * 128) * 4 : 0) +
          (mlp == 2 ? kStepUmmaBytes : 0);
 }
 
@@ -611,8 +620,9 @@ __device__ __forceinline__ void wall_feq(typename std::conditional<MODE == MODE_
 // values before any wall condition), the wall condition when it applies, stores.
 // fsrc / fdst are the step's population buffers, inlet_u(iy) the inlet velocity
 // (double2) of row iy.  Returns the fixed-point density added to the step's sum; sets
-// *nan on a NaN.
-template <class S, int MODE, int P, bool YY = false, class InletFn>
+// *nan on a NaN.  FORM: the compiler's contractions (0), or those of the one-cell step spelled
+// out, u^2 of the deferred outlet from x (1) or y (2) on.
+template <class S, int MODE, int P, int FORM = 0, class InletFn>
 __device__ __forceinline__ long long near_cell(const StepArgs& a, const void* fsrc, void* fdst, int write_macro,
                                                long long t, double corr, InletFn inlet_u, int* nan) {
   using T = typename S::T;
@@ -657,7 +667,7 @@ __device__ __forceinline__ long long near_cell(const StepArgs& a, const void* fs
   Mac mr, mx, my, mz;
   {
     Real r, ux, uy, uz;
-    if constexpr (MODE == MODE_FAST) collide_f32<YY>(v, r, ux, uy, uz, (float)a.tau0, (float)a.k_smag);
+    if constexpr (MODE == MODE_FAST) collide_f32<FORM != 0>(v, r, ux, uy, uz, (float)a.tau0, (float)a.k_smag);
     else collide_f64<MODE == MODE_MIRROR, false>(v, r, ux, uy, uz, a.tau0, a.k_smag);
     mr = (Mac)r; mx = (Mac)ux; my = (Mac)uy; mz = (Mac)uz;
   }
@@ -693,12 +703,18 @@ __device__ __forceinline__ long long near_cell(const StepArgs& a, const void* fs
     T* out = blk + nx - 1;
     Mac ro;
     if constexpr (MODE == MODE_FAST) {
-      const float r2 = (float)mr * 0.85f + 0.15f;
+      const float r2 = FORM ? __fmaf_rn((float)mr, 0.85f, 0.15f) : (float)mr * 0.85f + 0.15f;
+      auto heq = [](int d, float rho, float x, float y, float z) {
+        return FORM ? heq32_fused<FORM == 2>(d, rho, x, y, z) : heq32(d, rho, x, y, z);
+      };
+      auto blend = [](float v, float q) {
+        return FORM ? __fmaf_rn(0.75f, v, __fmul_rn(0.25f, q)) : 0.75f * v + 0.25f * q;
+      };
       if constexpr (S::kCompensate) {
         float q[19];
 #pragma unroll
         for (int d = 0; d < 19; ++d)
-          q[d] = S::kOutScale * (0.75f * v[d] + 0.25f * heq32(d, r2, (float)mx, (float)my, (float)mz));
+          q[d] = S::kOutScale * blend(v[d], heq(d, r2, (float)mx, (float)my, (float)mz));
         compensate_cell<S>(q);
 #pragma unroll
         for (int d = 0; d < 19; ++d) out[slot_of(d) * pitch] = S::store(q[d]);
@@ -706,7 +722,7 @@ __device__ __forceinline__ long long near_cell(const StepArgs& a, const void* fs
 #pragma unroll
         for (int d = 0; d < 19; ++d)
           out[slot_of(d) * pitch] =
-              S::raw_of_h(0.75f * v[d] + 0.25f * heq32(d, r2, (float)mx, (float)my, (float)mz), d);
+              S::raw_of_h(blend(v[d], heq(d, r2, (float)mx, (float)my, (float)mz)), d);
       }
       ro = (Mac)r2;
     } else {
@@ -1147,9 +1163,10 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE, MLP>())
       (reinterpret_cast<uintptr_t>(s_xo + kConsumerWarps * 24) + 15) & ~uintptr_t(15));  // [19]
   int* s_dslot = reinterpret_cast<int*>(s_dcw + 19);                                     // [19]
   // learned closure: weight fragments, biases, one staging block per consumer warp
-  uint32_t* s_mfrag = reinterpret_cast<uint32_t*>(s_dslot + 19);                          // [24 * 32]
+  uint32_t* s_mfrag =
+      reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(s_dslot + 19) + 15) & ~uintptr_t(15));  // [24 * 32]
   float* s_mbias = reinterpret_cast<float*>(s_mfrag + kMlpFragWords * 32);               // [65]
-  uint32_t* s_mstage = reinterpret_cast<uint32_t*>(s_mbias + kMlpBias + 3);              // [8][128]
+  uint32_t* s_mstage = reinterpret_cast<uint32_t*>(s_mbias + kMlpBias);                  // [8][128]
   if constexpr (MLP != MLP_NONE) {
     for (int i = threadIdx.x; i < kMlpFragWords * 32; i += blockDim.x) s_mfrag[i] = a.mlp_frag[i];
     for (int i = threadIdx.x; i < kMlpBias; i += blockDim.x) s_mbias[i] = a.mlp_bias[i];
@@ -1253,7 +1270,8 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE, MLP>())
     long long t = (long long)blockIdx.x * 32 + lane;
     const long long t_step = (long long)gridDim.x * 32;
     for (; t < a.n_near; t += t_step)
-      my_sum += near_cell<S, MODE, P>(a, a.fsrc, a.fdst, a.write_macro, t, corr, inlet_d, &my_nan);
+      my_sum += near_cell<S, MODE, P, MODE != MODE_FAST ? 0 : S::kCompensate ? 2 : 1>(a, a.fsrc, a.fdst, a.write_macro, t,
+                                                                                      corr, inlet_d, &my_nan);
     if (__any_sync(0xffffffffu, my_nan) && lane == 0) nan_flag = 1;
     if (failed && lane == 0) atomicOr(&a.st->error, STEP_ERR_PIPELINE_TIMEOUT);
   } else if (warp == kProducerWarp) {

@@ -61,7 +61,7 @@ cudaError_t step_entry(const StepArgs& a, dim3 block, unsigned grid, size_t smem
 // of 32) with the pitch as a constant; other pitches and the double modes take the
 // run-time pitch.  With the learned closure (a.mlp_frag set): pitches 128 and 256, or
 // the run-time pitch, as warp-level mma.sync tiles, two cells per thread from 4 cells a row
-// (256x128x128 FP32 220.5 us per step with one, 189.5 with two; 160x80x80 81.3 and 60.2); with a.mlp_umma set as well, the
+// (256x128x128 FP32 220.5 us per step with one, 162.5 with two; 160x80x80 81.3 and 51.9); with a.mlp_umma set as well, the
 // 128-cell tcgen05 tiles, for pitches 128 and 256 (rows of 97..256 cells: every item
 // keeps all 8 consumer warps busy, two full groups of four).
 template <class S, int MODE>

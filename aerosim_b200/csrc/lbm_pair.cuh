@@ -77,7 +77,8 @@ __device__ __forceinline__ void heq_pair(float2 (&v)[19], float2 r, float2 ux, f
 // post-collision values in the storage domain; r, u: the clamped, Mach-limited moments.
 // dec = (storage scale x pending rescale, rescale - 1) as in collide_fast.  With MLP the
 // relaxation time comes from the learned closure (all 32 lanes call together): one tile
-// evaluation for the warp's first cells and one for the second.
+// evaluation for the warp's first cells and one for the second, as a loop (60 bytes of spills,
+// unrolled 296).
 struct PairMlp {
   const uint32_t* frag;  // shared memory
   const float* bias;
@@ -140,13 +141,17 @@ __device__ __forceinline__ void collide_fast2(float2 (&h)[19], float2& r, float2
   const float2 arg = f2fma(f2(tau0), f2(tau0), f2mul(f2mul(f2(k_smag), pn), ir));
   float2 tau = f2mul(f2(0.5f), f2add(f2(tau0), make_float2(sqrt_approx_(arg.x), sqrt_approx_(arg.y))));
   if constexpr (MLP) {
-    float x[kMlpIn];
-    mlp_features(pxx.x, pyy.x, pzz.x, pxy.x, pxz.x, pyz.x, r.x, tau.x, (float)((cls2 & 0xffu) >> 3), x);
-    float tm = fmaf(3.0f * m->nu0, 1.0f + mlp_nut_warp(x, m->frag, m->bias, m->stage, lane), 0.5f);
-    if (tm == tm && tm < 1.0e30f) tau.x = tm;
-    mlp_features(pxx.y, pyy.y, pzz.y, pxy.y, pxz.y, pyz.y, r.y, tau.y, (float)((cls2 & 0xffffu) >> 11), x);
-    tm = fmaf(3.0f * m->nu0, 1.0f + mlp_nut_warp(x, m->frag, m->bias, m->stage, lane), 0.5f);
-    if (tm == tm && tm < 1.0e30f) tau.y = tm;
+#pragma unroll 1
+    for (int c = 0; c < 2; ++c) {
+      float x[kMlpIn];
+      mlp_features(c ? pxx.y : pxx.x, c ? pyy.y : pyy.x, c ? pzz.y : pzz.x, c ? pxy.y : pxy.x, c ? pxz.y : pxz.x,
+                   c ? pyz.y : pyz.x, c ? r.y : r.x, c ? tau.y : tau.x, (float)((cls2 >> (8 * c) & 0xffu) >> 3), x);
+      const float tm = fmaf(3.0f * m->nu0, 1.0f + mlp_nut_warp(x, m->frag, m->bias, m->stage, lane), 0.5f);
+      if (tm == tm && tm < 1.0e30f) {
+        if (c) tau.y = tm;
+        else tau.x = tm;
+      }
+    }
   }
   const float2 om = make_float2(rcp_approx_(fmaxf(0.5015f, fminf(1.95f, tau.x))),
                                 rcp_approx_(fmaxf(0.5015f, fminf(1.95f, tau.y))));

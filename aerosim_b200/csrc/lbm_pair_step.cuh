@@ -15,9 +15,9 @@
 // What bounds it (ncu, 256x128x128): with 16-bit storage issue and fixed latencies at 20 warps
 // per SM (39.2 M warp instructions, 2.3 of 4 per cycle, DRAM 52 %), with FP32 DRAM (70 % cold,
 // 0.95 of the copy peak in a run of steps).  Microseconds per step, before -> with this kernel:
-// 256x128x128 F16S 68.5 -> 60.3, BF16S 69.5 -> 59.6, F16C 73.1 -> 64, FP32 101.6 -> 101.4;
+// 256x128x128 F16S 68.5 -> 58.2, BF16S 69.5 -> 59.6, F16C 73.1 -> 64, FP32 101.6 -> 101.0;
 // 160x80x80 F16S 28.2 -> 22.1; 200x100x96 F16S 43.1 -> 37.1; 128x64x64 FP32 20.3 -> 16.5;
-// 64x32x32 FP32 11.4 -> 9.6; 191x95x97 (one cell per thread before) BF16S 43.8 -> 33.8, FP32
+// 64x32x32 FP32 11.4 -> 9.3; 191x95x97 (one cell per thread before) BF16S 43.8 -> 33.8, FP32
 // 58.4 -> 50.1.  What made the difference: the bulk copies issued by one elected
 // lane from uniform registers, 37 an item of 4 rows (by 32 lanes they are replayed one by one,
 // about 20 instructions each, and the producer warp was the limit: 63.5 us), the flat pair
@@ -55,7 +55,13 @@ constexpr int kEndScratch = 23;
 __host__ __device__ inline size_t pair_smem_bytes(int pitch, int ny, int rows, int stages, size_t elem, bool mlp = false) {
   return kSmemGuard + (size_t)stages * rows * pitch * (19 * elem + 1) + kSmemGuard + 16 * (size_t)stages +
          2 * (size_t)ny * sizeof(double) + 19 * sizeof(float4) + kPairWarps * kEndScratch * sizeof(float) + 19 +
-         (size_t)stages * rows + 16 + (mlp ? 16 + (kMlpFragWords * 32 + kMlpBias + 3 + kPairWarps * 128) * 4 : 0);
+         (size_t)stages * rows + 16 + (mlp ? 16 + (kMlpFragWords * 32 + kMlpBias + kPairWarps * 128) * 4 : 0);
+}
+
+// p rounded up to 16 bytes, by its offset in the (aligned) shared memory: going through an
+// integer would leave the compiler with generic loads.
+__device__ __forceinline__ unsigned char* align16(unsigned char* base, void* p) {
+  return base + (((uint32_t)(static_cast<unsigned char*>(p) - base) + 15u) & ~15u);
 }
 
 // What a consumer warp needs of an item beyond its slot.
@@ -373,15 +379,14 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(const __grid_cons
   uint64_t* const empty = full + S_;
   double* const s_uxi = reinterpret_cast<double*>(empty + S_);
   double* const s_uyi = s_uxi + ny;
-  float4* const s_dcw = reinterpret_cast<float4*>((reinterpret_cast<uintptr_t>(s_uyi + ny) + 15) & ~uintptr_t(15));  // [19]
+  float4* const s_dcw = reinterpret_cast<float4*>(align16(smem_raw, s_uyi + ny));          // [19]
   float* const s_xo = reinterpret_cast<float*>(s_dcw + 19);                                // [kPairWarps][kEndScratch]
   uint8_t* const s_dslot = reinterpret_cast<uint8_t*>(s_xo + kPairWarps * kEndScratch);    // [19]
   uint8_t* const s_wall = s_dslot + 19;                                                    // [S_][R]
 
-  uint32_t* const s_mfrag =
-      reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(s_wall + S_ * R) + 15) & ~uintptr_t(15));  // [24 * 32]
+  uint32_t* const s_mfrag = reinterpret_cast<uint32_t*>(align16(smem_raw, s_wall + S_ * R));  // [24 * 32]
   float* const s_mbias = reinterpret_cast<float*>(s_mfrag + kMlpFragWords * 32);   // [65]
-  uint32_t* const s_mstage = reinterpret_cast<uint32_t*>(s_mbias + kMlpBias + 3);  // [kPairWarps][128]
+  uint32_t* const s_mstage = reinterpret_cast<uint32_t*>(s_mbias + kMlpBias);      // [kPairWarps][128]
   if constexpr (MLP) {
     for (int i = threadIdx.x; i < kMlpFragWords * 32; i += blockDim.x) s_mfrag[i] = a.mlp_frag[i];
     for (int i = threadIdx.x; i < kMlpBias; i += blockDim.x) s_mbias[i] = a.mlp_bias[i];
@@ -470,9 +475,10 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(const __grid_cons
     const int pslot = (a.step_index + 1) & 1;  // pending rescale of the previous step
     const double corr = a.st->apply[pslot] ? a.st->corr[pslot] : 1.0;
     auto inlet = [&](int y) { return make_double2(s_uxi[y], s_uyi[y]); };
+    constexpr int kForm = S::kCompensate && (ODD || MLP) ? 2 : (sizeof(T) == 2 || ODD || MLP) ? 1 : 0;
     for (long long t = ((long long)warp * gridDim.x + blockIdx.x) * 32 + lane; t < a.n_near;
          t += (long long)gridDim.x * (kPairWarps * 32))
-      my_sum += near_cell<S, MODE_FAST, P, sizeof(T) == 2 || ODD || MLP>(a, a.fsrc, a.fdst, a.write_macro, t, corr, inlet, &my_nan);
+      my_sum += near_cell<S, MODE_FAST, P, kForm>(a, a.fsrc, a.fdst, a.write_macro, t, corr, inlet, &my_nan);
     const float corrf = (float)corr;
     PairItem<T> it;
     it.nx = nx; it.np = nx / 2; it.pitch = pitch; it.magic = a.pair_magic;

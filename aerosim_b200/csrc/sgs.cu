@@ -320,9 +320,9 @@ __global__ void mlp_forward_kernel(const float* __restrict__ Pg, const float* __
 // 32 rows, rows past n evaluated on zeros and discarded.
 __global__ void mlp_forward_tc_kernel(const uint32_t* __restrict__ frag_g, const float* __restrict__ bias_g,
                                       const float* __restrict__ X, long long n, float* __restrict__ out) {
-  __shared__ uint32_t frag[kMlpFragWords * 32];
-  __shared__ float bias[kMlpBias];
-  __shared__ uint32_t stage[4][32 * 4];
+  __shared__ __align__(16) uint32_t frag[kMlpFragWords * 32];
+  __shared__ __align__(16) float bias[kMlpBias];
+  __shared__ __align__(16) uint32_t stage[4][32 * 4];
   for (int i = threadIdx.x; i < kMlpFragWords * 32; i += blockDim.x) frag[i] = frag_g[i];
   for (int i = threadIdx.x; i < kMlpBias; i += blockDim.x) bias[i] = bias_g[i];
   __syncthreads();
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kUmmaRows) mlp_forward_umma_kernel(const uint4
   uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + 16384 + 520);
   const int tid = threadIdx.x, warp = tid >> 5;
   for (int i = tid; i < kUmmaBBytes / 16; i += kUmmaRows) reinterpret_cast<uint4*>(sB)[i] = bimg[i];
-  for (int i = tid; i < kMlpBias; i += kUmmaRows) sbias[i] = bias_g[i];
+  for (int i = tid; i < 65; i += kUmmaRows) sbias[i] = bias_g[i];
   *reinterpret_cast<uint4*>(sA1 + umma_off(tid, 8, 16)) = make_uint4(0u, 0u, 0u, 0u);  // K padding
   const uint32_t mb = (uint32_t)__cvta_generic_to_shared(mbar);
   if (tid == 0) umma_mbar_init(mb);

@@ -52,15 +52,18 @@ __host__ __device__ inline void mlp_features(float pxx, float pyy, float pzz, fl
 // N tiles, the 8 inputs padded to K = 16.  The D fragments of a layer are, pair by
 // pair, the A fragments of the next, so activations never leave the registers.
 //
-// Weight fragments are pre-packed per lane (mlp_pack_fragments): word w of lane l at
-// frag[w * 32 + l] (a warp's load of one word touches 32 consecutive words):
-//   w 0..3        layer 1, N tile t:       (W1[n][k], W1[n][k+1]),  n = 8t + l/4, k = 2(l%4)
-//   w 4..19       layer 2, (kt, t, half):  (W2[n][k], W2[n][k+1]),  k = 16kt + 2(l%4) + 8 half
-//   w 20..23      layer 3, (kt, half):     (W3[k], W3[k+1]) for l/4 == 0, else 0
+// Weight fragments are pre-packed per lane (mlp_pack_fragments) in six 16-byte vectors:
+// word j of vector g of lane l at frag[(g * 32 + l) * 4 + j]:
+//   g 0           layer 1, j = N tile t:             (W1[n][k], W1[n][k+1]),  n = 8t + l/4, k = 2(l%4)
+//   g 1..4        layer 2, t = g - 1, j = 2kt+half:  (W2[n][k], W2[n][k+1]),  k = 16kt + 2(l%4) + 8 half
+//   g 5           layer 3, j = 2kt+half:             (W3[k], W3[k+1]) for l/4 == 0, else 0
 // W2 and W3 are packed as halves: their inputs are twice the GELU (gelu2_bf16x2).
-// Biases: bias[0..31] = b1, bias[32..63] = b2, bias[64] = b3.
+// Biases: bias[0..31] = b1, bias[32..63] = b2, bias[64] = b3; from kMlpBiasQuads on the
+// accumulators' start values of layer 1 and 2, N tile t, lanes l with l % 4 = q, as the vectors
+// (b[8t+2q], b[8t+2q+1], the same again) at 4 * (16 (layer - 1) + 4t + q).
 constexpr int kMlpFragWords = 24;
-constexpr int kMlpBias = 65;
+constexpr int kMlpBiasQuads = 68;
+constexpr int kMlpBias = kMlpBiasQuads + 128;
 
 __host__ inline uint16_t bf16_bits_rn(float f) {  // round to nearest even
   uint32_t u;
@@ -76,19 +79,19 @@ __host__ inline void mlp_pack_fragments(const float* P, uint32_t* frag /*[24 * 3
     const int k0 = 2 * (l % 4), n0 = l / 4;
     for (int t = 0; t < 4; ++t) {
       const int n = 8 * t + n0;
-      frag[t * 32 + l] = pair(P[kMlpW1 + n * kMlpIn + k0], P[kMlpW1 + n * kMlpIn + k0 + 1]);
+      frag[l * 4 + t] = pair(P[kMlpW1 + n * kMlpIn + k0], P[kMlpW1 + n * kMlpIn + k0 + 1]);
     }
     for (int kt = 0; kt < 2; ++kt)
       for (int t = 0; t < 4; ++t)
         for (int h = 0; h < 2; ++h) {
           const int n = 8 * t + n0, k = 16 * kt + k0 + 8 * h;
-          frag[(4 + (kt * 4 + t) * 2 + h) * 32 + l] =
+          frag[((1 + t) * 32 + l) * 4 + 2 * kt + h] =
               pair(0.5f * P[kMlpW2 + n * kMlpHidden + k], 0.5f * P[kMlpW2 + n * kMlpHidden + k + 1]);
         }
     for (int kt = 0; kt < 2; ++kt)
       for (int h = 0; h < 2; ++h) {
         const int k = 16 * kt + k0 + 8 * h;
-        frag[(20 + kt * 2 + h) * 32 + l] = n0 == 0 ? pair(0.5f * P[kMlpW3 + k], 0.5f * P[kMlpW3 + k + 1]) : 0u;
+        frag[(5 * 32 + l) * 4 + 2 * kt + h] = n0 == 0 ? pair(0.5f * P[kMlpW3 + k], 0.5f * P[kMlpW3 + k + 1]) : 0u;
       }
   }
   for (int j = 0; j < 32; ++j) {
@@ -96,16 +99,26 @@ __host__ inline void mlp_pack_fragments(const float* P, uint32_t* frag /*[24 * 3
     bias[32 + j] = P[kMlpB2 + j];
   }
   bias[64] = P[kMlpB3];
+  for (int j = 65; j < kMlpBiasQuads; ++j) bias[j] = 0.0f;
+  for (int i = 0; i < 128; ++i) {
+    const int layer = i / 64, t = i / 16 % 4, q = i / 4 % 4;
+    bias[kMlpBiasQuads + i] = bias[32 * layer + 8 * t + 2 * q + (i & 1)];
+  }
 }
 
 #ifdef __CUDACC__
+// D = A B + C; C in registers of its own, so that start values shared by tiles need no copies.
 __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                               uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+                                               uint32_t b0, uint32_t b1, const float4& c) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%10,%11,%12,%13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c.x), "f"(c.y), "f"(c.z), "f"(c.w));
+}
+__device__ __forceinline__ void mma_bf16_1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0, const float4& c) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%8,%9,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(b0), "f"(c.x), "f"(c.y), "f"(c.z), "f"(c.w));
 }
 __device__ __forceinline__ uint32_t bf16x2_of(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -140,17 +153,25 @@ __device__ __forceinline__ uint32_t gelu2_bf16x2(float a, float b) {
   return r;
 }
 
+// What bounds it (256x128x128 FP32 step, ncu): issue, about 900 instructions for 32 cells of the
+// closure and the step together, of them 64 MUFU.TANH (66 us of that unit) and 28 tensor
+// instructions (12 % of theirs).  Fragments and start values as 16-byte shared loads, the
+// accumulators' start values not copied and layer 1 at its own K took the two-cell step from
+// 189.5 to 168.3 us, and with items of 256 pairs to 162.5.
+//
 // nu_t / nu_0 of this lane's cell.  All 32 lanes must call it together.  x: the lane's
-// 8 inputs; frag / bias: the packed weights (shared memory); stage: 32 x 8 BF16 of
-// shared memory owned by the warp.
+// 8 inputs; frag / bias: the packed weights (shared memory, 16-byte aligned); stage: 32 x 8
+// BF16 of shared memory owned by the warp, 16-byte aligned.
 __device__ __forceinline__ float mlp_nut_warp(const float (&x)[kMlpIn], const uint32_t* __restrict__ frag,
                                               const float* __restrict__ bias, uint32_t* __restrict__ stage,
                                               int lane) {
   // inputs to the A-fragment layout through shared memory (row = cell, 4 words each)
-#pragma unroll
-  for (int i = 0; i < 4; ++i) stage[lane * 4 + i] = bf16x2_of(x[2 * i], x[2 * i + 1]);
+  reinterpret_cast<uint4*>(stage)[lane] =
+      make_uint4(bf16x2_of(x[0], x[1]), bf16x2_of(x[2], x[3]), bf16x2_of(x[4], x[5]), bf16x2_of(x[6], x[7]));
   __syncwarp();
   const int r = lane >> 2, q = lane & 3;
+  const uint4* const fv = reinterpret_cast<const uint4*>(frag) + lane;
+  const float4* const cv = reinterpret_cast<const float4*>(bias + kMlpBiasQuads) + q;
   uint32_t a1[2][2];
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt) {
@@ -158,17 +179,15 @@ __device__ __forceinline__ float mlp_nut_warp(const float (&x)[kMlpIn], const ui
     a1[mt][1] = stage[(16 * mt + r + 8) * 4 + q];
   }
   __syncwarp();
-  // layer 1: 8 (padded to 16) -> 32
+  // layer 1: 8 -> 32
   float h[2][4][4];
+  const uint4 w1 = fv[0];
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
-    const uint32_t b = frag[t * 32 + lane];
-    const float c0 = bias[8 * t + 2 * q], c1 = bias[8 * t + 2 * q + 1];
+    const float4 c = cv[4 * t];
+    const uint32_t b = t == 0 ? w1.x : t == 1 ? w1.y : t == 2 ? w1.z : w1.w;
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
-      h[mt][t][0] = c0; h[mt][t][1] = c1; h[mt][t][2] = c0; h[mt][t][3] = c1;
-      mma_bf16_16816(h[mt][t], a1[mt][0], a1[mt][1], 0u, 0u, b, 0u);
-    }
+    for (int mt = 0; mt < 2; ++mt) mma_bf16_1688(h[mt][t], a1[mt][0], a1[mt][1], b, c);
   }
   uint32_t a2[2][2][4];  // [mt][kt][reg]
 #pragma unroll
@@ -185,18 +204,13 @@ __device__ __forceinline__ float mlp_nut_warp(const float (&x)[kMlpIn], const ui
   // layer 2: 32 -> 32
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
-    const float c0 = bias[32 + 8 * t + 2 * q], c1 = bias[32 + 8 * t + 2 * q + 1];
+    const float4 c = cv[16 + 4 * t];
+    const uint4 w = fv[32 * (1 + t)];
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt) {
-      h[mt][t][0] = c0; h[mt][t][1] = c1; h[mt][t][2] = c0; h[mt][t][3] = c1;
-    }
-#pragma unroll
-    for (int kt = 0; kt < 2; ++kt) {
-      const uint32_t b0 = frag[(4 + (kt * 4 + t) * 2) * 32 + lane];
-      const uint32_t b1 = frag[(5 + (kt * 4 + t) * 2) * 32 + lane];
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
-        mma_bf16_16816(h[mt][t], a2[mt][kt][0], a2[mt][kt][1], a2[mt][kt][2], a2[mt][kt][3], b0, b1);
+      mma_bf16_16816(h[mt][t], a2[mt][0][0], a2[mt][0][1], a2[mt][0][2], a2[mt][0][3], w.x, w.y, c);
+      const float4 d = make_float4(h[mt][t][0], h[mt][t][1], h[mt][t][2], h[mt][t][3]);
+      mma_bf16_16816(h[mt][t], a2[mt][1][0], a2[mt][1][1], a2[mt][1][2], a2[mt][1][3], w.z, w.w, d);
     }
   }
 #pragma unroll
@@ -213,13 +227,13 @@ __device__ __forceinline__ float mlp_nut_warp(const float (&x)[kMlpIn], const ui
   // layer 3: 32 -> 1 (N padded to 8; column 0 is the output)
   float o[2][4];
   const float c3 = q == 0 ? bias[64] : 0.0f;
+  const uint4 w3 = fv[32 * 5];
 #pragma unroll
   for (int mt = 0; mt < 2; ++mt) {
-    o[mt][0] = c3; o[mt][1] = 0.0f; o[mt][2] = c3; o[mt][3] = 0.0f;
-#pragma unroll
-    for (int kt = 0; kt < 2; ++kt)
-      mma_bf16_16816(o[mt], a2[mt][kt][0], a2[mt][kt][1], a2[mt][kt][2], a2[mt][kt][3],
-                     frag[(20 + kt * 2) * 32 + lane], frag[(21 + kt * 2) * 32 + lane]);
+    mma_bf16_16816(o[mt], a2[mt][0][0], a2[mt][0][1], a2[mt][0][2], a2[mt][0][3], w3.x, w3.y,
+                   make_float4(c3, 0.0f, c3, 0.0f));
+    const float4 d = make_float4(o[mt][0], o[mt][1], o[mt][2], o[mt][3]);
+    mma_bf16_16816(o[mt], a2[mt][1][0], a2[mt][1][1], a2[mt][1][2], a2[mt][1][3], w3.z, w3.w, d);
   }
   // cell i's output sits in lane 4 (i % 8): o[i / 16][0] for i % 16 < 8, else o[i / 16][2]
   const int src = 4 * (lane & 7);
