@@ -349,8 +349,10 @@ __host__ __device__ inline size_t batch_pair_smem_bytes(long long slot_elems, lo
 // single lattice; density sums go to the instances' own state, and the last CTA takes every
 // instance's decision.  Launched as a programmatic dependent of the step before it (inside the
 // captured graphs too), so a step's prologue runs while the last CTAs of the step before finish.
-// 12 tunnels of 128x64x64 .. 172x86x86 (8.6 M cells, mixed row pitches): F16S 269 -> 219 us per
-// step, FP32 333 -> 298.  The run-time pitch costs about a quarter of the instructions.
+// 12 tunnels of 128x64x64 .. 172x86x86 (10.4 M cells, mixed row pitches): F16S 269 -> 206 us per
+// step (219 with the run-time pitch in the item loop and the instance's data read for every
+// item), FP32 333 -> 299 (0.81 of the copy peak).  With 16-bit storage waits bound it, for the
+// ring's two slots (half of the stalls); three smaller ones cost more per item (211 us).
 template <class S, int P>
 __global__ void __launch_bounds__(kPairThreads, 2) batch_pair_kernel(const __grid_constant__ BatchArgs b) {
   using T = typename S::T;
@@ -365,7 +367,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) batch_pair_kernel(const __gri
   uint8_t* const scls = smem_raw + kSmemGuard + (size_t)S_ * b.slot_elems * sizeof(T);
   uint64_t* const full = reinterpret_cast<uint64_t*>(scls + (size_t)S_ * b.slot_cls + kSmemGuard);
   uint64_t* const empty = full + S_;
-  float4* const s_dcw = reinterpret_cast<float4*>((reinterpret_cast<uintptr_t>(empty + S_) + 15) & ~uintptr_t(15));
+  float4* const s_dcw = reinterpret_cast<float4*>(align16(smem_raw, empty + S_));
   float* const s_xo = reinterpret_cast<float*>(s_dcw + 19);
   uint8_t* const s_dslot = reinterpret_cast<uint8_t*>(s_xo + kPairWarps * kEndScratch);
   uint8_t* const s_wall = s_dslot + 19;  // [S_][kMaxRowsPerItem]
@@ -462,6 +464,22 @@ __global__ void __launch_bounds__(kPairThreads, 2) batch_pair_kernel(const __gri
     int s = 0;
     uint32_t ph = 0;
     int deal = warp;
+    // The items come in the instances' order, so an instance's data stay in registers until the
+    // next one's first item; its density sum leaves the warp then.
+    int cur_inst = -1;
+    PairItem<T> it;
+    T* dst = nullptr;
+    long long sum = 0;
+    int nan = 0;
+    auto flush = [&] {
+      if (cur_inst < 0) return;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+      if (lane == 0 && sum) atomicAdd(&s_sum[cur_inst], (unsigned long long)sum);
+      if (__any_sync(0xffffffffu, nan) && lane == 0) b.pair[cur_inst].st->nan_seen = 1;
+      sum = 0;
+      nan = 0;
+    };
     for (;;) {
       const bool ok = mbar_wait(&full[s], ph, b.wait_limit);
       if (!__any_sync(0xffffffffu, ok)) {
@@ -470,29 +488,43 @@ __global__ void __launch_bounds__(kPairThreads, 2) batch_pair_kernel(const __gri
       }
       const int k = s_inst[s];
       if (k < 0) break;
-      const PairInst& in = b.pair[k];
-      PairItem<T> it;
-      it.r0 = s_first[s];
-      it.nr = s_rows[s];
-      it.np = in.np;
-      const int chunks = (it.nr * it.np + 31) >> 5;
-      if (deal < chunks) {
-        it.nx = in.nx; it.pitch = in.pitch; it.magic = in.magic;
+      if (k != cur_inst) {
+        flush();
+        cur_inst = k;
+        const PairInst& in = b.pair[k];
+        it.nx = in.nx; it.np = in.np; it.pitch = in.pitch; it.magic = in.magic;
         it.ny = in.ny; it.nz = in.nz; it.ground_no_slip = in.ground_no_slip; it.write_macro = b.write_macro;
         it.tau0 = in.tau0; it.k_smag = in.k_smag;
         const float corrf = in.st->apply[pslot] ? (float)in.st->corr[pslot] : 1.0f;
         it.dec = make_float2(corrf * S::kRawScale, corrf - 1.0f);  // raw-moment decode
-        const int pitch = P ? P : it.pitch;
-        it.dst = static_cast<T*>(in.buf[cur ^ 1]) + (long long)it.r0 * (19 * pitch);
+        dst = static_cast<T*>(in.buf[cur ^ 1]);
+      }
+      it.r0 = s_first[s];
+      it.nr = s_rows[s];
+      const int chunks = (it.nr * it.np + 31) >> 5;
+      if (deal < chunks) {
         const StepArgs& ia = b.inst[k];
-        long long sum = 0;
-        int nan = 0;
-        pair_item<S, P>(it, ia, spop + (size_t)s * b.slot_elems, scls + (size_t)s * b.slot_cls, s_wall + s * kMaxRowsPerItem,
-                        deal, &empty[s], ends, [&](int y) { return inlet_of(ia, y); }, lane, sum, nan);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
-        if (lane == 0 && sum) atomicAdd(&s_sum[k], (unsigned long long)sum);
-        if (__any_sync(0xffffffffu, nan) && lane == 0) in.st->nan_seen = 1;
+        auto run = [&](auto pc) {
+          constexpr int Q = decltype(pc)::value;
+          it.dst = dst + (long long)it.r0 * (19 * (Q ? Q : it.pitch));
+          pair_item<S, Q>(it, ia, spop + (size_t)s * b.slot_elems, scls + (size_t)s * b.slot_cls,
+                          s_wall + s * kMaxRowsPerItem, deal, &empty[s], ends,
+                          [&](int y) { return inlet_of(ia, y); }, lane, sum, nan);
+        };
+        if constexpr (P != 0) {
+          run(std::integral_constant<int, P>());
+        } else {  // mixed pitches: the constant-pitch code for each
+          switch (it.pitch) {
+            case 64: run(std::integral_constant<int, 64>()); break;
+            case 96: run(std::integral_constant<int, 96>()); break;
+            case 128: run(std::integral_constant<int, 128>()); break;
+            case 160: run(std::integral_constant<int, 160>()); break;
+            case 192: run(std::integral_constant<int, 192>()); break;
+            case 224: run(std::integral_constant<int, 224>()); break;
+            case 256: run(std::integral_constant<int, 256>()); break;
+            default: run(std::integral_constant<int, 0>());
+          }
+        }
       } else {
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[s]);
@@ -501,6 +533,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) batch_pair_kernel(const __gri
       if (deal < 0) deal += kPairWarps;
       if (++s == S_) { s = 0; ph ^= 1u; }
     }
+    flush();
     if (failed && lane == 0) atomicOr(b.error, STEP_ERR_PIPELINE_TIMEOUT);
   }
 
