@@ -181,8 +181,8 @@ int configure_step(aerosim_engine* h) {
   // ends would hang on one pair); AEROSIM_CELLS_PER_THREAD (1 or 2) overrides the choice for
   // any fast-mode lattice that allows it
   const bool pairs_fit = mlp != 2 && L.nx >= 4;
-  // two cells per thread vs one, us per step: 256x128x128 FP32 101.4 vs 108.4, F16S 60.3 vs
-  // 80.6, BF16S 59.6 vs 80.4; 191x95x97 FP32 50.1 vs 58.4, BF16S 33.8 vs 43.8
+  // two cells per thread vs one, us per step: 256x128x128 FP32 101.4 vs 108.4, F16S 58.4 vs
+  // 80.6, BF16S 58.5 vs 80.4; 191x95x97 FP32 50.1 vs 58.4, BF16S 33.8 vs 43.8
   int cpt = (fast && pairs_fit) ? 2 : 1;
   if (const char* cenv = getenv("AEROSIM_CELLS_PER_THREAD")) {
     const int want = atoi(cenv);

@@ -15,8 +15,8 @@
 // What bounds it (ncu, 256x128x128): with 16-bit storage issue and fixed latencies at 20 warps
 // per SM (39.2 M warp instructions, 2.3 of 4 per cycle, DRAM 52 %), with FP32 DRAM (70 % cold,
 // 0.95 of the copy peak in a run of steps).  Microseconds per step, before -> with this kernel:
-// 256x128x128 F16S 68.5 -> 58.2, BF16S 69.5 -> 59.6, F16C 73.1 -> 64, FP32 101.6 -> 101.0;
-// 160x80x80 F16S 28.2 -> 22.1; 200x100x96 F16S 43.1 -> 37.1; 128x64x64 FP32 20.3 -> 16.5;
+// 256x128x128 F16S 68.5 -> 58.2, BF16S 69.5 -> 58.5, F16C 73.1 -> 63.6, FP32 101.6 -> 101.0;
+// 160x80x80 F16S 28.2 -> 21.3; 200x100x96 F16S 43.1 -> 36.4; 128x64x64 FP32 20.3 -> 16.5;
 // 64x32x32 FP32 11.4 -> 9.3; 191x95x97 (one cell per thread before) BF16S 43.8 -> 33.8, FP32
 // 58.4 -> 50.1.  What made the difference: the bulk copies issued by one elected
 // lane from uniform registers, 37 an item of 4 rows (by 32 lanes they are replayed one by one,
