@@ -48,7 +48,8 @@ struct TriKey {
 // Host BVH build, bvh.ts:34-253: where the device build hands back a mesh whose split leaves
 // one side empty (the reference then halves the triangles in their current order, which
 // depends on every swap so far; it takes centroids a rounding apart, at coordinates above
-// 4096, or overflow) or a wait in it ran out.
+// 4096, or overflow), where a scanline's hits hold a NaN (scanline_hits_ordered) or a wait in
+// it ran out.
 // ---------------------------------------------------------------------------
 struct HostBvh {
   int tri_count = 0;
@@ -155,9 +156,11 @@ struct BvhView {
   const BvhNode* nodes;
   const int32_t* tidx;
   int tri_count;
+  int host_order;  // the triangles of a leaf stand in the host build's order
 };
 
-enum { VOX_ERR_STACK = 1, VOX_ERR_HITS = 2 };
+// VOX_NAN_HITS is no error: a NaN among a scanline's hits, in a tree of the device build.
+enum { VOX_ERR_STACK = 1, VOX_ERR_HITS = 2, VOX_NAN_HITS = 4 };
 
 // ---------------------------------------------------------------------------
 // Device BVH build.
@@ -491,6 +494,23 @@ __device__ __forceinline__ BvhNode load_node(const BvhNode* p) {
   return n;
 }
 
+// One triangle of bvh.ts:375-457 collectXScanlineHits; x is where the line meets it.
+__device__ __forceinline__ bool scanline_hit(const double* T, double py, double pz, double& x) {
+  const double ax = T[0], ay = T[1], az = T[2];
+  const double e1x = T[3], e1y = T[4], e1z = T[5];
+  const double e2x = T[6], e2y = T[7], e2z = T[8];
+  const double det = -e1y * e2z + e1z * e2y;
+  if (fabs(det) < 1e-13) return false;
+  const double inv = 1.0 / det;
+  const double ty = py - ay, tz = pz - az;
+  const double u = (-ty * e2z + tz * e2y) * inv;
+  if (u < 0.0 || u > 1.0) return false;
+  const double v = (ty * e1z - tz * e1y) * inv;
+  if (v < 0.0 || u + v > 1.0) return false;
+  x = ax + u * e1x + v * e2x;
+  return true;
+}
+
 // bvh.ts:375-457 collectXScanlineHits by a warp: up to 32 waiting nodes at a time, a lane
 // each; hits (unsorted) go to shared memory.  With the stack nearly full the warp takes one
 // node at a time, depth first, which needs at most kStack - 1 more entries (a deeper path is
@@ -515,20 +535,10 @@ __device__ int scanline_hits_warp(const BvhView& b, double y, double z, int* sta
       if (!(py < nd.lo[1] || py > nd.hi[1] || pz < nd.lo[2] || pz > nd.hi[2])) {
         if (nd.count > 0) {
           for (int i = nd.first; i < nd.first + nd.count; ++i) {
-            const double* T = b.tri + (size_t)b.tidx[i] * 9;
-            const double ax = T[0], ay = T[1], az = T[2];
-            const double e1x = T[3], e1y = T[4], e1z = T[5];
-            const double e2x = T[6], e2y = T[7], e2z = T[8];
-            const double det = -e1y * e2z + e1z * e2y;
-            if (fabs(det) < 1e-13) continue;
-            const double inv = 1.0 / det;
-            const double ty = py - ay, tz = pz - az;
-            const double u = (-ty * e2z + tz * e2y) * inv;
-            if (u < 0.0 || u > 1.0) continue;
-            const double v = (ty * e1z - tz * e1y) * inv;
-            if (v < 0.0 || u + v > 1.0) continue;
+            double x;
+            if (!scanline_hit(b.tri + (size_t)b.tidx[i] * 9, py, pz, x)) continue;
             const int at = atomicAdd(s_n, 1);
-            if (at < kMaxHits) hits[at] = ax + u * e1x + v * e2x;
+            if (at < kMaxHits) hits[at] = x;
             else atomicOr(err, VOX_ERR_HITS);
           }
         } else if (nd.left_turns + 2 > kStack) {
@@ -553,6 +563,41 @@ __device__ int scanline_hits_warp(const BvhView& b, double y, double z, int* sta
   }
   const int n = *s_n;
   return n < kMaxHits ? n : kMaxHits;
+}
+
+// The same by one thread, in the reference's order (leaves left to right, triangles as the host
+// build left them), and its insertion sort.  Hits that hold a NaN (a vertex without an x, as
+// damaged STL files have them) come out of a sort in an order that depends on the one they
+// came in, and so does what they fill.
+__device__ int scanline_hits_ordered(const BvhView& b, double y, double z, int* stack, double* hits, int* err) {
+  const double py = y + 1.37e-8, pz = z + 2.93e-8;
+  int sp = 0, n = 0;
+  stack[sp++] = 0;
+  while (sp > 0) {
+    const BvhNode nd = load_node(b.nodes + stack[--sp]);
+    if (py < nd.lo[1] || py > nd.hi[1] || pz < nd.lo[2] || pz > nd.hi[2]) continue;
+    if (nd.count == 0) {
+      if (sp + 2 > kStack) { atomicOr(err, VOX_ERR_STACK); return 0; }
+      stack[sp++] = nd.first + 1;
+      stack[sp++] = nd.first;
+      continue;
+    }
+    for (int i = nd.first; i < nd.first + nd.count; ++i) {
+      double x;
+      if (!scanline_hit(b.tri + (size_t)b.tidx[i] * 9, py, pz, x)) continue;
+      if (n < kMaxHits) hits[n] = x;
+      else atomicOr(err, VOX_ERR_HITS);
+      ++n;
+    }
+  }
+  n = n < kMaxHits ? n : kMaxHits;
+  for (int i = 1; i < n; ++i) {
+    const double key = hits[i];
+    int j = i - 1;
+    while (j >= 0 && hits[j] > key) { hits[j + 1] = hits[j]; --j; }
+    hits[j + 1] = key;
+  }
+  return n;
 }
 
 // bvh.ts:499-589 countRayIntersections
@@ -741,11 +786,20 @@ __global__ void __launch_bounds__(kScanWarps * 32) scan_fill_kernel(BvhView b, L
   // ascending numeric sort by rank (equal hits in any order: they are the same number)
   const double* const raw = s_hits[warp][0];
   double* const hits = s_hits[warp][1];
+  bool nan = false;
   for (int i = lane; i < hc; i += 32) {
     const double v = raw[i];
     int rank = 0;
     for (int j = 0; j < hc; ++j) rank += raw[j] < v || (raw[j] == v && j < i);
     hits[rank] = v;
+    nan |= v != v;
+  }
+  if (__any_sync(0xffffffffu, nan)) {  // ranks are none
+    if (!b.host_order) {  // the host starts over with its own tree
+      if (lane == 0) atomicOr(err, VOX_NAN_HITS);
+      return;
+    }
+    if (lane == 0) scanline_hits_ordered(b, y, z, s_stack[warp], hits, err);
   }
   __syncwarp();
   uint8_t* row = flags + (long long)L.nx * (iy + (long long)L.ny * iz);
@@ -965,7 +1019,19 @@ int run_voxelizer(const float* pos, int64_t nverts, const int32_t* idx, int64_t 
   *total = 0;
   *h_solid = 0;
   *h_err = 0;
-  const BvhView bv{d_tri, d_nodes, d_tidx, T};
+  BvhView bv{d_tri, d_nodes, d_tidx, T, 0};
+  auto host_tree = [&]() -> cudaError_t {
+    HostBvh hb;
+    hb.build(pos, nverts, idx, nidx, world16);
+    std::vector<BvhNode> nodes;
+    host_nodes(hb, &nodes);
+    cudaError_t e = cudaMemcpyAsync(d_nodes, nodes.data(), nodes.size() * sizeof(BvhNode), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_tidx, hb.tidx.data(), hb.tidx.size() * 4, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    *h_root = nodes[0];
+    bv.host_order = 1;
+    return e;
+  };
   double bmin[3] = {INFINITY, INFINITY, INFINITY}, bmax[3] = {-INFINITY, -INFINITY, -INFINITY};
   if (T > 0) {
     VCHECK(cudaMemcpyAsync(d_pos, pos, (size_t)nverts * 12, cudaMemcpyHostToDevice, s));
@@ -995,16 +1061,7 @@ int run_voxelizer(const float* pos, int64_t nverts, const int32_t* idx, int64_t 
     VCHECK(cudaMemcpyAsync(h_build, d_build, sizeof(BuildState), cudaMemcpyDeviceToHost, s));
     VCHECK(cudaMemcpyAsync(h_root, d_nodes, sizeof(BvhNode), cudaMemcpyDeviceToHost, s));
     VCHECK(cudaStreamSynchronize(s));
-    if (h_build->error) {
-      HostBvh hb;
-      hb.build(pos, nverts, idx, nidx, world16);
-      std::vector<BvhNode> nodes;
-      host_nodes(hb, &nodes);
-      VCHECK(cudaMemcpyAsync(d_nodes, nodes.data(), nodes.size() * sizeof(BvhNode), cudaMemcpyHostToDevice, s));
-      VCHECK(cudaMemcpyAsync(d_tidx, hb.tidx.data(), hb.tidx.size() * 4, cudaMemcpyHostToDevice, s));
-      VCHECK(cudaStreamSynchronize(s));
-      *h_root = nodes[0];
-    }
+    if (h_build->error) VCHECK(host_tree());
     for (int a = 0; a < 3; ++a) {  // the mesh bounds are the root's box
       bmin[a] = h_root->lo[a];
       bmax[a] = h_root->hi[a];
@@ -1026,35 +1083,42 @@ int run_voxelizer(const float* pos, int64_t nverts, const int32_t* idx, int64_t 
   long long brows = 0;
   int sx0 = 0, sy0 = 0, sz0 = 0, wx = 0, wy = 0;
   unsigned bgrid = 0;
-  if (T > 0) {
-    // STEP 1 (window may be empty when the mesh lies outside the lattice)
-    const long long rows = (long long)(L.w[3] - L.w[2] + 1) * (L.w[5] - L.w[4] + 1);
-    if (L.w[0] <= L.w[1] && L.w[2] <= L.w[3] && L.w[4] <= L.w[5] && rows > 0) {
-      scan_fill_kernel<<<(unsigned)((rows + kScanWarps - 1) / kScanWarps), kScanWarps * 32, 0, s>>>(bv, L, g->flags, d_solid, d_err);
-      VCHECK(cudaGetLastError());
+  for (;;) {
+    if (T > 0) {
+      // STEP 1 (window may be empty when the mesh lies outside the lattice)
+      const long long rows = (long long)(L.w[3] - L.w[2] + 1) * (L.w[5] - L.w[4] + 1);
+      if (L.w[0] <= L.w[1] && L.w[2] <= L.w[3] && L.w[4] <= L.w[5] && rows > 0) {
+        scan_fill_kernel<<<(unsigned)((rows + kScanWarps - 1) / kScanWarps), kScanWarps * 32, 0, s>>>(bv, L, g->flags, d_solid, d_err);
+        VCHECK(cudaGetLastError());
+      }
+      // STEP 2
+      sx0 = std::max(0, L.w[0] - 1); sy0 = std::max(0, L.w[2] - 1); sz0 = std::max(0, L.w[4] - 1);
+      // cells along each axis of the window +-1, none when the mesh lies outside the lattice;
+      // a mesh whose bounds leave the int range can make them wrap, which is refused
+      const long long cx = std::min<long long>(nx - 1, (long long)L.w[1] + 1) - sx0 + 1,
+                      cy = std::min<long long>(ny - 1, (long long)L.w[3] + 1) - sy0 + 1,
+                      cz = std::min<long long>(nz - 1, (long long)L.w[5] + 1) - sz0 + 1;
+      if (cx < INT_MIN || cy < INT_MIN || cz < INT_MIN) {
+        *err = "voxelizer: the mesh's bounds are out of range of the lattice's cell indices";
+        return -3;
+      }
+      brows = (cx > 0 && cy > 0 && cz > 0) ? cy * cz : 0;
+      wx = (int)cx;
+      wy = (int)cy;
+      if (brows > 0) {
+        bgrid = (unsigned)((brows * 32 + 255) / 256);
+        boundary_rows_kernel<<<bgrid, 256, 0, s>>>(g->flags, L, sx0, sy0, sz0, wx, wy, brows, d_rows, nullptr, nullptr, nullptr);
+        VCHECK(launch_scan_rows(d_rows, brows, w->host, s));
+      }
     }
-    // STEP 2
-    sx0 = std::max(0, L.w[0] - 1); sy0 = std::max(0, L.w[2] - 1); sz0 = std::max(0, L.w[4] - 1);
-    // cells along each axis of the window +-1, none when the mesh lies outside the lattice;
-    // a mesh whose bounds leave the int range can make them wrap, which is refused
-    const long long cx = std::min<long long>(nx - 1, (long long)L.w[1] + 1) - sx0 + 1,
-                    cy = std::min<long long>(ny - 1, (long long)L.w[3] + 1) - sy0 + 1,
-                    cz = std::min<long long>(nz - 1, (long long)L.w[5] + 1) - sz0 + 1;
-    if (cx < INT_MIN || cy < INT_MIN || cz < INT_MIN) {
-      *err = "voxelizer: the mesh's bounds are out of range of the lattice's cell indices";
-      return -3;
-    }
-    brows = (cx > 0 && cy > 0 && cz > 0) ? cy * cz : 0;
-    wx = (int)cx;
-    wy = (int)cy;
-    if (brows > 0) {
-      bgrid = (unsigned)((brows * 32 + 255) / 256);
-      boundary_rows_kernel<<<bgrid, 256, 0, s>>>(g->flags, L, sx0, sy0, sz0, wx, wy, brows, d_rows, nullptr, nullptr, nullptr);
-      VCHECK(launch_scan_rows(d_rows, brows, w->host, s));
-    }
+    VCHECK(cudaMemcpyAsync(h_solid, d_solid, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    VCHECK(cudaMemcpyAsync(h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    VCHECK(cudaStreamSynchronize(s));
+    if (!(*h_err & VOX_NAN_HITS)) break;  // the kernel does not set it in a tree of the host
+    VCHECK(host_tree());
+    VCHECK(cudaMemsetAsync(g->flags, 0, N, s));
+    VCHECK(cudaMemsetAsync(counters, 0, 16, s));  // d_solid, d_err
   }
-  VCHECK(cudaMemcpyAsync(h_solid, d_solid, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-  VCHECK(cudaStreamSynchronize(s));
   const long long B = (long long)*total;
   g->B = B;
   g->solid = (long long)*h_solid;
