@@ -1086,23 +1086,26 @@ int run_voxelizer(const float* pos, int64_t nverts, const int32_t* idx, int64_t 
   for (;;) {
     if (T > 0) {
       // STEP 1 (window may be empty when the mesh lies outside the lattice)
-      const long long rows = (long long)(L.w[3] - L.w[2] + 1) * (L.w[5] - L.w[4] + 1);
+      const long long rows = ((long long)L.w[3] - L.w[2] + 1) * ((long long)L.w[5] - L.w[4] + 1);
       if (L.w[0] <= L.w[1] && L.w[2] <= L.w[3] && L.w[4] <= L.w[5] && rows > 0) {
         scan_fill_kernel<<<(unsigned)((rows + kScanWarps - 1) / kScanWarps), kScanWarps * 32, 0, s>>>(bv, L, g->flags, d_solid, d_err);
         VCHECK(cudaGetLastError());
       }
       // STEP 2
       sx0 = std::max(0, L.w[0] - 1); sy0 = std::max(0, L.w[2] - 1); sz0 = std::max(0, L.w[4] - 1);
-      // cells along each axis of the window +-1, none when the mesh lies outside the lattice;
-      // a mesh whose bounds leave the int range can make them wrap, which is refused
+      // cells along each axis of the window +-1, none when the mesh lies outside the lattice
+      // along any of them; bounds that leave the int range can make a count wrap, which is
+      // refused unless another axis leaves the window empty
       const long long cx = std::min<long long>(nx - 1, (long long)L.w[1] + 1) - sx0 + 1,
                       cy = std::min<long long>(ny - 1, (long long)L.w[3] + 1) - sy0 + 1,
                       cz = std::min<long long>(nz - 1, (long long)L.w[5] + 1) - sz0 + 1;
-      if (cx < INT_MIN || cy < INT_MIN || cz < INT_MIN) {
+      const auto none = [](long long n) { return n <= 0 && n >= INT_MIN; };
+      const bool empty = none(cx) || none(cy) || none(cz);
+      if (!empty && (cx < INT_MIN || cy < INT_MIN || cz < INT_MIN)) {
         *err = "voxelizer: the mesh's bounds are out of range of the lattice's cell indices";
         return -3;
       }
-      brows = (cx > 0 && cy > 0 && cz > 0) ? cy * cz : 0;
+      brows = empty ? 0 : cy * cz;
       wx = (int)cx;
       wy = (int)cy;
       if (brows > 0) {
