@@ -427,7 +427,7 @@ int aerosim_create(int device, aerosim_engine** out) {
   if (e == cudaSuccess) e = cudaMalloc(&h->force_ticket, sizeof(unsigned int));
   if (e == cudaSuccess) e = cudaMalloc(&h->force_out, 8 * sizeof(double));
   if (e == cudaSuccess) e = cudaMalloc(&h->stats_buf, 4 * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = cudaMemset(h->force_ticket, 0, sizeof(unsigned int));
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->force_ticket, 0, sizeof(unsigned int), h->stream);
   if (e != cudaSuccess) {
     std::string msg = std::string("aerosim_create: ") + cudaGetErrorString(e);
     aerosim_destroy(h);
@@ -578,13 +578,15 @@ int aerosim_set_voxel_grid(aerosim_engine* h, int32_t nx, int32_t ny, int32_t nz
       const float v = q[b * 18 + k];
       if (v > 0.0f && v < mq[b]) mq[b] = v;
     }
-  if ((e = cudaMemcpy(ng.flags, flags, N, cudaMemcpyHostToDevice)) != cudaSuccess) return bad(e);
-  if ((e = cudaMemcpy(ng.bmap, bmap, N * 4, cudaMemcpyHostToDevice)) != cudaSuccess) return bad(e);
-  if (B > 0) {
-    if ((e = cudaMemcpy(ng.bcells, bcells, B * 4, cudaMemcpyHostToDevice)) != cudaSuccess) return bad(e);
-    if ((e = cudaMemcpy(ng.q, q, B * 18 * 4, cudaMemcpyHostToDevice)) != cudaSuccess) return bad(e);
-    if ((e = cudaMemcpy(ng.minq, mq.data(), B * 4, cudaMemcpyHostToDevice)) != cudaSuccess) return bad(e);
-  }
+  // on the engine's stream, which builds the link table from these arrays (it does not wait
+  // for the default stream); install_grid drains it before the host arrays go
+  auto up = [&](void* d, const void* p, size_t n) { return cudaMemcpyAsync(d, p, n, cudaMemcpyHostToDevice, h->stream); };
+  e = up(ng.flags, flags, N);
+  if (e == cudaSuccess) e = up(ng.bmap, bmap, N * 4);
+  if (e == cudaSuccess && B > 0) e = up(ng.bcells, bcells, B * 4);
+  if (e == cudaSuccess && B > 0) e = up(ng.q, q, B * 18 * 4);
+  if (e == cudaSuccess && B > 0) e = up(ng.minq, mq.data(), B * 4);
+  if (e != cudaSuccess) return bad(e);
   const double org[3] = {ng.ox, ng.oy, ng.oz};
   const int rc = install_grid(h, ng, dx, org, reset_flow);
   grid_free(&ng);
@@ -1113,9 +1115,10 @@ int aerosim_set_sgs_mlp(aerosim_engine* h, const float* params) {
       CU(h, cudaMalloc(&h->mlp_bias, bias.size() * sizeof(float)));
       CU(h, cudaMalloc(&h->mlp_umma, kUmmaBBytes));
     }
-    CU(h, cudaMemcpy(h->mlp_frag, frag.data(), frag.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    CU(h, cudaMemcpy(h->mlp_bias, bias.data(), bias.size() * sizeof(float), cudaMemcpyHostToDevice));
-    CU(h, cudaMemcpy(h->mlp_umma, img.data(), kUmmaBBytes, cudaMemcpyHostToDevice));
+    CU(h, cudaMemcpyAsync(h->mlp_frag, frag.data(), frag.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
+    CU(h, cudaMemcpyAsync(h->mlp_bias, bias.data(), bias.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream));
+    CU(h, cudaMemcpyAsync(h->mlp_umma, img.data(), kUmmaBBytes, cudaMemcpyHostToDevice, h->stream));
+    CU(h, cudaStreamSynchronize(h->stream));
     if (h->have_grid) {
       int rc = ensure_wall_distance(h);
       if (rc) return rc;
@@ -1323,8 +1326,9 @@ int batch_build_items(aerosim_batch* b, int item_cells) {
     slot_elems = std::max<long long>(slot_elems, (long long)RY * 19 * L.pitch);
     slot_cls = std::max<long long>(slot_cls, (long long)RY * L.pitch);
   }
-  BCU(cudaMemcpy(b->d_item_begin, item_begin.data(), item_begin.size() * sizeof(long long), cudaMemcpyHostToDevice));
-  BCU(cudaMemcpy(b->d_geo, geo.data(), geo.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  BCU(cudaMemcpyAsync(b->d_item_begin, item_begin.data(), item_begin.size() * sizeof(long long), cudaMemcpyHostToDevice, b->stream));
+  BCU(cudaMemcpyAsync(b->d_geo, geo.data(), geo.size() * sizeof(int4), cudaMemcpyHostToDevice, b->stream));
+  BCU(cudaStreamSynchronize(b->stream));
   b->n_items = item_begin[n];
   b->item_begin = item_begin;
   b->item_rows = rows_of;
@@ -1508,9 +1512,9 @@ int aerosim_batch_create(aerosim_engine* const* engines, int32_t n, aerosim_batc
   if (e == cudaSuccess) e = cudaMalloc(&b->d_step, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_error, sizeof(int));
   if (e == cudaSuccess)
-    e = cudaMemcpy(b->d_bufs, bufs.data(), bufs.size() * sizeof(void*), cudaMemcpyHostToDevice);
+    e = cudaMemcpyAsync(b->d_bufs, bufs.data(), bufs.size() * sizeof(void*), cudaMemcpyHostToDevice, b->stream);
   if (e == cudaSuccess)
-    e = cudaMemcpy(b->d_near_begin, near_begin.data(), near_begin.size() * sizeof(long long), cudaMemcpyHostToDevice);
+    e = cudaMemcpyAsync(b->d_near_begin, near_begin.data(), near_begin.size() * sizeof(long long), cudaMemcpyHostToDevice, b->stream);
   if (e != cudaSuccess) {
     bfail(AEROSIM_ERR_CUDA, std::string("batch_create: ") + cudaGetErrorString(e));
     return bail(AEROSIM_ERR_CUDA);
