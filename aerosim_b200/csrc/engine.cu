@@ -101,9 +101,11 @@ int fail(aerosim_engine* h, int code, const std::string& msg) {
 #define CU(h, x)                                                                          \
   do {                                                                                    \
     cudaError_t e_ = (x);                                                                 \
-    if (e_ != cudaSuccess)                                                                \
+    if (e_ != cudaSuccess) {                                                              \
+      cudaGetLastError(); /* reported here: not by the next launch's check too */         \
       return fail(h, e_ == cudaErrorMemoryAllocation ? AEROSIM_ERR_NOMEM : AEROSIM_ERR_CUDA, \
                   std::string(#x) + ": " + cudaGetErrorString(e_));                       \
+    }                                                                                     \
   } while (0)
 
 // A grid to build into: the spare arrays, if there are any.
@@ -275,6 +277,7 @@ int ensure_pops(aerosim_engine* h, bool* reallocated) {
     h->vox.release();
     e = alloc_pops(h);
   }
+  if (e != cudaSuccess) free_pops(h);  // never some of the buffers
   CU(h, e);
   h->f_prec = h->cfg.precision;
   h->f_cells = N;
@@ -616,7 +619,7 @@ int aerosim_get_config(aerosim_engine* h, aerosim_config* cfg) {
 
 int aerosim_reset_flow(aerosim_engine* h) {
   if (!h) return AEROSIM_ERR_ARG;
-  if (!h->have_grid) return fail(h, AEROSIM_ERR_STATE, "reset_flow: no voxel grid");
+  if (!h->have_grid || !h->f[0]) return fail(h, AEROSIM_ERR_STATE, "reset_flow: no voxel grid");
   CU(h, cudaSetDevice(h->device));
   return do_reset(h);
 }
