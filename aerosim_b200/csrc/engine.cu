@@ -20,6 +20,18 @@
 
 using namespace aerosim;
 
+// Launch shape of the persistent step kernel (plan_step).
+struct StepLaunch {
+  dim3 block{256, 1, 1};
+  unsigned grid = 1;
+  size_t smem = 0;
+  int stages = 3;
+  int item_groups = 1;       // row groups per work item
+  int cells_per_thread = 1;  // consumer cells per thread (1 or 2)
+  int item_rows = 1;         // two cells per thread: x-rows per work item
+  int dynamic_items = 1;     // work items from a device counter (1) or dealt round-robin (0)
+};
+
 struct aerosim_engine {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -35,24 +47,15 @@ struct aerosim_engine {
   int f_prec = -1;
   long long f_cells = 0;
   Layout L{};
-  // persistent step-kernel launch shape
-  dim3 block{256, 1, 1};
-  unsigned grid = 1;
-  size_t smem = 0;
-  int stages = 3;
-  int item_groups = 1;  // row groups per work item of the step kernel
-  int cells_per_thread = 1;  // consumer cells per thread of the step kernel (1 or 2)
-  int item_rows = 1;         // two cells per thread: x-rows per work item
-  int dynamic_items = 1;     // work items from a device counter (1) or dealt round-robin (0)
-  int occupancy = 0;
+  StepLaunch launch;
   int num_sms = 148;
   float *mux = nullptr, *muy = nullptr, *muz = nullptr, *mrho = nullptr;
   NearTable near;                 // near-wall cells and their link tables
-  // The arrays of the grid before the current one, of the same lattice size: the next
-  // voxelization (a body turned or moved in its tunnel) builds into them instead of
-  // allocating (6 bytes a cell against 152 of FP32 populations).  Given back when the
-  // lattice changes, when memory runs out and with the engine.
+  // The arrays of the grid and the table before the current ones, of the same lattice size:
+  // the next voxelization (a body turned or moved in its tunnel) builds into them instead of
+  // allocating (6 bytes a cell against 152 of FP32 populations, 916 a near-wall cell).
   DevGrid spare;
+  NearTable near_spare;
   VoxScratch vox;
   double* abl = nullptr;
   double* sin_tab = nullptr;
@@ -158,22 +161,22 @@ int do_reset(aerosim_engine* h) {
 // The tcgen05 weight image when the closure runs as 128-cell tcgen05 tiles: that path was
 // chosen and the lattice's row pitch is 128 or 256 (every work item then keeps the 8
 // consumer warps busy as two groups of four); otherwise null (warp-level mma.sync).
-const uint4* closure_umma(const aerosim_engine* h) {
-  if (!h->mlp_frag || !h->mlp_umma || !h->have_grid) return nullptr;
-  const bool fits = h->L.pitch == 128 || h->L.pitch == 256;
+const uint4* closure_umma(const aerosim_engine* h, const Layout& L) {
+  if (!h->mlp_frag || !h->mlp_umma) return nullptr;
+  const bool fits = L.pitch == 128 || L.pitch == 256;
   return (h->mlp_path == AEROSIM_SGS_PATH_TCGEN05 && fits) ? h->mlp_umma : nullptr;
 }
 
 // Chooses the persistent step-kernel launch: CTAs of 8 consumer warps + 1 producer
 // warp, as many resident per SM as registers and shared memory allow, and the
-// deepest shared-memory ring (up to 4 slots) that keeps that residency.
-int configure_step(aerosim_engine* h) {
-  const Layout& L = h->L;
+// deepest shared-memory ring (up to 4 slots) that keeps that residency.  For lattice L with
+// the engine's precision and closure; *out changes only when a launch fits.
+int plan_step(aerosim_engine* h, const Layout& L, StepLaunch* out) {
   const size_t eb = precision_bytes(h->cfg.precision);
   StepArgs dummy{};
   dummy.L = L;  // the kernel instance depends on the row pitch and the closure
   dummy.mlp_frag = h->mlp_frag;
-  dummy.mlp_umma = closure_umma(h);
+  dummy.mlp_umma = closure_umma(h, L);
   const int mlp = h->mlp_frag ? (dummy.mlp_umma ? 2 : 1) : 0;
   const bool half = h->cfg.precision == AEROSIM_PREC_F16S || h->cfg.precision == AEROSIM_PREC_BF16S ||
                     h->cfg.precision == AEROSIM_PREC_F16C;
@@ -230,27 +233,31 @@ int configure_step(aerosim_engine* h) {
     }
   }
   if (best_s == 0) return fail(h, AEROSIM_ERR_ARG, "step kernel: no launch configuration fits shared memory");
-  h->block = block;
-  h->stages = best_s;
-  h->smem = smem_for(best_s);
-  h->item_rows = item_rows;
-  h->item_groups = groups;
-  h->cells_per_thread = cpt;
+  StepLaunch p;
+  p.block = block;
+  p.stages = best_s;
+  p.smem = smem_for(best_s);
+  p.item_rows = item_rows;
+  p.item_groups = groups;
+  p.cells_per_thread = cpt;
   // work items from the step's counter (108.8 vs 115.8 us FP32 with one cell per thread):
   // AEROSIM_DYNAMIC_ITEMS (0 or 1) overrides the default deal
-  if (const char* denv = getenv("AEROSIM_DYNAMIC_ITEMS")) h->dynamic_items = atoi(denv) ? 1 : 0;
+  p.dynamic_items = out->dynamic_items;
+  if (const char* denv = getenv("AEROSIM_DYNAMIC_ITEMS")) p.dynamic_items = atoi(denv) ? 1 : 0;
   // the occupancy of the chosen configuration
-  CU(h, launch_step(h->cfg.precision, dummy, block, 0, h->smem, h->stream, &best_occ, nullptr));
-  h->occupancy = best_occ;
+  CU(h, launch_step(h->cfg.precision, dummy, block, 0, p.smem, h->stream, &best_occ, nullptr));
   const long long per_item = cpt == 2 ? item_rows : (long long)rows_per_item(L.nx) * groups;
   const long long items = (all_rows + per_item - 1) / per_item;
   long long grid = (long long)best_occ * h->num_sms;
   const char* genv = getenv("AEROSIM_CTAS_PER_SM");
   if (genv && atoi(genv) > 0 && atoi(genv) <= best_occ) grid = (long long)atoi(genv) * h->num_sms;
   if (grid > items) grid = items;
-  h->grid = (unsigned)(grid < 1 ? 1 : grid);
+  p.grid = (unsigned)(grid < 1 ? 1 : grid);
+  *out = p;
   return AEROSIM_OK;
 }
+
+int configure_step(aerosim_engine* h) { return plan_step(h, h->L, &h->launch); }
 
 cudaError_t alloc_pops(aerosim_engine* h) {
   const size_t N = (size_t)h->g.N, eb = precision_bytes(h->cfg.precision);
@@ -267,7 +274,7 @@ cudaError_t alloc_pops(aerosim_engine* h) {
 int ensure_pops(aerosim_engine* h, bool* reallocated) {
   *reallocated = false;
   const long long N = h->g.N;
-  if (h->f[0] && h->f_prec == h->cfg.precision && h->f_cells == N) return configure_step(h);
+  if (h->f[0] && h->f_prec == h->cfg.precision && h->f_cells == N) return AEROSIM_OK;
   free_pops(h);
   cudaError_t e = alloc_pops(h);
   if (e == cudaErrorMemoryAllocation && (h->spare.cell_mem || h->vox.dev)) {  // once more without what is kept for later
@@ -282,7 +289,7 @@ int ensure_pops(aerosim_engine* h, bool* reallocated) {
   h->f_prec = h->cfg.precision;
   h->f_cells = N;
   *reallocated = true;
-  return configure_step(h);
+  return AEROSIM_OK;
 }
 
 int ensure_staging(aerosim_engine* h, size_t bytes) {
@@ -297,11 +304,7 @@ int ensure_staging(aerosim_engine* h, size_t bytes) {
 
 // Tables of the inlet condition that the reference evaluates with Math.pow and
 // Math.sin (lbmCpuReference.ts:121-125, 334-342), computed once on the host.
-int upload_tables(aerosim_engine* h) {
-  const int ny = h->g.ny;
-  if (h->tab_ny == ny && h->abl) return AEROSIM_OK;
-  cudaFree(h->abl); cudaFree(h->sin_tab);
-  h->abl = nullptr; h->sin_tab = nullptr;
+int make_tables(aerosim_engine* h, int ny, double** abl_out, double** sin_out) {
   std::vector<double> abl(ny), st((size_t)120 * ny);
   for (int iy = 0; iy < ny; ++iy) {
     const double yf = (iy + 0.5) / ny;
@@ -310,56 +313,96 @@ int upload_tables(aerosim_engine* h) {
   for (int s = 0; s < 120; ++s)
     for (int iy = 0; iy < ny; ++iy)
       st[(size_t)s * ny + iy] = std::sin(s * 0.15 + ((double)iy / ny) * M_PI * 2.0);
-  CU(h, cudaMalloc(&h->abl, ny * sizeof(double)));
-  CU(h, cudaMalloc(&h->sin_tab, st.size() * sizeof(double)));
-  CU(h, cudaMemcpyAsync(h->abl, abl.data(), ny * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-  CU(h, cudaMemcpyAsync(h->sin_tab, st.data(), st.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  CU(h, cudaMalloc(abl_out, ny * sizeof(double)));
+  CU(h, cudaMalloc(sin_out, st.size() * sizeof(double)));
+  CU(h, cudaMemcpyAsync(*abl_out, abl.data(), ny * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  CU(h, cudaMemcpyAsync(*sin_out, st.data(), st.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
   CU(h, cudaStreamSynchronize(h->stream));
-  h->tab_ny = ny;
   return AEROSIM_OK;
 }
 
-// Installs a freshly built device grid (voxelizer output or host upload).
-int install_grid(aerosim_engine* h, DevGrid& ng, double dx, const double origin[3], int reset_flow) {
-  // A pending rescale belongs to the old flags: apply it before they change.
-  if (h->have_grid && h->f[0] && !reset_flow) {
-    CU(h, launch_materialize(h->f_prec, h->f[h->cur], h->g.cls, h->st, prev_slot(h), h->L, h->g.N,
-                             h->stream));
-    int rc = reset_state(h);
+// What a new grid brings along: built aside, so that a call that fails half-way leaves the
+// engine with the grid, the near-wall table, the tables and the launch it steps with.
+struct GridParts {
+  Layout L{};
+  StepLaunch launch;
+  NearTable near;
+  double *abl = nullptr, *sin_tab = nullptr;  // when the engine's are for another ny
+  double* force_partials = nullptr;           // when the engine's are too few
+  long long force_blocks = 0;
+};
+
+int build_parts(aerosim_engine* h, const DevGrid& ng, int reset_flow, GridParts* p) {
+  if ((long long)19 * p->L.plane >= (1LL << 32))
+    return fail(h, AEROSIM_ERR_ARG, "lattice too large for 32-bit population offsets");
+  p->launch = h->launch;
+  int rc = plan_step(h, p->L, &p->launch);
+  if (rc) return rc;
+  CU(h, cudaMemsetAsync(ng.cls, CELL_SOLID, (size_t)ng.ny * ng.nz * p->L.pitch, h->stream));
+  CU(h, launch_classify(ng.flags, ng.cls, p->L, h->stream));
+  CU(h, build_near_table(ng, p->L, &h->vox, h->stream, &p->near));
+  if (h->mlp_frag)  // the learned closure reads wall distances from the class bytes
+    CU(h, compute_wall_distance(ng.flags, ng.nx, ng.ny, ng.nz, nullptr, ng.cls, p->L.pitch, h->stream));
+  if (h->tab_ny != ng.ny) {
+    rc = make_tables(h, ng.ny, &p->abl, &p->sin_tab);
     if (rc) return rc;
   }
-  const Layout nl = make_layout(ng.nx, ng.ny, ng.nz);
-  if ((long long)19 * nl.plane >= (1LL << 32))
-    return fail(h, AEROSIM_ERR_ARG, "lattice too large for 32-bit population offsets");
-  CU(h, cudaMemsetAsync(ng.cls, CELL_SOLID, (size_t)ng.ny * ng.nz * nl.pitch, h->stream));
-  CU(h, launch_classify(ng.flags, ng.cls, nl, h->stream));
-  CU(h, build_near_table(ng, nl, &h->vox, h->stream, &h->near));
-  h->wall_ready = false;
-  if (h->mlp_frag) {  // the learned closure reads wall distances from the class bytes
-    CU(h, compute_wall_distance(ng.flags, ng.nx, ng.ny, ng.nz, nullptr, ng.cls, nl.pitch, h->stream));
-    h->wall_ready = true;
+  // force reduction: 8 boundary cells per CTA and round, at most 2 CTAs per SM
+  p->force_blocks = std::max<long long>(1, std::min<long long>((ng.B + 7) / 8, 2LL * h->num_sms));
+  if (p->force_blocks > h->force_blocks_cap) CU(h, cudaMalloc(&p->force_partials, p->force_blocks * 8 * sizeof(double)));
+  // a pending rescale belongs to the old flags: apply it before they change
+  if (h->have_grid && h->f[0] && !reset_flow) {
+    CU(h, launch_materialize(h->f_prec, h->f[h->cur], h->g.cls, h->st, prev_slot(h), h->L, h->g.N, h->stream));
+    rc = reset_state(h);
   }
-  const bool same = h->have_grid && nl.nx == h->L.nx && nl.ny == h->L.ny && nl.nz == h->L.nz;
-  if (h->f[0] && (nl.pitch != h->L.pitch || nl.plane != h->L.plane)) free_pops(h);
-  if (same) give_spare(h, h->g);
-  else grid_free(&h->g);
+  return rc;
+}
+
+// Installs a freshly built device grid (voxelizer output or host upload): all of it or, where
+// a call fails, nothing.  What can still fail afterwards is the allocation of the populations
+// of another lattice size, whose old ones are given back first: the engine then has the grid
+// and no flow, and the calls that need one refuse.
+int install_grid(aerosim_engine* h, DevGrid& ng, double dx, const double origin[3], int reset_flow) {
+  GridParts p;
+  p.L = make_layout(ng.nx, ng.ny, ng.nz);
+  std::swap(p.near, h->near_spare);
+  int rc = build_parts(h, ng, reset_flow, &p);
+  if (rc) {
+    cudaStreamSynchronize(h->stream);  // nothing reads the parts, or the caller's arrays, any more
+    near_free(&p.near);
+    cudaFree(p.abl); cudaFree(p.sin_tab); cudaFree(p.force_partials);
+    return rc;
+  }
+  const bool same = h->have_grid && ng.nx == h->L.nx && ng.ny == h->L.ny && ng.nz == h->L.nz;
+  if (h->f[0] && (p.L.pitch != h->L.pitch || p.L.plane != h->L.plane)) free_pops(h);
+  if (same) {
+    give_spare(h, h->g);
+  } else {
+    grid_free(&h->g);
+    near_free(&h->near);
+  }
+  std::swap(h->near, p.near);
+  h->near_spare = p.near;  // the old table's memory, none after another lattice
   h->g = ng;
-  h->L = nl;
   ng = DevGrid();
+  h->L = p.L;
+  h->launch = p.launch;
+  h->wall_ready = h->mlp_frag != nullptr;
   h->have_grid = true;
   h->dx = dx;
   h->origin[0] = origin[0]; h->origin[1] = origin[1]; h->origin[2] = origin[2];
   h->fluid_count = h->g.N - h->g.solid;
-  // force reduction: 8 boundary cells per CTA and round, at most 2 CTAs per SM
-  const long long blocks = std::max<long long>(1, std::min<long long>((h->g.B + 7) / 8, 2LL * h->num_sms));
-  if (blocks > h->force_blocks_cap) {
-    cudaFree(h->force_partials);
-    h->force_partials = nullptr;
-    CU(h, cudaMalloc(&h->force_partials, blocks * 8 * sizeof(double)));
-    h->force_blocks_cap = blocks;
+  if (p.abl) {
+    cudaFree(h->abl); cudaFree(h->sin_tab);
+    h->abl = p.abl;
+    h->sin_tab = p.sin_tab;
+    h->tab_ny = h->g.ny;
   }
-  int rc = upload_tables(h);
-  if (rc) return rc;
+  if (p.force_partials) {
+    cudaFree(h->force_partials);
+    h->force_partials = p.force_partials;
+    h->force_blocks_cap = p.force_blocks;
+  }
   bool realloc = false;
   rc = ensure_pops(h, &realloc);
   if (rc) return rc;
@@ -454,6 +497,7 @@ int aerosim_destroy(aerosim_engine* h) {
   h->vox.release();
   if (h->vox.host) cudaFreeHost(h->vox.host);
   near_free(&h->near);
+  near_free(&h->near_spare);
   free_pops(h);
   cudaFree(h->abl); cudaFree(h->sin_tab); cudaFree(h->st);
   cudaFree(h->force_partials); cudaFree(h->force_ticket); cudaFree(h->force_out);
@@ -605,6 +649,7 @@ int aerosim_set_config(aerosim_engine* h, const aerosim_config* cfg) {
   if (h->have_grid && cfg->precision != old_prec) {
     bool realloc = false;
     int rc = ensure_pops(h, &realloc);
+    if (!rc) rc = configure_step(h);
     if (rc) return rc;
     return do_reset(h);
   }
@@ -644,7 +689,7 @@ int enqueue_steps(aerosim_engine* h, int32_t n) {
   a.near_cells = h->near.cells; a.n_near = h->near.n;
   a.links = h->near.links;
   a.links_f = h->near.links_f;
-  a.stages = h->stages;
+  a.stages = h->launch.stages;
   a.ground_no_slip = h->cfg.ground_no_slip;
   a.u_inlet = h->cfg.u_inlet_lattice;
   a.tau0 = 3.0 * h->cfg.nu_lattice + 0.5;
@@ -652,12 +697,12 @@ int enqueue_steps(aerosim_engine* h, int32_t n) {
   a.k_smag = 18.0 * M_SQRT2 * cs2;
   a.mlp_frag = h->mlp_frag;
   a.mlp_bias = h->mlp_bias;
-  a.mlp_umma = closure_umma(h);
+  a.mlp_umma = closure_umma(h, h->L);
   a.mlp_nu0 = (float)((std::max(a.tau0, 0.5015) - 0.5) / 3.0);
-  a.item_groups = h->item_groups;
-  a.cells_per_thread = h->cells_per_thread;
-  a.dynamic_items = h->dynamic_items;
-  a.item_rows = h->item_rows;
+  a.item_groups = h->launch.item_groups;
+  a.cells_per_thread = h->launch.cells_per_thread;
+  a.dynamic_items = h->launch.dynamic_items;
+  a.item_rows = h->launch.item_rows;
   a.pair_magic = pair_magic(std::max(1, h->L.nx / 2));
   a.wait_limit = h->wait_limit;
   long long launches = 0;
@@ -668,7 +713,7 @@ int enqueue_steps(aerosim_engine* h, int32_t n) {
     a.step_index = (int)h->step_index;
     a.write_macro = (s == n - 1) ? 1 : 0;
     int nl = 0;
-    CU(h, launch_step(h->cfg.precision, a, h->block, h->grid, h->smem, h->stream, nullptr, &nl));
+    CU(h, launch_step(h->cfg.precision, a, h->launch.block, h->launch.grid, h->launch.smem, h->stream, nullptr, &nl));
     launches += nl;
     h->cur ^= 1;
     h->step_index += 1;
@@ -1143,7 +1188,7 @@ int aerosim_set_sgs_mlp_path(aerosim_engine* h, int32_t path, int32_t* in_use) {
   }
   if (in_use)
     *in_use = !h->mlp_frag ? AEROSIM_SGS_PATH_DEFAULT
-                           : (closure_umma(h) ? AEROSIM_SGS_PATH_TCGEN05 : AEROSIM_SGS_PATH_WARP);
+                           : (closure_umma(h, h->L) ? AEROSIM_SGS_PATH_TCGEN05 : AEROSIM_SGS_PATH_WARP);
   return AEROSIM_OK;
 }
 
