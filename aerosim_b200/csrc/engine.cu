@@ -649,7 +649,7 @@ int aerosim_set_config(aerosim_engine* h, const aerosim_config* cfg) {
   if (h->have_grid && cfg->precision != old_prec) {
     bool realloc = false;
     int rc = ensure_pops(h, &realloc);
-    if (!rc) rc = configure_step(h);
+    if (!rc && (rc = configure_step(h))) free_pops(h);  // the launch in force is the other precision's
     if (rc) return rc;
     return do_reset(h);
   }

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from aerosim_b200 import AerosimError, meshes, sgs
+from aerosim_b200 import _native as N
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +66,28 @@ def test_refused_grid_leaves_the_engine_as_it_was(gpu_engine_cls, precision, clo
     _same(e, fresh)
     for x in (e, untouched, fresh):
         x.close()
+
+
+@pytest.mark.parametrize("then", ["back", "other lattice"])
+def test_precision_that_does_not_fit_leaves_no_flow(gpu_engine_cls, then):
+    """Rows of 2000 cells fit the ring in 16 bits, not in 32: the engine must not step 32-bit
+    populations with the launch of the 16-bit ones."""
+    e, fresh = gpu_engine_cls(0), gpu_engine_cls(0)
+    _voxelize(e, (2000, 6, 6), "f16s")
+    e.step(2)
+    with pytest.raises(AerosimError) as err:
+        e.update_config({"precision": "f32"})
+    assert err.value.code == N.ERR_ARG
+    for call in (lambda: e.step(1), e.reset_flow, e.read_populations):
+        with pytest.raises(AerosimError) as err:
+            call()
+        assert err.value.code == N.ERR_STATE
+    if then == "back":
+        e.update_config({"precision": "f16s"})
+        _voxelize(fresh, (2000, 6, 6), "f16s")
+    else:
+        for x in (e, fresh):
+            _voxelize(x, SMALL, "f32")
+    e.step(4), fresh.step(4)
+    _same(e, fresh)
+    e.close(), fresh.close()
