@@ -1134,6 +1134,13 @@ int ensure_wall_distance(aerosim_engine* h) {
   return AEROSIM_OK;
 }
 
+void free_closure(aerosim_engine* h) {
+  cudaFree(h->mlp_frag); cudaFree(h->mlp_bias); cudaFree(h->mlp_umma);
+  h->mlp_frag = nullptr;
+  h->mlp_bias = nullptr;
+  h->mlp_umma = nullptr;
+}
+
 double effective_nu0(const aerosim_engine* h) {
   return (std::max(3.0 * h->cfg.nu_lattice + 0.5, 0.5015) - 0.5) / 3.0;
 }
@@ -1146,10 +1153,7 @@ int aerosim_set_sgs_mlp(aerosim_engine* h, const float* params) {
   if (!h) return AEROSIM_ERR_ARG;
   CU(h, cudaSetDevice(h->device));
   if (!params) {
-    cudaFree(h->mlp_frag); cudaFree(h->mlp_bias); cudaFree(h->mlp_umma);
-    h->mlp_frag = nullptr;
-    h->mlp_bias = nullptr;
-    h->mlp_umma = nullptr;
+    free_closure(h);
   } else {
     for (int i = 0; i < kMlpParams; ++i)
       if (!std::isfinite(params[i])) return fail(h, AEROSIM_ERR_ARG, "set_sgs_mlp: non-finite parameter");
@@ -1158,19 +1162,27 @@ int aerosim_set_sgs_mlp(aerosim_engine* h, const float* params) {
     mlp_pack_fragments(params, frag.data(), bias.data());
     std::vector<uint16_t> img(kUmmaBBytes / 2);
     mlp_pack_umma(params, img.data());
-    if (!h->mlp_frag) {
-      CU(h, cudaMalloc(&h->mlp_frag, frag.size() * sizeof(uint32_t)));
-      CU(h, cudaMalloc(&h->mlp_bias, bias.size() * sizeof(float)));
-      CU(h, cudaMalloc(&h->mlp_umma, kUmmaBBytes));
+    if (h->have_grid) {
+      int rc = ensure_wall_distance(h);
+      if (rc) return rc;
+    }
+    const bool added = !h->mlp_frag;
+    if (added) {
+      cudaError_t e = cudaMalloc(&h->mlp_frag, frag.size() * sizeof(uint32_t));
+      if (e == cudaSuccess) e = cudaMalloc(&h->mlp_bias, bias.size() * sizeof(float));
+      if (e == cudaSuccess) e = cudaMalloc(&h->mlp_umma, kUmmaBBytes);
+      if (e != cudaSuccess) {
+        free_closure(h);
+        CU(h, e);
+      }
     }
     CU(h, cudaMemcpyAsync(h->mlp_frag, frag.data(), frag.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream));
     CU(h, cudaMemcpyAsync(h->mlp_bias, bias.data(), bias.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream));
     CU(h, cudaMemcpyAsync(h->mlp_umma, img.data(), kUmmaBBytes, cudaMemcpyHostToDevice, h->stream));
     CU(h, cudaStreamSynchronize(h->stream));
-    if (h->have_grid) {
-      int rc = ensure_wall_distance(h);
-      if (rc) return rc;
-    }
+    const int rc = h->have_grid && h->f[0] ? configure_step(h) : AEROSIM_OK;
+    if (rc && added) free_closure(h);  // the launch in force has no room for it
+    return rc;
   }
   if (h->have_grid && h->f[0]) return configure_step(h);
   return AEROSIM_OK;
@@ -1181,10 +1193,14 @@ int aerosim_set_sgs_mlp_path(aerosim_engine* h, int32_t path, int32_t* in_use) {
   if (path != AEROSIM_SGS_PATH_DEFAULT && path != AEROSIM_SGS_PATH_WARP && path != AEROSIM_SGS_PATH_TCGEN05)
     return fail(h, AEROSIM_ERR_ARG, "set_sgs_mlp_path: unknown path");
   CU(h, cudaSetDevice(h->device));
+  const int old = h->mlp_path;
   h->mlp_path = path;
   if (h->have_grid && h->f[0]) {
     const int rc = configure_step(h);
-    if (rc) return rc;
+    if (rc) {
+      h->mlp_path = old;
+      return rc;
+    }
   }
   if (in_use)
     *in_use = !h->mlp_frag ? AEROSIM_SGS_PATH_DEFAULT

@@ -91,3 +91,24 @@ def test_precision_that_does_not_fit_leaves_no_flow(gpu_engine_cls, then):
     e.step(4), fresh.step(4)
     _same(e, fresh)
     e.close(), fresh.close()
+
+
+@pytest.mark.parametrize("dims", [(1040, 8, 8), (40, 6, 1030)], ids=str)
+def test_refused_closure_leaves_the_engine_as_it_was(gpu_engine_cls, dims):
+    """Wall distances are refused above 1024 cells a side: no closure then, and the launch
+    without one goes on."""
+    e, untouched = gpu_engine_cls(0), gpu_engine_cls(0)
+    for x in (e, untouched):
+        _voxelize(x, dims, "f32")
+        x.step(3)
+    for _ in range(2):
+        with pytest.raises(AerosimError):
+            e.set_sgs_mlp(sgs.init_params(3))
+        e.step(3), untouched.step(3)
+        _same(e, untouched)
+    # a lattice that allows one: none is set
+    for x in (e, untouched):
+        _voxelize(x, SMALL, "f32")
+        x.step(3)
+    _same(e, untouched)
+    e.close(), untouched.close()
