@@ -51,9 +51,11 @@ struct aerosim_engine {
   int num_sms = 148;
   float *mux = nullptr, *muy = nullptr, *muz = nullptr, *mrho = nullptr;
   NearTable near;                 // near-wall cells and their link tables
-  // The arrays of the grid and the table before the current ones, of the same lattice size:
-  // the next voxelization (a body turned or moved in its tunnel) builds into them instead of
-  // allocating (6 bytes a cell against 152 of FP32 populations, 916 a near-wall cell).
+  // The arrays of the grid and the table before the current ones, when those were of the same
+  // lattice size: the next voxelization (a body turned or moved in its tunnel) builds into them
+  // instead of allocating (6 bytes a cell against 152 of FP32 populations, 916 a near-wall
+  // cell).  Arrays more than kKeepSlack too large for the grid they would hold are not taken
+  // up, and what is kept here goes back wherever an allocation fails (with_room).
   DevGrid spare;
   NearTable near_spare;
   VoxScratch vox;
@@ -124,6 +126,18 @@ void give_spare(aerosim_engine* h, DevGrid& g) {
   h->spare.list_mem = g.list_mem;
   h->spare.list_cap = g.list_cap;
   g = DevGrid();
+}
+
+// An allocating call; when memory runs out, once more without what is kept for later.
+template <class F>
+cudaError_t with_room(aerosim_engine* h, F call) {
+  const cudaError_t e = call();
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  grid_free(&h->spare);
+  near_free(&h->near_spare);
+  h->vox.release();
+  return call();
 }
 
 void free_pops(aerosim_engine* h) {
@@ -275,15 +289,10 @@ int ensure_pops(aerosim_engine* h, bool* reallocated) {
   *reallocated = false;
   const long long N = h->g.N;
   if (h->f[0] && h->f_prec == h->cfg.precision && h->f_cells == N) return AEROSIM_OK;
-  free_pops(h);
-  cudaError_t e = alloc_pops(h);
-  if (e == cudaErrorMemoryAllocation && (h->spare.cell_mem || h->vox.dev)) {  // once more without what is kept for later
-    cudaGetLastError();
+  const cudaError_t e = with_room(h, [&] {
     free_pops(h);
-    grid_free(&h->spare);
-    h->vox.release();
-    e = alloc_pops(h);
-  }
+    return alloc_pops(h);
+  });
   if (e != cudaSuccess) free_pops(h);  // never some of the buffers
   CU(h, e);
   h->f_prec = h->cfg.precision;
@@ -297,7 +306,7 @@ int ensure_staging(aerosim_engine* h, size_t bytes) {
   cudaFree(h->staging);
   h->staging = nullptr;
   h->staging_bytes = 0;
-  CU(h, cudaMalloc(&h->staging, bytes));
+  CU(h, with_room(h, [&] { return cudaMalloc(&h->staging, bytes); }));
   h->staging_bytes = bytes;
   return AEROSIM_OK;
 }
@@ -340,9 +349,11 @@ int build_parts(aerosim_engine* h, const DevGrid& ng, int reset_flow, GridParts*
   if (rc) return rc;
   CU(h, cudaMemsetAsync(ng.cls, CELL_SOLID, (size_t)ng.ny * ng.nz * p->L.pitch, h->stream));
   CU(h, launch_classify(ng.flags, ng.cls, p->L, h->stream));
-  CU(h, build_near_table(ng, p->L, &h->vox, h->stream, &p->near));
+  CU(h, with_room(h, [&] { return build_near_table(ng, p->L, &h->vox, h->stream, &p->near); }));
   if (h->mlp_frag)  // the learned closure reads wall distances from the class bytes
-    CU(h, compute_wall_distance(ng.flags, ng.nx, ng.ny, ng.nz, nullptr, ng.cls, p->L.pitch, h->stream));
+    CU(h, with_room(h, [&] {
+         return compute_wall_distance(ng.flags, ng.nx, ng.ny, ng.nz, nullptr, ng.cls, p->L.pitch, h->stream);
+       }));
   if (h->tab_ny != ng.ny) {
     rc = make_tables(h, ng.ny, &p->abl, &p->sin_tab);
     if (rc) return rc;
@@ -530,9 +541,15 @@ int aerosim_voxelize(aerosim_engine* h, const float* positions, int64_t vertex_c
   CU(h, cudaSetDevice(h->device));
   DevGrid ng = take_spare(h);
   std::string e;
-  const int rc = run_voxelizer(positions, vertex_count, indices, index_count, world16, tunnel.height, nx, ny,
-                               nz, h->stream, &h->vox, &ng, &e);
+  int rc = 0;
+  with_room(h, [&] {
+    if (rc) grid_free(&ng);
+    rc = run_voxelizer(positions, vertex_count, indices, index_count, world16, tunnel.height, nx, ny, nz, h->stream, &h->vox,
+                       &ng, &e);
+    return rc == -5 ? cudaErrorMemoryAllocation : cudaSuccess;
+  });
   if (rc) {
+    cudaGetLastError();
     grid_free(&ng);
     return fail(h, rc == -4 ? AEROSIM_ERR_DEVICE : AEROSIM_ERR_CUDA, e);
   }
@@ -613,12 +630,14 @@ int aerosim_set_voxel_grid(aerosim_engine* h, int32_t nx, int32_t ny, int32_t nz
   ng.oz = origin ? origin[2] : -nz * dx * 0.5;
   ng.B = B; ng.solid = solid;
   auto bad = [&](cudaError_t e) {
+    cudaGetLastError();
     grid_free(&ng);
     return fail(h, AEROSIM_ERR_CUDA, std::string("set_voxel_grid: ") + cudaGetErrorString(e));
   };
   cudaError_t e;
-  if ((e = grid_cells(&ng, N, (size_t)make_layout(nx, ny, nz).plane)) != cudaSuccess) return bad(e);
-  if ((e = grid_lists(&ng, B)) != cudaSuccess) return bad(e);
+  e = with_room(h, [&] { return grid_cells(&ng, N, (size_t)make_layout(nx, ny, nz).plane); });
+  if (e == cudaSuccess) e = with_room(h, [&] { return grid_lists(&ng, B); });
+  if (e != cudaSuccess) return bad(e);
   std::vector<float> mq(std::max<int64_t>(B, 1), 1.0f);
   for (int64_t b = 0; b < B; ++b)
     for (int k = 0; k < 18; ++k) {
@@ -1106,7 +1125,7 @@ extern "C" int aerosim_q_criterion_fields(aerosim_engine* h, int32_t nx, int32_t
   CU(h, cudaSetDevice(h->device));
   const long long N = (long long)nx * ny * nz;
   void* buf = nullptr;
-  CU(h, cudaMalloc(&buf, N * (3 * sizeof(float) + 1)));
+  CU(h, with_room(h, [&] { return cudaMalloc(&buf, N * (3 * sizeof(float) + 1)); }));
   float* d = static_cast<float*>(buf);
   uint8_t* df = reinterpret_cast<uint8_t*>(d + 3 * N);
   cudaError_t e = cudaMemcpyAsync(d, ux, N * 4, cudaMemcpyHostToDevice, h->stream);
@@ -1128,7 +1147,9 @@ namespace {
 
 int ensure_wall_distance(aerosim_engine* h) {
   if (h->wall_ready) return AEROSIM_OK;
-  CU(h, compute_wall_distance(h->g.flags, h->g.nx, h->g.ny, h->g.nz, nullptr, h->g.cls, h->L.pitch, h->stream));
+  CU(h, with_room(h, [&] {
+       return compute_wall_distance(h->g.flags, h->g.nx, h->g.ny, h->g.nz, nullptr, h->g.cls, h->L.pitch, h->stream);
+     }));
   CU(h, cudaStreamSynchronize(h->stream));
   h->wall_ready = true;
   return AEROSIM_OK;
@@ -1215,8 +1236,10 @@ int aerosim_read_wall_distance(aerosim_engine* h, float* out) {
   const long long N = h->g.N;
   int rc = ensure_staging(h, N * sizeof(float));
   if (rc) return rc;
-  CU(h, compute_wall_distance(h->g.flags, h->g.nx, h->g.ny, h->g.nz, static_cast<float*>(h->staging), h->g.cls,
-                              h->L.pitch, h->stream));
+  CU(h, with_room(h, [&] {
+       return compute_wall_distance(h->g.flags, h->g.nx, h->g.ny, h->g.nz, static_cast<float*>(h->staging), h->g.cls,
+                                    h->L.pitch, h->stream);
+     }));
   h->wall_ready = true;
   CU(h, cudaMemcpyAsync(out, h->staging, N * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
   CU(h, cudaStreamSynchronize(h->stream));
@@ -1241,15 +1264,15 @@ int aerosim_sgs_samples(aerosim_engine* fine, aerosim_engine* coarse, float min_
   const long long Nc = c.N;
   float *dx = nullptr, *dy = nullptr;
   uint8_t* dv = nullptr;
-  cudaError_t e = cudaMalloc(&dx, Nc * kMlpIn * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&dy, Nc * sizeof(float));
-  if (e == cudaSuccess) e = cudaMalloc(&dv, Nc);
+  cudaError_t e = with_room(coarse, [&] { return cudaMalloc(&dx, Nc * kMlpIn * sizeof(float)); });
+  if (e == cudaSuccess) e = with_room(coarse, [&] { return cudaMalloc(&dy, Nc * sizeof(float)); });
+  if (e == cudaSuccess) e = with_room(coarse, [&] { return cudaMalloc(&dv, Nc); });
   if (e == cudaSuccess)
-    e = launch_sgs_samples(fine->mux, fine->muy, fine->muz, fine->mrho, f.flags, f.nx, f.ny, f.nz, c.cls,
-                           coarse->L.pitch, c.nx, c.ny, c.nz, (float)effective_nu0(coarse), min_ratio, max_ratio,
-                           average_radius,
-                           dx, dy, dv,
-                           coarse->stream);
+    e = with_room(coarse, [&] {
+      return launch_sgs_samples(fine->mux, fine->muy, fine->muz, fine->mrho, f.flags, f.nx, f.ny, f.nz, c.cls,
+                                coarse->L.pitch, c.nx, c.ny, c.nz, (float)effective_nu0(coarse), min_ratio, max_ratio,
+                                average_radius, dx, dy, dv, coarse->stream);
+    });
   if (e == cudaSuccess) e = cudaMemcpyAsync(X, dx, Nc * kMlpIn * sizeof(float), cudaMemcpyDeviceToHost, coarse->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(Y, dy, Nc * sizeof(float), cudaMemcpyDeviceToHost, coarse->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(valid, dv, Nc, cudaMemcpyDeviceToHost, coarse->stream);

@@ -30,6 +30,8 @@ struct DevGrid {
   void *cell_mem = nullptr, *list_mem = nullptr;
   size_t cell_cap = 0, list_cap = 0;
 };
+// Memory kept for the next grid may exceed what that grid needs by this much (bytes).
+constexpr size_t kKeepSlack = (size_t)64 << 20;
 // Arrays for N cells (cls_bytes of classes), and lists for B boundary cells.
 cudaError_t grid_cells(DevGrid* g, long long N, size_t cls_bytes);
 cudaError_t grid_lists(DevGrid* g, long long B);
@@ -43,7 +45,7 @@ struct VoxScratch {
   unsigned long long* host = nullptr;  // pinned [32]
   cudaError_t device(size_t n);        // at least n bytes
   cudaError_t pinned();
-  void trim();     // gives back device memory above 64 MB
+  void trim();     // gives back device memory above kKeepSlack
   void release();
 };
 

@@ -19,6 +19,9 @@ namespace {
 
 size_t up256(size_t b) { return (b + 255) / 256 * 256; }
 
+// Whether kept memory serves a need: large enough, and not much larger.
+bool fits(size_t cap, size_t need) { return cap >= need && cap - need <= kKeepSlack + need / 8; }
+
 // Near-wall cells per x-row, one warp per row.
 __global__ void near_count_kernel(const uint8_t* __restrict__ cls, const Layout L, long long rows, uint32_t* __restrict__ counts) {
   const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -176,7 +179,7 @@ cudaError_t build_near_table(const DevGrid& g, const Layout& L, VoxScratch* w, c
                links = up256((size_t)std::max<long long>(n, 1) * 19 * sizeof(NearLink)),
                links_f = up256((size_t)std::max<long long>(n, 1) * 19 * sizeof(NearLinkF));
   const size_t need = cells + links + links_f;
-  if (t->cap < need) {
+  if (!fits(t->cap, need)) {
     near_free(t);
     const size_t room = need + need / 8;  // a turned body has a few more cells
     e = cudaMalloc(&t->mem, room);
@@ -206,7 +209,7 @@ void near_free(NearTable* t) {
 
 cudaError_t grid_cells(DevGrid* g, long long N, size_t cls_bytes) {
   const size_t bf = up256((size_t)N), bc = up256(std::max<size_t>(cls_bytes, 1)), bm = up256((size_t)N * 4);
-  if (g->cell_cap < bf + bc + bm) {
+  if (!fits(g->cell_cap, bf + bc + bm)) {
     cudaFree(g->cell_mem);
     g->cell_mem = nullptr;
     g->cell_cap = 0;
@@ -227,7 +230,7 @@ cudaError_t grid_cells(DevGrid* g, long long N, size_t cls_bytes) {
 cudaError_t grid_lists(DevGrid* g, long long B) {
   const size_t n = (size_t)std::max<long long>(B, 1);
   const size_t bc = up256(n * 4), bq = up256(n * 18 * 4), bm = up256(n * 4);
-  if (g->list_cap < bc + bq + bm) {
+  if (!fits(g->list_cap, bc + bq + bm)) {
     cudaFree(g->list_mem);
     g->list_mem = nullptr;
     g->list_cap = 0;
@@ -275,7 +278,7 @@ void VoxScratch::release() {
   bytes = 0;
 }
 void VoxScratch::trim() {
-  if (bytes > ((size_t)64 << 20)) release();
+  if (bytes > kKeepSlack) release();
 }
 
 }  // namespace aerosim

@@ -963,7 +963,7 @@ void host_nodes(const HostBvh& hb, std::vector<BvhNode>* out) {
     cudaError_t e_ = (x);                                                      \
     if (e_ != cudaSuccess) {                                                   \
       *err = std::string("voxelizer: ") + #x + ": " + cudaGetErrorString(e_);  \
-      return -3;                                                               \
+      return e_ == cudaErrorMemoryAllocation ? -5 : -3;                        \
     }                                                                          \
   } while (0)
 

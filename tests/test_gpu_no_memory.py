@@ -40,3 +40,33 @@ def test_no_memory_for_the_populations(gpu_engine_cls):
     assert np.array_equal(e.read_populations().view(np.uint32), fresh.read_populations().view(np.uint32))
     assert e.read_forces().fx == fresh.read_forces().fx and e.mass_stats() == fresh.mass_stats()
     e.close(), fresh.close()
+
+
+def test_what_is_kept_for_the_next_grid_goes_back(gpu_engine_cls):
+    """After two voxelizations of 33.5 M cells an engine holds the first one's arrays (201 MB)
+    for a third.  An allocation that fails gets them, and a small lattice keeps none of them."""
+    import torch
+    e = gpu_engine_cls(0)
+    for _ in range(2):
+        _voxelize(e, (512, 256, 256), "f16s")
+    free, _ = torch.cuda.mem_get_info()
+    hog = torch.empty(free - (100 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        assert e.read_macro()["rho"].min() > 0.9  # through 134 MB of staging
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    e.close()
+
+    def used_after(grids):
+        e = gpu_engine_cls(0)
+        before, _ = torch.cuda.mem_get_info()
+        for dims in grids:
+            _voxelize(e, dims, "f16s")
+        after, _ = torch.cuda.mem_get_info()
+        e.close()
+        return before - after
+
+    used_after([(64, 24, 26)])
+    # both keep at most 64 MB of scratch, and the arrays of two grids of 40 000 cells
+    assert abs(used_after([(512, 256, 256)] * 3 + [(64, 24, 26)] * 2) - used_after([(64, 24, 26)] * 2)) <= 70 << 20
