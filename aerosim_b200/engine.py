@@ -21,6 +21,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import threading
 from dataclasses import dataclass
 
 import numpy as np
@@ -128,15 +129,17 @@ def read_voxel_grid(handle: _Handle) -> VoxelGridResult:
 
 
 _shared_voxelizer: _Handle | None = None
+_shared_voxelizer_lock = threading.Lock()
 
 
 def voxelize_mesh_to_lattice(geometry, world_matrix, tunnel, grid, device: int = 0) -> VoxelGridResult:
     """voxelizeMeshToLattice (voxelizer.ts:86-281) on the GPU; returns host arrays."""
     global _shared_voxelizer
-    if _shared_voxelizer is None:
-        _shared_voxelizer = _Handle(device)
-    voxelize_into(_shared_voxelizer, geometry, world_matrix, tunnel, grid)
-    return read_voxel_grid(_shared_voxelizer)
+    with _shared_voxelizer_lock:  # one engine, its grid and its scratch: a call at a time
+        if _shared_voxelizer is None:
+            _shared_voxelizer = _Handle(device)
+        voxelize_into(_shared_voxelizer, geometry, world_matrix, tunnel, grid)
+        return read_voxel_grid(_shared_voxelizer)
 
 
 voxelizeMeshToLattice = voxelize_mesh_to_lattice
