@@ -51,11 +51,12 @@ struct aerosim_engine {
   int num_sms = 148;
   float *mux = nullptr, *muy = nullptr, *muz = nullptr, *mrho = nullptr;
   NearTable near;                 // near-wall cells and their link tables
-  // The arrays of the grid and the table before the current ones, when those were of the same
-  // lattice size: the next voxelization (a body turned or moved in its tunnel) builds into them
-  // instead of allocating (6 bytes a cell against 152 of FP32 populations, 916 a near-wall
-  // cell).  Arrays more than kKeepSlack too large for the grid they would hold are not taken
-  // up, and what is kept here goes back wherever an allocation fails (with_room).
+  // The arrays of the grid before the current one, when that was of the same lattice size, and
+  // of the near-wall table before the current one: the next voxelization (a body turned or
+  // moved in its tunnel) builds into them instead of allocating (6 bytes a cell against 152 of
+  // FP32 populations, 916 a near-wall cell).  Memory more than kKeepSlack too large for what it
+  // would hold is not taken up, a table's of another lattice not kept above it, and what is
+  // kept goes back wherever an allocation fails (with_room).
   DevGrid spare;
   NearTable near_spare;
   VoxScratch vox;
@@ -386,14 +387,11 @@ int install_grid(aerosim_engine* h, DevGrid& ng, double dx, const double origin[
   }
   const bool same = h->have_grid && ng.nx == h->L.nx && ng.ny == h->L.ny && ng.nz == h->L.nz;
   if (h->f[0] && (p.L.pitch != h->L.pitch || p.L.plane != h->L.plane)) free_pops(h);
-  if (same) {
-    give_spare(h, h->g);
-  } else {
-    grid_free(&h->g);
-    near_free(&h->near);
-  }
+  if (same) give_spare(h, h->g);
+  else grid_free(&h->g);
   std::swap(h->near, p.near);
-  h->near_spare = p.near;  // the old table's memory, none after another lattice
+  if (!same && p.near.cap > kKeepSlack) near_free(&p.near);
+  h->near_spare = p.near;  // the old table's memory
   h->g = ng;
   ng = DevGrid();
   h->L = p.L;

@@ -1114,8 +1114,8 @@ int run_voxelizer(const float* pos, int64_t nverts, const int32_t* idx, int64_t 
         VCHECK(launch_scan_rows(d_rows, brows, w->host, s));
       }
     }
-    VCHECK(cudaMemcpyAsync(h_solid, d_solid, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    VCHECK(cudaMemcpyAsync(h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    // (the error word follows the count on both sides)
+    VCHECK(cudaMemcpyAsync(h_solid, d_solid, sizeof(unsigned long long) + sizeof(int), cudaMemcpyDeviceToHost, s));
     VCHECK(cudaStreamSynchronize(s));
     if (!(*h_err & VOX_NAN_HITS)) break;  // the kernel does not set it in a tree of the host
     VCHECK(host_tree());
