@@ -302,7 +302,7 @@ __device__ __forceinline__ void collide_f32(float (&h)[19], float& r, float& ux,
   const float pxy = fmaf(-rux, uy, sxy);
   const float pxz = fmaf(-rux, uz, sxz);
   const float pyz = fmaf(-ruy, uz, syz);
-const float off = YY ? fmaf(pyz, pyz, fmaf(pxy, pxy, __fmul_rn(pxz, pxz))) : pxy * pxy + pxz * pxz + pyz * pyz;
+  const float off = YY ? fmaf(pyz, pyz, fmaf(pxy, pxy, __fmul_rn(pxz, pxz))) : pxy * pxy + pxz * pxz + pyz * pyz;
   const float sq = YY ? fmaf(2.0f, off, fmaf(pzz, pzz, fmaf(pyy, pyy, __fmul_rn(pxx, pxx))))
                       : pxx * pxx + pyy * pyy + pzz * pzz + 2.0f * off;
   const float pn = sqrtf(sq);
@@ -1165,7 +1165,7 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<S, MODE, MLP>())
   // learned closure: weight fragments, biases, one staging block per consumer warp
   uint32_t* s_mfrag =
       reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(s_dslot + 19) + 15) & ~uintptr_t(15));  // [24 * 32]
-  float* s_mbias = reinterpret_cast<float*>(s_mfrag + kMlpFragWords * 32);               // [65]
+  float* s_mbias = reinterpret_cast<float*>(s_mfrag + kMlpFragWords * 32);               // [kMlpBias]
   uint32_t* s_mstage = reinterpret_cast<uint32_t*>(s_mbias + kMlpBias);                  // [8][128]
   if constexpr (MLP != MLP_NONE) {
     for (int i = threadIdx.x; i < kMlpFragWords * 32; i += blockDim.x) s_mfrag[i] = a.mlp_frag[i];

@@ -1,7 +1,7 @@
 // The two-cells-per-thread step of a single lattice (pair_kernel) and the item loop it
 // shares with the batched step: FP32 arithmetic, with MLP the learned closure as warp tiles,
-// rows of 4 and more cells (a batch: of an even count).  With ODD the pairs cover cells 0 .. nx-2 and the outlet cell nx-1 follows
-// the last of them.
+// rows of 4 and more cells (a batch: of an even count).  With ODD the pairs cover cells
+// 0 .. nx-2 and the outlet cell nx-1 follows the last of them.
 //
 // A work item is R consecutive x-rows; its pairs of cells form one list, and each consumer
 // warp takes chunks of 32 consecutive pairs of it, across row ends, dealt cyclically (the
@@ -13,15 +13,15 @@
 // producer leaves beside it.  A chunk of plain fluid (one vote) has no per-cell tests.
 //
 // What bounds it (ncu, 256x128x128): with 16-bit storage issue and fixed latencies at 20 warps
-// per SM (39.2 M warp instructions, 2.3 of 4 per cycle, DRAM 52 %), with FP32 DRAM (70 % cold,
-// 0.95 of the copy peak in a run of steps).  Microseconds per step, before -> with this kernel:
+// per SM (36.7 M warp instructions, 2.35 of 4 per cycle, DRAM 53 %), with FP32 DRAM (72 % cold,
+// 0.97 of the copy peak in a run of steps).  Microseconds per step, before -> with this kernel:
 // 256x128x128 F16S 68.5 -> 58.2, BF16S 69.5 -> 58.5, F16C 73.1 -> 63.6, FP32 101.6 -> 101.0;
 // 160x80x80 F16S 28.2 -> 21.3; 200x100x96 F16S 43.1 -> 36.4; 128x64x64 FP32 20.3 -> 16.5;
 // 64x32x32 FP32 11.4 -> 9.3; 191x95x97 (one cell per thread before) BF16S 43.8 -> 33.8, FP32
 // 58.4 -> 50.1.  What made the difference: the bulk copies issued by one elected
 // lane from uniform registers, 37 an item of 4 rows (by 32 lanes they are replayed one by one,
 // about 20 instructions each, and the producer warp was the limit: 63.5 us), the flat pair
-// list (the helper warp's row ends were 6 M of 46 M instructions, on the critical path) and
+// list (the row ends on a helper warp were 6 M of 44 M instructions, on the critical path) and
 // the near-wall cells at the start of the step, while the ring fills.  Not kept: 14 to 19
 // consumer warps in one CTA per SM (93-96 us: one producer cannot feed an SM); a tail of
 // one-row items (59.5 us here, but 9.7 -> 10.3 at 64x32x32).
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_kernel(const __grid_cons
   uint8_t* const s_wall = s_dslot + 19;                                                    // [S_][R]
 
   uint32_t* const s_mfrag = reinterpret_cast<uint32_t*>(align16(smem_raw, s_wall + S_ * R));  // [24 * 32]
-  float* const s_mbias = reinterpret_cast<float*>(s_mfrag + kMlpFragWords * 32);   // [65]
+  float* const s_mbias = reinterpret_cast<float*>(s_mfrag + kMlpFragWords * 32);   // [kMlpBias]
   uint32_t* const s_mstage = reinterpret_cast<uint32_t*>(s_mbias + kMlpBias);      // [kPairWarps][128]
   if constexpr (MLP) {
     for (int i = threadIdx.x; i < kMlpFragWords * 32; i += blockDim.x) s_mfrag[i] = a.mlp_frag[i];

@@ -17,25 +17,22 @@
 namespace aerosim {
 namespace {
 
-// Forward pass of one sample; keeps the pre-activations for the backward pass.
-__device__ __forceinline__ float mlp_forward_keep(const float* P, const float (&x)[kMlpIn], float (&z1)[kMlpHidden],
-                                                  float (&z2)[kMlpHidden], float& o) {
+// Forward pass of one sample in FP32.
+__device__ __forceinline__ float mlp_forward_one(const float* P, const float (&x)[kMlpIn]) {
   float h1[kMlpHidden];
 #pragma unroll
   for (int j = 0; j < kMlpHidden; ++j) {
     float s = P[kMlpB1 + j];
 #pragma unroll
     for (int i = 0; i < kMlpIn; ++i) s = fmaf(P[kMlpW1 + j * kMlpIn + i], x[i], s);
-    z1[j] = s;
     h1[j] = gelu_f(s);
   }
-  o = P[kMlpB3];
+  float o = P[kMlpB3];
 #pragma unroll 4
   for (int j = 0; j < kMlpHidden; ++j) {
     float s = P[kMlpB2 + j];
 #pragma unroll
     for (int i = 0; i < kMlpHidden; ++i) s = fmaf(P[kMlpW2 + j * kMlpHidden + i], h1[i], s);
-    z2[j] = s;
     o = fmaf(P[kMlpW3 + j], gelu_f(s), o);
   }
   return softplus_f(o);
@@ -312,8 +309,7 @@ __global__ void mlp_forward_kernel(const float* __restrict__ Pg, const float* __
   float x[kMlpIn];
 #pragma unroll
   for (int i = 0; i < kMlpIn; ++i) x[i] = X[t * kMlpIn + i];
-  float z1[kMlpHidden], z2[kMlpHidden], o;
-  out[t] = mlp_forward_keep(P, x, z1, z2, o);
+  out[t] = mlp_forward_one(P, x);
 }
 
 // The step kernel's tensor-core evaluation (mlp_nut_warp) over rows of X: one warp per

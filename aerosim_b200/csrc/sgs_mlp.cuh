@@ -26,10 +26,6 @@ constexpr float kGeluK = 0.7978845608028654f;  // sqrt(2 / pi)
 __host__ __device__ inline float gelu_f(float x) {
   return 0.5f * x * (1.0f + tanhf(kGeluK * (x + 0.044715f * x * x * x)));
 }
-__host__ __device__ inline float gelu_grad(float x) {
-  const float t = tanhf(kGeluK * (x + 0.044715f * x * x * x));
-  return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * kGeluK * (1.0f + 3.0f * 0.044715f * x * x);
-}
 __host__ __device__ inline float softplus_f(float o) { return o > 20.0f ? o : log1pf(expf(o)); }
 __host__ __device__ inline float sigmoid_f(float o) { return 1.0f / (1.0f + expf(-o)); }
 
@@ -73,7 +69,7 @@ __host__ inline uint16_t bf16_bits_rn(float f) {  // round to nearest even
   return (uint16_t)(u >> 16);
 }
 
-__host__ inline void mlp_pack_fragments(const float* P, uint32_t* frag /*[24 * 32]*/, float* bias /*[65]*/) {
+__host__ inline void mlp_pack_fragments(const float* P, uint32_t* frag /*[24 * 32]*/, float* bias /*[kMlpBias]*/) {
   auto pair = [](float lo, float hi) { return (uint32_t)bf16_bits_rn(lo) | ((uint32_t)bf16_bits_rn(hi) << 16); };
   for (int l = 0; l < 32; ++l) {
     const int k0 = 2 * (l % 4), n0 = l / 4;
@@ -153,7 +149,7 @@ __device__ __forceinline__ uint32_t gelu2_bf16x2(float a, float b) {
   return r;
 }
 
-// What bounds it (256x128x128 FP32 step, ncu): issue, about 900 instructions for 32 cells of the
+// What bounds it (256x128x128 FP32 step, ncu): issue, about 740 instructions for 32 cells of the
 // closure and the step together, of them 64 MUFU.TANH (66 us of that unit) and 28 tensor
 // instructions (12 % of theirs).  Fragments and start values as 16-byte shared loads, the
 // accumulators' start values not copied and layer 1 at its own K took the two-cell step from

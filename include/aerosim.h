@@ -312,7 +312,7 @@ typedef struct {
 } aerosim_batch_tuning;
 
 /* engines: n (1..64) engines on one device, each with a voxel grid, all with the same
- * FP32-arithmetic precision (F32, F16S or BF16S).  Resets the flow of every instance;
+ * FP32-arithmetic precision (F32, F16S, BF16S or F16C).  Resets the flow of every instance;
  * the engines must outlive the batch and must not be stepped alone while it exists
  * (per-engine reads are fine).  Errors: aerosim_last_error(NULL). */
 int aerosim_batch_create(aerosim_engine* const* engines, int32_t n, aerosim_batch** out);
