@@ -1301,6 +1301,9 @@ struct aerosim_batch {
   unsigned int* d_ticket = nullptr;  // [4]: CTAs done, then next item, per step parity
   std::vector<long long> item_begin;  // the flat item list: first item and rows per item of each instance
   std::vector<int> item_rows;
+  std::vector<long long> near_begin;  // first near-wall cell of each instance, as uploaded
+  std::vector<Layout> layouts;        // the engines' lattices and populations that the batch was made for
+  std::vector<void*> bufs;
   int* d_step = nullptr;
   int* d_error = nullptr;
   long long n_items = 0, n_near = 0, cells = 0;
@@ -1342,8 +1345,40 @@ void batch_free(aerosim_batch* b) {
   if (b->stream) cudaStreamDestroy(b->stream);
 }
 
+// The near-wall cells of all instances as one list, from the engines' current grids (an engine
+// may be given another body between steps); captured launches carry their number.
+int batch_upload_near(aerosim_batch* b) {
+  std::vector<long long> begin(b->eng.size() + 1, 0);
+  for (size_t k = 0; k < b->eng.size(); ++k) begin[k + 1] = begin[k] + b->eng[k]->near.n;
+  if (begin == b->near_begin) return AEROSIM_OK;
+  BCU(cudaMemcpyAsync(b->d_near_begin, begin.data(), begin.size() * sizeof(long long), cudaMemcpyHostToDevice, b->stream));
+  BCU(cudaStreamSynchronize(b->stream));
+  b->near_begin = begin;
+  b->n_near = begin.back();
+  if (b->graph) {
+    cudaGraphExecDestroy(b->graph);
+    b->graph = nullptr;
+  }
+  return AEROSIM_OK;
+}
+
+// Items and buffers are those of the engines' lattices and populations at creation.
+int batch_check(aerosim_batch* b) {
+  for (size_t k = 0; k < b->eng.size(); ++k) {
+    const aerosim_engine* e = b->eng[k];
+    const Layout& l = b->layouts[k];
+    if (e->L.nx != l.nx || e->L.ny != l.ny || e->L.nz != l.nz || e->f_prec != b->precision || !e->f[0] ||
+        e->f[0] != b->bufs[2 * k] || e->f[1] != b->bufs[2 * k + 1])
+      return bfail(AEROSIM_ERR_STATE, "batch: an engine's lattice or precision has changed since the batch was created");
+  }
+  return AEROSIM_OK;
+}
+
 // The solver arguments of every instance, from its engine's current configuration.
 int batch_upload_table(aerosim_batch* b) {
+  int rc = batch_check(b);
+  if (!rc) rc = batch_upload_near(b);
+  if (rc) return rc;
   std::vector<StepArgs> t(b->eng.size());
   for (size_t k = 0; k < b->eng.size(); ++k) {
     const aerosim_engine* e = b->eng[k];
@@ -1473,6 +1508,7 @@ int batch_apply_tuning(aerosim_batch* b, const aerosim_batch_tuning& t) {
 
 // Fresh flow in every instance and the batch's step counter at zero.
 int batch_reset(aerosim_batch* b) {
+  if (int rc = batch_check(b)) return rc;
   for (aerosim_engine* e : b->eng) {
     BCU(cudaSetDevice(e->device));
     if (do_reset(e)) return bfail(AEROSIM_ERR_CUDA, "batch: reset of an instance failed: " + e->err);
@@ -1568,20 +1604,19 @@ int aerosim_batch_create(aerosim_engine* const* engines, int32_t n, aerosim_batc
     return bfail(rc, msg);
   };
   cudaError_t e = cudaSetDevice(b->device);
-  std::vector<long long> near_begin(n + 1, 0);
-  std::vector<void*> bufs(2 * (size_t)n);
+  b->bufs.resize(2 * (size_t)n);
+  b->layouts.resize(n);
   int pitch = engines[0]->L.pitch;
   for (int k = 0; k < n; ++k) {
     const aerosim_engine* en = engines[k];
     const Layout& L = en->L;
-    near_begin[k + 1] = near_begin[k] + en->near.n;
-    bufs[2 * k] = en->f[0];
-    bufs[2 * k + 1] = en->f[1];
+    b->layouts[k] = L;
+    b->bufs[2 * k] = en->f[0];
+    b->bufs[2 * k + 1] = en->f[1];
     b->cells += en->g.N;
     if (L.pitch != pitch) pitch = 0;
   }
   b->pitch = (pitch == 64 || pitch == 128 || pitch == 192 || pitch == 256) ? pitch : 0;
-  b->n_near = near_begin[n];
   const size_t part = (size_t)3 * b->num_sms * n;
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
@@ -1597,9 +1632,7 @@ int aerosim_batch_create(aerosim_engine* const* engines, int32_t n, aerosim_batc
   if (e == cudaSuccess) e = cudaMalloc(&b->d_step, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_error, sizeof(int));
   if (e == cudaSuccess)
-    e = cudaMemcpyAsync(b->d_bufs, bufs.data(), bufs.size() * sizeof(void*), cudaMemcpyHostToDevice, b->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(b->d_near_begin, near_begin.data(), near_begin.size() * sizeof(long long), cudaMemcpyHostToDevice, b->stream);
+    e = cudaMemcpyAsync(b->d_bufs, b->bufs.data(), b->bufs.size() * sizeof(void*), cudaMemcpyHostToDevice, b->stream);
   if (e != cudaSuccess) {
     bfail(AEROSIM_ERR_CUDA, std::string("batch_create: ") + cudaGetErrorString(e));
     return bail(AEROSIM_ERR_CUDA);

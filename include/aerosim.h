@@ -314,7 +314,8 @@ typedef struct {
 /* engines: n (1..64) engines on one device, each with a voxel grid, all with the same
  * FP32-arithmetic precision (F32, F16S, BF16S or F16C).  Resets the flow of every instance;
  * the engines must outlive the batch and must not be stepped alone while it exists
- * (per-engine reads are fine).  Errors: aerosim_last_error(NULL). */
+ * (per-engine reads, new parameters and another body on the same lattice are fine; after a
+ * change of an engine's lattice or precision the batch's steps fail with AEROSIM_ERR_STATE).  Errors: aerosim_last_error(NULL). */
 int aerosim_batch_create(aerosim_engine* const* engines, int32_t n, aerosim_batch** out);
 int aerosim_batch_destroy(aerosim_batch* b);
 /* n steps of every instance; each engine's step count and readouts advance with it. */
