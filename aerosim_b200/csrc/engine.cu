@@ -549,6 +549,7 @@ int aerosim_voxelize(aerosim_engine* h, const float* positions, int64_t vertex_c
   if (rc) {
     cudaGetLastError();
     grid_free(&ng);
+    h->vox.trim();
     return fail(h, rc == -4 ? AEROSIM_ERR_DEVICE : AEROSIM_ERR_CUDA, e);
   }
   const double origin[3] = {ng.ox, ng.oy, ng.oz};

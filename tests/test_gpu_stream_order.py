@@ -26,6 +26,8 @@ def _streams(call):
             uploads.setdefault(e.device_resource_id(), []).append(e.name())
         elif not e.name().startswith("Mem"):
             kernels.setdefault(e.device_resource_id(), []).append(e.name())
+    if not kernels and not uploads:
+        pytest.skip("the profiler sees no device activity on this machine")
     return kernels, uploads
 
 
